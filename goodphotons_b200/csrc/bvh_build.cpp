@@ -313,6 +313,7 @@ std::vector<FNode> widen_nodes(const WideBvh& bvh) {
         FNode& f = out[i];
         f.child_base = w.child_base;
         f.prim_base = w.prim_base;
+        f.pad[0] = f.pad[1] = 0;
         const float p[3] = {w.px, w.py, w.pz};
         const int eb[3] = {w.ex, w.ey, w.ez};
         float sc[3] = {0.0f, 0.0f, 0.0f};
@@ -322,7 +323,9 @@ std::vector<FNode> widen_nodes(const WideBvh& bvh) {
         const uint8_t* qhi[3] = {w.qhi_x, w.qhi_y, w.qhi_z};
         for (int k = 0; k < FTB_WIDTH; ++k) {
             const uint8_t m = w.meta[k];
-            f.meta[k] = (m != 0 && ((w.imask >> k) & 1u)) ? (uint8_t)((FNODE_INNER << 5) | (m & 31u)) : m;
+            const bool inner = m != 0 && ((w.imask >> k) & 1u);
+            f.meta[k] = inner ? (uint8_t)((FNODE_INNER << 5) | (m & 31u)) : m;
+            f.code[k] = inner || !m ? (uint8_t)(m & 31u) : (uint8_t)(128u | ((m & 31u) << 2) | ((m >> 5) - 1u));
             for (int a = 0; a < 3; ++a) {
                 const float s = sc[a];
                 if (!m) {

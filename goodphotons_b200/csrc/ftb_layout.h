@@ -2,7 +2,7 @@
 // bvh_build.cpp) and the kernels (ftb_kernels.cu).
 //
 // HBM layout of a baked scene:
-//   nodes   : FNode[n_nodes], 208 B each, 16 B aligned -- 8-wide BVH.  The builders make
+//   nodes   : FNode[n_nodes], 224 B each, 32 B aligned -- 8-wide BVH.  The builders make
 //             compressed 80-byte WNodes (child boxes 8-bit quantized against the node's
 //             float grid (p, 2^e), rounded outward, so the fp32 traversal never culls a
 //             primitive the exact fp64 test would accept); the upload widens each to an
@@ -44,17 +44,23 @@ static_assert(sizeof(WNode) == 80, "WNode must be 80 bytes");
 // float the 8-bit form decodes to (fmaf(q, 2^e, p), the value the builders check against
 // the exact box), so traversal reads planes instead of decoding bytes.  Planes are kept
 // per axis and side, so a ray takes its near and far planes by its direction's signs with
-// no per-child select.  meta byte: 0 = empty; count<<5 | offset for a leaf (count 1..4,
-// offset from prim_base); 7<<5 | offset for an inner child (offset from child_base).  An
-// empty child has lo = +inf and hi = -inf on every axis, which every ray's slab test misses.
-struct alignas(16) FNode {
+// no per-child select.  Every row of eight planes, and the header, is one 32-byte sector:
+// a node visit is six 32-byte loads and one of 16 (a node is 224 B, so rows stay aligned).
+// meta byte: 0 = empty; count<<5 | offset for a leaf (count 1..4, offset from prim_base);
+// 7<<5 | offset for an inner child (offset from child_base).  code byte, the same child as
+// the traversal adds it to a base: 0..127 an inner child's offset; 128 | offset<<2 |
+// (count - 1) a leaf's.  An empty child has lo = +inf and hi = -inf on every axis, which
+// every ray's slab test misses.
+struct alignas(32) FNode {
     uint32_t child_base;
     uint32_t prim_base;
+    uint8_t code[8];
     uint8_t meta[8];
+    uint32_t pad[2];
     float lo[3][8];
     float hi[3][8];
 };
-static_assert(sizeof(FNode) == 208, "FNode must be 208 bytes");
+static_assert(sizeof(FNode) == 224, "FNode must be 224 bytes");
 #define FNODE_INNER 7u
 
 // 80-byte primitive record.  d[9] holds two int32: prim (global index) and
