@@ -1864,13 +1864,37 @@ __global__ void __launch_bounds__(128, MEDIA ? FTB_SHADE_MEDIA_MINB : FTB_SHADE_
     tally_finish(acc, jobs, multi, n_jobs);
 }
 
+// Add a splat's four words to a pixel: one 32-byte bulk reduction (sm_90+ cp.reduce of u64
+// sums) from a shared-memory slot of the thread's own, or four atomics where the caller's film
+// is not 16-byte aligned, which the bulk operation requires.  Both are exact integer sums in
+// any order.  The four separate atomics bounded the connection kernel: Cornell, 256^2, 2^24
+// photons (40 M connections): 5.1 ms with them, 2.8 ms with the bulk reduction, 2.4 ms with
+// no film update at all; glass, 1024^2, 2^27 photons: 33.5 and 32.0 ms.
+__device__ __forceinline__ void film_add(int64_t* film, int pix, long long x, long long y, long long z, long long n) {
+    __shared__ alignas(32) long long slot[128][4];   // blocks are of 128 threads
+    long long* px = reinterpret_cast<long long*>(film) + 4 * (size_t)pix;
+    if ((reinterpret_cast<uintptr_t>(film) & 15) == 0) {
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the slot's last reduction has read it
+        long long* sp = slot[threadIdx.x];
+        sp[0] = x; sp[1] = y; sp[2] = z; sp[3] = n;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], 32;"
+                     :: "l"(px), "r"((uint32_t)__cvta_generic_to_shared(sp)) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        return;
+    }
+    atomicAdd(reinterpret_cast<unsigned long long*>(px), (unsigned long long)x);
+    atomicAdd(reinterpret_cast<unsigned long long*>(px + 1), (unsigned long long)y);
+    atomicAdd(reinterpret_cast<unsigned long long*>(px + 2), (unsigned long long)z);
+    atomicAdd(reinterpret_cast<unsigned long long*>(px + 3), (unsigned long long)n);
+}
+// Every thread of a kernel that splats, before it ends: its reductions are complete.
+__device__ __forceinline__ void film_finish() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 __device__ __forceinline__ void splat(const DevJob& J, int view, int pix, double X, double Y, double Z,
                                       int32_t* status) {
-    long long* px = reinterpret_cast<long long*>(view_film(J, view)) + 4 * (size_t)pix;
-    atomicAdd(reinterpret_cast<unsigned long long*>(px), (unsigned long long)to_fixed(X, J.film_scale_inv, status));
-    atomicAdd(reinterpret_cast<unsigned long long*>(px + 1), (unsigned long long)to_fixed(Y, J.film_scale_inv, status));
-    atomicAdd(reinterpret_cast<unsigned long long*>(px + 2), (unsigned long long)to_fixed(Z, J.film_scale_inv, status));
-    atomicAdd(reinterpret_cast<unsigned long long*>(px + 3), 1ull);
+    film_add(view_film(J, view), pix, to_fixed(X, J.film_scale_inv, status), to_fixed(Y, J.film_scale_inv, status),
+             to_fixed(Z, J.film_scale_inv, status), 1);
 }
 
 // A mirror record's tests, in connectSpecularPlane's order (render.h:1366-1379): the light
@@ -1972,6 +1996,7 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow(Wave w, const Dev
         if (traverse_any<COUNT, INST, SHAPES>(sc, R, EPS_RAY, max_dist - EPS_RAY, f.status, cnt)) continue;
         splat(J, w.sview[i], w.spix[i], w.sxyz[i], w.sxyz[w.S + i], w.sxyz[2 * (size_t)w.S + i], f.status);
     }
+    film_finish();
     if (COUNT) {
         block_add3(f.stats + 3, rays, cnt.nodes, cnt.recs);
         block_add1(f.stats + 7, cnt.exact);
@@ -2346,11 +2371,7 @@ __device__ __noinline__ void mirror_splat_hero(const DevJob& J, const Wave& w, c
         ++hits;
     }
     if (!hits) return;
-    long long* px = reinterpret_cast<long long*>(view_film(J, w.sview[i] & 0xffff)) + 4 * (size_t)~w.spix[i];
-    atomicAdd(reinterpret_cast<unsigned long long*>(px), (unsigned long long)sx);
-    atomicAdd(reinterpret_cast<unsigned long long*>(px + 1), (unsigned long long)sy);
-    atomicAdd(reinterpret_cast<unsigned long long*>(px + 2), (unsigned long long)sz);
-    atomicAdd(reinterpret_cast<unsigned long long*>(px + 3), (unsigned long long)hits);
+    film_add(view_film(J, w.sview[i] & 0xffff), ~w.spix[i], sx, sy, sz, hits);
 }
 
 // Connections of bundles: one occlusion test, then a splat per wavelength.  MIRROR: the queue
@@ -2375,10 +2396,9 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow_hero(Wave w, cons
         double max_dist = w.smax[i];
         RayCtx R = make_ray(o, d);
         if (traverse_any<COUNT, INST, SHAPES>(sc, R, EPS_RAY, max_dist - EPS_RAY, f.status, cnt)) continue;
-        long long* px = reinterpret_cast<long long*>(view_film(J, w.sview[i])) + 4 * (size_t)w.spix[i];
         const int nup = w.snup[i];
         // every wavelength is one Film::add, each rounded to fixed point on its own; their
-        // integer sum goes to the pixel in one atomic per channel (integer sums are exact)
+        // integer sum goes to the pixel at once (integer sums are exact)
         long long sx = 0, sy = 0, sz = 0;
         for (int k = 0; k < nup; ++k) {
             double lam = k == 0 ? w.slam[i] : w.xlam[(size_t)(k - 1) * w.S + i];
@@ -2388,11 +2408,9 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow_hero(Wave w, cons
             sy += to_fixed(Y, J.film_scale_inv, f.status);
             sz += to_fixed(Z, J.film_scale_inv, f.status);
         }
-        atomicAdd(reinterpret_cast<unsigned long long*>(px), (unsigned long long)sx);
-        atomicAdd(reinterpret_cast<unsigned long long*>(px + 1), (unsigned long long)sy);
-        atomicAdd(reinterpret_cast<unsigned long long*>(px + 2), (unsigned long long)sz);
-        atomicAdd(reinterpret_cast<unsigned long long*>(px + 3), (unsigned long long)nup);
+        film_add(view_film(J, w.sview[i]), w.spix[i], sx, sy, sz, nup);
     }
+    film_finish();
     if (COUNT) {
         block_add3(f.stats + 3, rays, cnt.nodes, cnt.recs);
         block_add1(f.stats + 7, cnt.exact);
