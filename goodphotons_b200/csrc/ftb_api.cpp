@@ -587,6 +587,17 @@ double box_maxabs(const ftb::Box& b, double m) {
 
 // Bake one BLAS on `device` (current): triangle boxes, wide BVH with a margin from the
 // local coordinate magnitude, records in leaf order (prim = the triangle's BLAS index).
+// Record rows (PrimRec): a triangle's vertices by axis, or up to three values per row; the
+// tail (prim, info) goes to the end of every row.
+void rec_triangle(PrimRec& R, const double* v) {
+    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < 3; ++k) R.row[a][k] = v[3 * k + a];
+}
+void rec_tail(PrimRec& R, int32_t prim, int32_t info) {
+    const uint64_t tail = (uint64_t)(uint32_t)prim | ((uint64_t)(uint32_t)info << 32);
+    for (auto& row : R.row) std::memcpy(&row[3], &tail, sizeof tail);
+}
+
 ftb_status bake_blas(const ftb_blas_desc& d, int device, ftb::BuildMethod method, std::shared_ptr<BlasDev>& out) {
     auto b = std::make_shared<BlasDev>();
     b->mem.device = device;
@@ -619,13 +630,12 @@ ftb_status bake_blas(const ftb_blas_desc& d, int device, ftb::BuildMethod method
         int p = bvh.order[r];
         PrimRec& R = recs[r];
         std::memset(&R, 0, sizeof R);
-        std::memcpy(R.d, d.tri_v + 9 * (size_t)p, 9 * sizeof(double));
-        R.prim = p;
+        rec_triangle(R, d.tri_v + 9 * (size_t)p);
         int smooth = 0;
         if (d.tri_n)
             for (int k = 0; k < 9; ++k) if (d.tri_n[9 * (size_t)p + k] != 0.0) smooth = 1;
         any_smooth |= smooth != 0;
-        R.info = d.tri_mat[p] | (REC_TRI << 24) | (smooth << 30);
+        rec_tail(R, p, d.tri_mat[p] | (REC_TRI << 24) | (smooth << 30));
     }
     const std::vector<FNode> fn = ftb::widen_nodes(bvh);
     ftb_status st = upload(b->mem, fn.data(), fn.size(), &b->nodes, "upload BLAS nodes");
@@ -1321,28 +1331,32 @@ ftb_status ftb_scene_create(const ftb_scene_desc* d, int32_t device, ftb_scene**
         int p = bvh.order[r];
         PrimRec& R = recs[r];
         std::memset(&R, 0, sizeof R);
-        R.prim = p;
         int ty, mat, smooth = 0;
         if (p < nt) {
-            std::memcpy(R.d, d->tri_v + 9 * (size_t)p, 9 * sizeof(double));
+            rec_triangle(R, d->tri_v + 9 * (size_t)p);
             ty = REC_TRI; mat = d->tri_mat[p];
             if (d->tri_n) {
                 const double* n = d->tri_n + 9 * (size_t)p;
                 for (int k = 0; k < 9; ++k) if (n[k] != 0.0) smooth = 1;
             }
         } else if (p < nt + ns) {
-            std::memcpy(R.d, d->sph + 4 * (size_t)(p - nt), 4 * sizeof(double));
+            const double* sp = d->sph + 4 * (size_t)(p - nt);
+            std::memcpy(R.row[0], sp, 3 * sizeof(double));
+            R.row[1][0] = sp[3];
             ty = REC_SPHERE; mat = d->sph_mat[p - nt];
         } else if (p < nt + ns + nc) {
-            std::memcpy(R.d, d->curve + 10 * (size_t)(p - nt - ns), 8 * sizeof(double));
+            const double* c = d->curve + 10 * (size_t)(p - nt - ns);
+            std::memcpy(R.row[0], c, 3 * sizeof(double));
+            std::memcpy(R.row[1], c + 3, 3 * sizeof(double));
+            std::memcpy(R.row[2], c + 6, 2 * sizeof(double));
             ty = REC_CURVE; mat = d->curve_mat[p - nt - ns];
         } else {
             int64_t k = p - nt - ns - nc;
-            std::memcpy(&R.d[0], &k, sizeof k);
+            std::memcpy(&R.row[0][0], &k, sizeof k);
             ty = REC_INST; mat = 0;
         }
         any_smooth |= smooth != 0;
-        R.info = mat | (ty << 24) | (smooth << 30);
+        rec_tail(R, p, mat | (ty << 24) | (smooth << 30));
     }
     std::vector<DevSpec> spec((size_t)d->n_spectra);
     for (int i = 0; i < d->n_spectra; ++i) {

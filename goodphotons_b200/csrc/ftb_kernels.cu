@@ -237,14 +237,17 @@ __device__ __forceinline__ double zero_fallback(double a, double b, double c, do
     return (ph - qh) + (pl - ql);
 }
 struct TriHitW { double u, v, w, inv_det; };
-// intersectTri acceptance (geometry.h:280-324); returns t or -1 (rejected)
-__device__ __forceinline__ bool tri_test(const Shear& sh, D3 ro, const double* v, double tmin,
-                                         double tbest, double& t_out, TriHitW* bw) {
-    D3 A = mk(v[0], v[1], v[2]) - ro, B = mk(v[3], v[4], v[5]) - ro, C = mk(v[6], v[7], v[8]) - ro;
-    double Akz = comp(A, sh.kz), Bkz = comp(B, sh.kz), Ckz = comp(C, sh.kz);
-    double Ax = comp(A, sh.kx) - sh.sx * Akz, Ay = comp(A, sh.ky) - sh.sy * Akz;
-    double Bx = comp(B, sh.kx) - sh.sx * Bkz, By = comp(B, sh.ky) - sh.sy * Bkz;
-    double Cx = comp(C, sh.kx) - sh.sx * Ckz, Cy = comp(C, sh.ky) - sh.sy * Ckz;
+// A row of a record: one coordinate of the three vertices, and the record's tail.
+struct RecRow { double a, b, c; uint32_t prim, info; };
+// intersectTri acceptance (geometry.h:280-324) on the vertex rows of the ray's axes kx, ky, kz
+// and the origin's components ox, oy, oz on those axes; returns t or rejects.
+__device__ __forceinline__ bool tri_test(double sx, double sy, double sz, double ox, double oy, double oz,
+                                         const RecRow& X, const RecRow& Y, const RecRow& Z, double tmin, double tbest,
+                                         double& t_out, TriHitW* bw) {
+    const double Akz = Z.a - oz, Bkz = Z.b - oz, Ckz = Z.c - oz;
+    const double Ax = (X.a - ox) - sx * Akz, Ay = (Y.a - oy) - sy * Akz;
+    const double Bx = (X.b - ox) - sx * Bkz, By = (Y.b - oy) - sy * Bkz;
+    const double Cx = (X.c - ox) - sx * Ckz, Cy = (Y.c - oy) - sy * Ckz;
     double U = Cx * By - Cy * Bx;
     double V = Ax * Cy - Ay * Cx;
     double W = Bx * Ay - By * Ax;
@@ -256,7 +259,7 @@ __device__ __forceinline__ bool tri_test(const Shear& sh, D3 ro, const double* v
     if ((U < 0.0 || V < 0.0 || W < 0.0) && (U > 0.0 || V > 0.0 || W > 0.0)) return false;
     double det = U + V + W;
     if (det == 0.0) return false;
-    double T = U * (sh.sz * Akz) + V * (sh.sz * Bkz) + W * (sh.sz * Ckz);
+    double T = U * (sz * Akz) + V * (sz * Bkz) + W * (sz * Ckz);
     double inv_det = 1.0 / det;
     double t = T * inv_det;
     if (t < tmin || t >= tbest) return false;
@@ -359,18 +362,37 @@ __device__ bool curve_test(const CurveRay& cr, D3 ro, const double* s, double tm
     return true;
 }
 
-__device__ __forceinline__ int rec_type(const PrimRec& r) { return (r.info >> 24) & 3; }
-__device__ __forceinline__ int rec_mat(const PrimRec& r) { return r.info & 0xffffff; }
-__device__ __forceinline__ bool rec_smooth(const PrimRec& r) { return (r.info >> 30) & 1; }
+// A record's rows in natural order: d[3 * row + k].
+struct Rec {
+    double d[9];
+    int32_t prim, info;
+};
+__device__ __forceinline__ int rec_type(uint32_t info) { return (info >> 24) & 3; }
+__device__ __forceinline__ int rec_type(const Rec& r) { return rec_type((uint32_t)r.info); }
+__device__ __forceinline__ int rec_mat(const Rec& r) { return r.info & 0xffffff; }
+__device__ __forceinline__ bool rec_smooth(const Rec& r) { return (r.info >> 30) & 1; }
 
-__device__ __forceinline__ void load_rec(const PrimRec* recs, int i, PrimRec& r) {
-    const double2* p = reinterpret_cast<const double2*>(recs + i);
-    double2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3), e = __ldg(p + 4);
-    r.d[0] = a.x; r.d[1] = a.y; r.d[2] = b.x; r.d[3] = b.y; r.d[4] = c.x; r.d[5] = c.y;
-    r.d[6] = d.x; r.d[7] = d.y; r.d[8] = e.x;
-    long long tail = __double_as_longlong(e.y);
-    r.prim = (int32_t)(tail & 0xffffffffLL);
-    r.info = (int32_t)(tail >> 32);
+// Row `off` / 32 (a byte offset) of record i, in one 32-byte load.  Bound: a record test is
+// instruction issue; loading the rows in the ray's axis order takes the place of the selects
+// that permuted each vertex (36 of ~130 instructions) and of two of the five loads.  Closest
+// hit of a frame against 80-byte vertex records (B200): Cornell 3.29 -> 2.88 ms, glass 135.7
+// -> 130.0, fog + strands 66.4 -> 60.8; occlusion 2.85 -> 2.71, 32.3 -> 31.2, 30.4 -> 31.3
+// (a curve reloads its rows in natural order there).
+__device__ __forceinline__ RecRow ld_rec_row(const PrimRec* recs, int i, uint32_t off) {
+    RecRow r;
+    const char* p = reinterpret_cast<const char*>(recs + i) + off;
+    double tail;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.a), "=d"(r.b), "=d"(r.c), "=d"(tail) : "l"(p));
+    r.prim = (uint32_t)__double2loint(tail);
+    r.info = (uint32_t)__double2hiint(tail);
+    return r;
+}
+__device__ __forceinline__ void load_rec(const PrimRec* recs, int i, Rec& r) {
+    const RecRow a = ld_rec_row(recs, i, 0), b = ld_rec_row(recs, i, 32), c = ld_rec_row(recs, i, 64);
+    r.d[0] = a.a; r.d[1] = a.b; r.d[2] = a.c; r.d[3] = b.a; r.d[4] = b.b; r.d[5] = b.c;
+    r.d[6] = c.a; r.d[7] = c.b; r.d[8] = c.c;
+    r.prim = (int32_t)a.prim;
+    r.info = (int32_t)a.info;
 }
 
 struct RayCtx {
@@ -378,16 +400,25 @@ struct RayCtx {
     Shear sh;
     CurveRay cr;
 };
-
-// SHAPES: the scene has spheres or curves besides triangles; without them the record test
-// is the triangle test alone (a smaller traversal kernel with fewer spills).
-template <bool SHAPES>
-__device__ __forceinline__ bool rec_test(const RayCtx& R, const PrimRec& r, double tmin, double tbest,
-                                         double& t) {
-    if (!SHAPES) return tri_test(R.sh, R.o, r.d, tmin, tbest, t, nullptr);
-    int ty = rec_type(r);
-    if (ty == REC_TRI) return tri_test(R.sh, R.o, r.d, tmin, tbest, t, nullptr);
-    if (ty == REC_SPHERE) return sphere_test(R.o, R.d, r.d, tmin, tbest, t);
+// A ray as the triangle test reads it: the shear, the origin's components on the axes kx, ky,
+// kz, and the byte offsets of those axes' rows in a record.
+struct TriRay {
+    double sx, sy, sz, ox, oy, oz;
+    uint32_t rx, ry, rz;
+};
+__device__ __forceinline__ TriRay tri_ray(const Shear& sh, D3 o) {
+    TriRay r;
+    r.sx = sh.sx; r.sy = sh.sy; r.sz = sh.sz;
+    r.ox = comp(o, sh.kx); r.oy = comp(o, sh.ky); r.oz = comp(o, sh.kz);
+    r.rx = 32u * sh.kx; r.ry = 32u * sh.ky; r.rz = 32u * sh.kz;
+    return r;
+}
+// Test of record i of a kind that is not a triangle.
+__device__ __forceinline__ bool shape_test(const RayCtx& R, const PrimRec* recs, int i, double tmin, double tbest,
+                                           double& t) {
+    Rec r;
+    load_rec(recs, i, r);
+    if (rec_type(r) == REC_SPHERE) return sphere_test(R.o, R.d, r.d, tmin, tbest, t);
     return curve_test(R.cr, R.o, r.d, tmin, tbest, t, nullptr);
 }
 
@@ -398,16 +429,19 @@ struct Hit {
     int mat, prim;
 };
 template <bool SHAPES>
-__device__ void hit_attributes(const double* __restrict__ tri_n, const RayCtx& R, const PrimRec& r, Hit& h) {
+__device__ void hit_attributes(const double* __restrict__ tri_n, const RayCtx& R, const PrimRec* recs, int i,
+                               const Rec& r, Hit& h) {
     int ty = SHAPES ? rec_type(r) : REC_TRI;
     h.mat = rec_mat(r);
     h.prim = r.prim;
     double t = 0.0;
     if (ty == REC_TRI) {
         TriHitW w;
-        tri_test(R.sh, R.o, r.d, EPS_RAY, DBL_MAX, t, &w);
+        const TriRay T = tri_ray(R.sh, R.o);
+        tri_test(T.sx, T.sy, T.sz, T.ox, T.oy, T.oz, ld_rec_row(recs, i, T.rx), ld_rec_row(recs, i, T.ry),
+                 ld_rec_row(recs, i, T.rz), EPS_RAY, DBL_MAX, t, &w);
         double b0 = w.u * w.inv_det, b1 = w.v * w.inv_det, b2 = w.w * w.inv_det;
-        D3 v0 = mk(r.d[0], r.d[1], r.d[2]), v1 = mk(r.d[3], r.d[4], r.d[5]), v2 = mk(r.d[6], r.d[7], r.d[8]);
+        D3 v0 = mk(r.d[0], r.d[3], r.d[6]), v1 = mk(r.d[1], r.d[4], r.d[7]), v2 = mk(r.d[2], r.d[5], r.d[8]);
         D3 tgn = normalize(cross(v1 - v0, v2 - v0));     // Tri::finalize (geometry.h:52)
         D3 n0 = tgn, n1 = tgn, n2 = tgn;
         if (rec_smooth(r)) {
@@ -701,7 +735,7 @@ __device__ __forceinline__ D3 xf_normal(const double* il, D3 n) {
               il[1] * n.x + il[4] * n.y + il[7] * n.z,
               il[2] * n.x + il[5] * n.y + il[8] * n.z);
 }
-__device__ __forceinline__ int rec_inst(const PrimRec& r) { return (int)__double_as_longlong(r.d[0]); }
+__device__ __forceinline__ int rec_inst(const Rec& r) { return (int)__double_as_longlong(r.d[0]); }
 
 // The world ray mapped into an instance's local space (Scene::closestHit instance leaf,
 // scene.h:2226-2228): local t equals world t, the direction is not renormalized.
@@ -731,20 +765,20 @@ __device__ __noinline__ int blas_closest(const DevInst& I, D3 wo, D3 wd, double 
                                          float& tmax_f, int inst_prim, BestHit& bh, int32_t* status,
                                          TravCount& cnt) {
     const LocalRay L = to_local(I, wo, wd);
-    const Shear sh = make_shear(L.d);
+    const TriRay T = tri_ray(make_shear(L.d), L.o);
     const RayF F = make_rayf(L.o, L.d);
     const PrimRec* __restrict__ recs = I.recs;
     int best = -1;
     auto leaf = [&](int first, int count, float tm) -> float {
         for (int k = 0; k < count; ++k) {
             if (COUNT) { cnt.recs++; cnt.exact++; }
-            PrimRec r;
-            load_rec(recs, first + k, r);
+            const RecRow X = ld_rec_row(recs, first + k, T.rx), Y = ld_rec_row(recs, first + k, T.ry);
+            const RecRow Z = ld_rec_row(recs, first + k, T.rz);
             double t;
-            if (tri_test(sh, L.o, r.d, tmin, next_up(best_t), t, nullptr) &&
-                (t < best_t || inst_prim < bh.prim || (inst_prim == bh.prim && r.prim < bh.sub_prim))) {
+            if (tri_test(T.sx, T.sy, T.sz, T.ox, T.oy, T.oz, X, Y, Z, tmin, next_up(best_t), t, nullptr) &&
+                (t < best_t || inst_prim < bh.prim || (inst_prim == bh.prim && (int)X.prim < bh.sub_prim))) {
                 best_t = t; best = first + k; tm = __double2float_ru(t);
-                bh.prim = inst_prim; bh.sub_prim = r.prim;
+                bh.prim = inst_prim; bh.sub_prim = (int)X.prim;
             }
         }
         return tm;
@@ -759,16 +793,16 @@ template <bool COUNT>
 __device__ __noinline__ bool blas_any(const DevInst& I, D3 wo, D3 wd, double tmin, double seg, float tmax_f,
                                       int32_t* status, TravCount& cnt) {
     const LocalRay L = to_local(I, wo, wd);
-    const Shear sh = make_shear(L.d);
+    const TriRay T = tri_ray(make_shear(L.d), L.o);
     const RayF F = make_rayf(L.o, L.d);
     const PrimRec* __restrict__ recs = I.recs;
     auto leaf = [&](int first, int count) -> bool {
         for (int k = 0; k < count; ++k) {
             if (COUNT) { cnt.recs++; cnt.exact++; }
-            PrimRec r;
-            load_rec(recs, first + k, r);
+            const RecRow X = ld_rec_row(recs, first + k, T.rx), Y = ld_rec_row(recs, first + k, T.ry);
+            const RecRow Z = ld_rec_row(recs, first + k, T.rz);
             double t;
-            if (tri_test(sh, L.o, r.d, tmin, seg, t, nullptr)) return true;
+            if (tri_test(T.sx, T.sy, T.sz, T.ox, T.oy, T.oz, X, Y, Z, tmin, seg, t, nullptr)) return true;
         }
         return false;
     };
@@ -783,34 +817,55 @@ template <bool COUNT, bool INST, bool SHAPES>
 __device__ int traverse_closest(const DevScene& sc, const RayCtx& R, double tmin, double& best_t, int* sub,
                                 int32_t* status, TravCount& cnt) {
     const RayF F = make_rayf(R.o, R.d);
+    const TriRay T = tri_ray(R.sh, R.o);
     best_t = DBL_MAX;
     int best = -1;
     BestHit bh{INT_MAX, INT_MAX};
     const PrimRec* __restrict__ recs = sc.recs;
+    // t <= best_t from a record test; a tie goes to the lower index
+    auto take = [&](bool hit, double t, int rec, int prim, float& tm) {
+        if (hit && (t < best_t || prim < bh.prim)) {
+            best_t = t; best = rec; tm = __double2float_ru(t);
+            bh.prim = prim; bh.sub_prim = INT_MAX;
+        }
+    };
     auto leaf = [&](int first, int count, float tm) -> float {
         for (int k = 0; k < count; ++k) {
             if (COUNT) cnt.recs++;
-            PrimRec r;
-            load_rec(recs, first + k, r);
-            if (INST && rec_type(r) == REC_INST) {
+            const RecRow X = ld_rec_row(recs, first + k, T.rx), Y = ld_rec_row(recs, first + k, T.ry);
+            const RecRow Z = ld_rec_row(recs, first + k, T.rz);
+            if (INST && rec_type(X.info) == REC_INST) {
+                Rec r;
+                load_rec(recs, first + k, r);
                 int s = blas_closest<COUNT>(sc.inst[rec_inst(r)], R.o, R.d, tmin, best_t, tm, r.prim, bh, status, cnt);
                 if (s >= 0) { best = first + k; *sub = s; }
                 continue;
             }
             if (COUNT) cnt.exact++;
             double t;
-            // t <= best_t from the test; a tie goes to the lower index
-            if (rec_test<SHAPES>(R, r, tmin, next_up(best_t), t) && (t < best_t || r.prim < bh.prim)) {
-                best_t = t; best = first + k; tm = __double2float_ru(t);
-                bh.prim = r.prim; bh.sub_prim = INT_MAX;
-            }
+            const bool hit = !SHAPES || rec_type(X.info) == REC_TRI
+                                 ? tri_test(T.sx, T.sy, T.sz, T.ox, T.oy, T.oz, X, Y, Z, tmin, next_up(best_t), t, nullptr)
+                                 : shape_test(R, recs, first + k, tmin, next_up(best_t), t);
+            take(hit, t, first + k, (int)X.prim, tm);
         }
         return tm;
     };
     LocalStack<uint2> st;
     const float tm = walk_closest<COUNT>(sc.nodes, F, __double2float_rd(tmin), FLT_MAX, st, leaf, status, cnt);
-    if (SHAPES && sc.root2 > 0)   // the curves' hierarchy, under the bound the first walk left
-        walk_closest<COUNT>(sc.nodes, F, __double2float_rd(tmin), tm, st, leaf, status, cnt, (uint32_t)sc.root2);
+    if (SHAPES && sc.root2 > 0) {   // the curves' hierarchy, under the bound the first walk left
+        auto curves = [&](int first, int count, float tm2) -> float {
+            for (int k = 0; k < count; ++k) {
+                if (COUNT) { cnt.recs++; cnt.exact++; }
+                Rec r;
+                load_rec(recs, first + k, r);
+                double t;
+                const bool hit = curve_test(R.cr, R.o, r.d, tmin, next_up(best_t), t, nullptr);
+                take(hit, t, first + k, r.prim, tm2);
+            }
+            return tm2;
+        };
+        walk_closest<COUNT>(sc.nodes, F, __double2float_rd(tmin), tm, st, curves, status, cnt, (uint32_t)sc.root2);
+    }
     return best;
 }
 
@@ -820,19 +875,26 @@ __device__ bool traverse_any(const DevScene& sc, const RayCtx& R, double tmin, d
                              TravCount& cnt) {
     const RayF F = make_rayf(R.o, R.d);
     const float tmin_f = __double2float_rd(tmin), tmax_f = __double2float_ru(seg);
+    const TriRay T = tri_ray(R.sh, R.o);
     const PrimRec* __restrict__ recs = sc.recs;
     auto leaf = [&](int first, int count) -> bool {
         for (int k = 0; k < count; ++k) {
             if (COUNT) cnt.recs++;
-            PrimRec r;
-            load_rec(recs, first + k, r);
-            if (INST && rec_type(r) == REC_INST) {
+            const RecRow X = ld_rec_row(recs, first + k, T.rx), Y = ld_rec_row(recs, first + k, T.ry);
+            const RecRow Z = ld_rec_row(recs, first + k, T.rz);
+            if (INST && rec_type(X.info) == REC_INST) {
+                Rec r;
+                load_rec(recs, first + k, r);
                 if (blas_any<COUNT>(sc.inst[rec_inst(r)], R.o, R.d, tmin, seg, tmax_f, status, cnt)) return true;
                 continue;
             }
             if (COUNT) cnt.exact++;
             double t;
-            if (rec_test<SHAPES>(R, r, tmin, seg, t)) return true;
+            if (!SHAPES || rec_type(X.info) == REC_TRI) {
+                if (tri_test(T.sx, T.sy, T.sz, T.ox, T.oy, T.oz, X, Y, Z, tmin, seg, t, nullptr)) return true;
+            } else if (shape_test(R, recs, first + k, tmin, seg, t)) {
+                return true;
+            }
         }
         return false;
     };
@@ -849,9 +911,9 @@ __device__ void instance_hit(const DevInst& I, int sub, D3 ro, D3 rd, Hit& h) {
     RayCtx R;
     R.o = L.o; R.d = L.d;
     R.sh = make_shear(L.d);
-    PrimRec br;
+    Rec br;
     load_rec(I.recs, sub, br);
-    hit_attributes<false>(I.tri_n, R, br, h);   // BLAS records are triangles
+    hit_attributes<false>(I.tri_n, R, I.recs, sub, br, h);   // BLAS records are triangles
     h.p = ro + rd * h.t;                        // world t == local t
     D3 wn = normalize(xf_normal(I.xl, h.n));
     D3 wng = normalize(xf_normal(I.xl, h.ng));
@@ -1307,10 +1369,13 @@ template <bool INST>
 __device__ __forceinline__ void log_hit(const Wave& w, const PathState& ps, int i, const DevScene& sc, int rec) {
     if (!w.logs) return;
     const int nh = ps.lnh[i];
-    const int prim = rec >= 0 ? sc.recs[rec].prim : -1;
+    Rec r;
+    r.prim = -1; r.info = 0;
+    if (rec >= 0) load_rec(sc.recs, rec, r);
+    const int prim = r.prim;
     uint64_t hsh = fnv_i32(ps.lhash[i], prim);
-    if (INST && rec >= 0 && rec_type(sc.recs[rec]) == REC_INST)   // and the BLAS triangle
-        hsh = fnv_i32(hsh, sc.inst[rec_inst(sc.recs[rec])].recs[w.hit_sub[i]].prim);
+    if (INST && rec >= 0 && rec_type(r) == REC_INST)   // and the BLAS triangle
+        hsh = fnv_i32(hsh, (int32_t)ld_rec_row(sc.inst[rec_inst(r)].recs, w.hit_sub[i], 0).prim);
     ps.lhash[i] = hsh;
     if (nh < 8) ps.lprims[nh * w.W + i] = prim;
     ps.lnh[i] = nh + 1;
@@ -1715,7 +1780,7 @@ __global__ void __launch_bounds__(128, MEDIA ? FTB_SHADE_MEDIA_MINB : FTB_SHADE_
         } else if (!valid) {
             fate = 1;
         } else {
-            PrimRec r;
+            Rec r;
             load_rec(sc.recs, rec, r);
             if (SHAPES && rec_type(r) == REC_CURVE) costly = true;
             Hit h;
@@ -1724,7 +1789,7 @@ __global__ void __launch_bounds__(128, MEDIA ? FTB_SHADE_MEDIA_MINB : FTB_SHADE_
                 h.prim = r.prim;
             } else {
                 RayCtx R = make_ray(ro, rd);
-                hit_attributes<SHAPES>(sc.tri_n, R, r, h);
+                hit_attributes<SHAPES>(sc.tri_n, R, sc.recs, rec, r, h);
             }
             const DevMat& m = sc.mats[h.mat];
             switch (m.type) {
@@ -1935,7 +2000,7 @@ __device__ __forceinline__ bool mirror_seen(const DevJob& J, const Wave& w, cons
     const int rec = traverse_closest<COUNT, INST, SHAPES>(sc, make_ray(eye, wE), EPS_RAY, t, &sub, f.status, cnt);
     if (rec < 0) return false;
     if (fabs(t - ms.dE) > 1e-4 * (1.0 + ms.dE)) return false;
-    PrimRec r;
+    Rec r;
     load_rec(sc.recs, rec, r);
     ms.mat = rec_mat(r);
     if (INST && rec_type(r) == REC_INST) {
@@ -2174,7 +2239,7 @@ __global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, cons
         if (!valid) {
             fate = 1;
         } else {
-            PrimRec r;
+            Rec r;
             load_rec(sc.recs, rec, r);
             if (SHAPES && rec_type(r) == REC_CURVE) costly = true;
             Hit h;
@@ -2183,7 +2248,7 @@ __global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, cons
                 h.prim = r.prim;
             } else {
                 RayCtx R = make_ray(ro, rd);
-                hit_attributes<SHAPES>(sc.tri_n, R, r, h);
+                hit_attributes<SHAPES>(sc.tri_n, R, sc.recs, rec, r, h);
             }
             const DevMat& m = sc.mats[h.mat];
             switch (m.type) {

@@ -7,10 +7,11 @@
 //             float grid (p, 2^e), rounded outward, so the fp32 traversal never culls a
 //             primitive the exact fp64 test would accept); the upload widens each to an
 //             FNode holding the float planes that the bytes decode to.
-//   recs    : PrimRec[n_recs], 80 B each -- one record per primitive, in leaf order.
+//   recs    : PrimRec[n_recs], 96 B each -- one record per primitive, in leaf order.
 //             Triangles keep their three vertices in double (the exact watertight test
-//             reads them); the last 8 B carry the global primitive index, material and
-//             type.  Leaf children of a node reference a contiguous run of records.
+//             reads them); the last 8 B of each row carry the global primitive index,
+//             material and type.  Leaf children of a node reference a contiguous run of
+//             records.
 //   tri_n   : optional per-triangle shading normals (9 doubles), by triangle index.
 //   planes  : DevPlane[n_planes] -- the planar mirrors the camera connections reflect in.
 //   inst    : DevInst[n_inst], 128 B each -- instances of shared BLAS assets.  The world
@@ -63,15 +64,17 @@ struct alignas(32) FNode {
 static_assert(sizeof(FNode) == 224, "FNode must be 224 bytes");
 #define FNODE_INNER 7u
 
-// 80-byte primitive record.  d[9] holds two int32: prim (global index) and
-// info = mat | type << 24 | smooth << 30.  An instance record (REC_INST) keeps its instance
-// index in d[0] (as an int64 bit pattern); a BLAS triangle's prim is its index in the BLAS.
-struct alignas(16) PrimRec {
-    double d[9];
-    int32_t prim;
-    int32_t info;
+// 96-byte primitive record: three rows of four doubles, one 32-byte sector each.  A triangle
+// keeps coordinate a of its vertices v0, v1, v2 in row a, so the watertight test loads its
+// rows in the ray's axis order (kx, ky, kz) and permutes nothing; a sphere is {center},
+// {radius}; a round cone {p0}, {p1}, {r0, r1}; an instance record (REC_INST) keeps its
+// instance index in row 0 (as an int64 bit pattern).  Every row ends in the record's tail:
+// prim (global index; a BLAS triangle's is its index in the BLAS) in the low half, info =
+// mat | type << 24 | smooth << 30 in the high half.
+struct alignas(32) PrimRec {
+    double row[3][4];
 };
-static_assert(sizeof(PrimRec) == 80, "PrimRec must be 80 bytes");
+static_assert(sizeof(PrimRec) == 96, "PrimRec must be 96 bytes");
 
 struct DevSpec {
     int32_t kind, n;
