@@ -90,7 +90,7 @@ struct Wave {
     int32_t* hit_sub;          // BLAS record when hit_rec is an instance
     int32_t* perm;             // optional traversal order of a queue (bucketed by direction)
     int32_t* counts;           // [2a], [2a+1]: the two ends of the queue in ps[a]; [4] shadow records;
-                               // [5..7] per-launch work counters
+                               // [5..7] per-launch work counters (kFetch*)
     int32_t* sjob;             // job of each shadow record
     DevJob* jobs;              // device job table, kWaveJobs entries
     int32_t* params;           // [0] jobs in the table, [1] paths in flight at most (written with
@@ -119,11 +119,12 @@ struct Frame {
 };
 
 // Queue counts of path buffer a (front and back end), the shadow-record count and the
-// per-launch work counters of the closest-hit, shading and shadow kernels in Wave::counts
-// ([4] .. [4 + kCountWords - 1] are cleared together after every connection launch).
-constexpr int kShadowCount = 4;
-constexpr int kFetchExtend = 5, kFetchShade = 6, kFetchShadow = 7;
-constexpr int kCountWords = 4;
+// per-launch work counters of the shadow, closest-hit and shading kernels in Wave::counts.
+// The connection words [4], [5] are cleared after a connection launch, the other two after
+// shading: a streaming pass runs a connection launch beside the next closest-hit launch.
+constexpr int kShadowCount = 4, kFetchShadow = 5, kShadowWords = 2;
+constexpr int kFetchExtend = 6, kFetchShade = 7;
+constexpr int kCountWords = 4;   // all of [4] .. [7]
 inline int32_t* queue_counts(const Wave& w, int a) { return w.counts + 2 * a; }
 
 // Shadow records per path: a path queues at most 2 connections per view per bounce, and in
@@ -213,9 +214,10 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
 // Trace a streaming pass on `stream`: the caller has written the table of photon ranges to
 // w.jobs (g0 consecutive from 0) and w.params = {ranges, slots, photons (int64 at [1]),
 // half-iteration cap (int64 at [2])}.  The pass keeps up to `slots` paths in flight: every
-// half-iteration runs closest hit, shading (the survivors are compacted into the other
-// path buffer), a refill that appends the next photons of the pass up to `slots` paths,
-// and the queued connections, until every photon is done.  With `graphs` and shape.graph the loop is one
+// half-iteration runs closest hit beside the connections queued so far, shading (the
+// survivors are compacted into the other path buffer) and a refill that appends the next
+// photons of the pass up to `slots` paths, until every photon is done; then the last
+// connections.  With `graphs` and shape.graph the loop is one
 // graph launch (a conditional while node whose condition the device sets); otherwise the
 // host issues half-iterations in groups and reads the progress word between groups.
 cudaError_t launch_stream(Wave& w, const WaveKind& kind, const Frame& f, int32_t sms, const LaunchShape& shape,
