@@ -734,12 +734,14 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
                     const std::vector<uint64_t>& seed, bool log, ftb_photon_log* d_logs, int64_t log_base,
                     cudaStream_t user_stream) {
     int64_t total = 0;
-    int32_t hero = 1;
+    int32_t hero = 1, fanout = 1;
     for (size_t i = 0; i < count.size(); ++i) {
         total += count[i];
         hero = std::max(hero, base[i].hero_c);
+        fanout = std::max(fanout, ftb::conn_fanout(base[i]));
     }
-    int32_t W = pick_wave(total, s->eng->wave_cap);
+    // a pass keeps W / fanout paths in flight, so few photons of a large fan-out get more room
+    int32_t W = pick_wave(std::min<int64_t>(total, s->eng->wave_cap) * fanout, s->eng->wave_cap);
     ftb_status st = ensure_waves(s, W, log, hero);   // may keep larger buffers; waves use W slots
     if (st != FTB_OK) return st;
     ftb::Frame f;
@@ -805,7 +807,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
-        e = ftb::launch_stream(w, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
+        e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                s->eng->graphs[k & 1]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
         ++k;

@@ -56,6 +56,9 @@ namespace cg = cooperative_groups;
 #ifndef FTB_SHADE_MINB
 #define FTB_SHADE_MINB 8
 #endif
+#ifndef FTB_TRACE_MINB         // whole paths: registers for traversal and shading at once
+#define FTB_TRACE_MINB 4
+#endif
 #ifndef FTB_SHADE_MEDIA_MINB   // shading with participating media: more registers pay off
 #define FTB_SHADE_MEDIA_MINB 4
 #endif
@@ -1081,16 +1084,42 @@ __device__ __forceinline__ int queue_entry(const Wave& w, int front, int p) {
 
 // A one-wavelength connection: the film increments cieX/Y/Z(lambda) * contribution in the
 // order Film::add forms them (scene_film.h:12), from the matching functions evaluated once
-// per path at emission.
-__device__ __forceinline__ void push_shadow(const Wave& w, const Frame& f, int job, int view, D3 o, D3 d,
-                                            double tmax, double val, const double* cie, int pix) {
+// per path at emission.  Returns false when the connection queue is full.
+__device__ __forceinline__ bool queue_shadow(const Wave& w, int job, int view, D3 o, D3 d, double tmax, double val,
+                                             const double* cie, int pix) {
     int i = agg_inc(&w.counts[kShadowCount]);
-    if (i >= w.S) { atomicOr(f.status, ST_QUEUE_OVERFLOW); return; }
+    if (i >= w.S) return false;
     w.sox[i] = o.x; w.soy[i] = o.y; w.soz[i] = o.z;
     w.sdx[i] = d.x; w.sdy[i] = d.y; w.sdz[i] = d.z;
     w.smax[i] = tmax; w.spix[i] = pix;
     w.sxyz[i] = cie[0] * val; w.sxyz[w.S + i] = cie[1] * val; w.sxyz[2 * (size_t)w.S + i] = cie[2] * val;
     w.sjob[i] = job; w.sview[i] = view;
+    return true;
+}
+
+// Where a kernel's connections go.  WaveQueue: the wave's connection queue, sized so that a
+// launch cannot overfill it (else a status bit fails the render).  PathQueue: the same queue,
+// but a path traced to its end in one launch may queue any number of connections, so one that
+// finds the queue full is tested and splatted on the spot.
+struct WaveQueue {
+    const Wave& w;
+};
+template <bool INST, bool SHAPES>
+struct PathQueue {
+    const Wave& w;
+};
+template <bool INST, bool SHAPES>
+__device__ __noinline__ void connect_now(const DevJob& J, const Frame& f, int view, D3 o, D3 d, double tmax, double X,
+                                         double Y, double Z, int pix);
+__device__ __forceinline__ void push_shadow(const WaveQueue& q, const DevJob&, const Frame& f, int job, int view, D3 o,
+                                            D3 d, double tmax, double val, const double* cie, int pix) {
+    if (!queue_shadow(q.w, job, view, o, d, tmax, val, cie, pix)) atomicOr(f.status, ST_QUEUE_OVERFLOW);
+}
+template <bool INST, bool SHAPES>
+__device__ __forceinline__ void push_shadow(const PathQueue<INST, SHAPES>& q, const DevJob& J, const Frame& f, int job,
+                                            int view, D3 o, D3 d, double tmax, double val, const double* cie, int pix) {
+    if (!queue_shadow(q.w, job, view, o, d, tmax, val, cie, pix))
+        connect_now<INST, SHAPES>(J, f, view, o, d, tmax, cie[0] * val, cie[1] * val, cie[2] * val, pix);
 }
 
 // The views a job's vertices connect to: its own camera, or every view of a multi-camera job.
@@ -1104,8 +1133,8 @@ __device__ __forceinline__ int64_t* view_film(const DevJob& J, int v) {
 
 // connectGeom + connect, model B (render.h:499-559); the occlusion test is deferred to
 // k_shadow, the rest of the contribution is formed here in the reference's order.
-template <bool MEDIA>
-__device__ void connect_surface(const DevScene& sc, const DevJob& J, const Wave& w, const Frame& f, int job,
+template <bool MEDIA, class Q>
+__device__ void connect_surface(const DevScene& sc, const DevJob& J, const Q& w, const Frame& f, int job,
                                 D3 p, D3 n, D3 ng, D3 wi, double lam, const double* cie, double beta, double rho) {
     for (int v = 0; v < view_count(J); ++v) {
         const DevCam& cam = view_cam(J, v);
@@ -1124,11 +1153,12 @@ __device__ void connect_surface(const DevScene& sc, const DevJob& J, const Wave&
         double fr = rho / PI_D;
         double contrib = beta * fr * cos_surf * corr / denom * stg;
         if (MEDIA && sc.n_med > 0) contrib *= media_transmittance(sc, p, wdir, dist, lam);
-        push_shadow(w, f, job, v, p + ng * 1e-6, wdir, dist - 2e-6, contrib, cie, py * cam.rx + px);
+        push_shadow(w, J, f, job, v, p + ng * 1e-6, wdir, dist - 2e-6, contrib, cie, py * cam.rx + px);
     }
 }
 // connectVolume (render.h:584-600)
-__device__ void connect_volume(const DevScene& sc, const DevJob& J, const Wave& w, const Frame& f, int job,
+template <class Q>
+__device__ void connect_volume(const DevScene& sc, const DevJob& J, const Q& w, const Frame& f, int job,
                                const DevMed& m, D3 p, D3 win, double lam, const double* cie, double beta) {
     for (int v = 0; v < view_count(J); ++v) {
         const DevCam& cam = view_cam(J, v);
@@ -1142,7 +1172,7 @@ __device__ void connect_volume(const DevScene& sc, const DevJob& J, const Wave& 
         double omega = cam_pixel_solid_angle(cam, cos_cam);
         double contrib = beta * alb * ph / (dist2 * omega);
         contrib *= media_transmittance(sc, p, wdir, dist, lam);
-        push_shadow(w, f, job, v, p + wdir * 1e-6, wdir, dist - 2e-6, contrib, cie, py * cam.rx + px);
+        push_shadow(w, J, f, job, v, p + wdir * 1e-6, wdir, dist - 2e-6, contrib, cie, py * cam.rx + px);
     }
 }
 
@@ -1152,16 +1182,32 @@ __device__ void connect_volume(const DevScene& sc, const DevJob& J, const Wave& 
 // the origin / direction / max fields, view | plane << 16, the wavelength, the vertex factor
 // beta * (weight * shape) and cieX/Y/Z(lambda) in place of the film increments -- the
 // mirror's reflectance is known only once k_shadow has seen which mirror the eye meets.
-__device__ __forceinline__ void push_mirror(const Wave& w, const Frame& f, int job, int view, int plane, D3 p, D3 wP,
-                                            double dP, double a, double lam, const double* cie, int pix) {
+__device__ __forceinline__ bool queue_mirror(const Wave& w, int job, int view, int plane, D3 p, D3 wP, double dP,
+                                             double a, double lam, const double* cie, int pix) {
     int i = agg_inc(&w.counts[kShadowCount]);
-    if (i >= w.S) { atomicOr(f.status, ST_QUEUE_OVERFLOW); return; }
+    if (i >= w.S) return false;
     w.sox[i] = p.x; w.soy[i] = p.y; w.soz[i] = p.z;
     w.sdx[i] = wP.x; w.sdy[i] = wP.y; w.sdz[i] = wP.z;
     w.smax[i] = dP; w.spix[i] = ~pix;
     w.sval[i] = a; w.slam[i] = lam;
     w.sxyz[i] = cie[0]; w.sxyz[w.S + i] = cie[1]; w.sxyz[2 * (size_t)w.S + i] = cie[2];
     w.sjob[i] = job; w.sview[i] = view | (plane << 16);
+    return true;
+}
+template <bool INST, bool SHAPES>
+__device__ __noinline__ void mirror_now(const DevJob& J, const Frame& f, int view, int plane, D3 p, D3 wP, double dP,
+                                        double a, double lam, double X, double Y, double Z, int pix);
+__device__ __forceinline__ void push_mirror(const WaveQueue& q, const DevJob&, const Frame& f, int job, int view,
+                                            int plane, D3 p, D3 wP, double dP, double a, double lam, const double* cie,
+                                            int pix) {
+    if (!queue_mirror(q.w, job, view, plane, p, wP, dP, a, lam, cie, pix)) atomicOr(f.status, ST_QUEUE_OVERFLOW);
+}
+template <bool INST, bool SHAPES>
+__device__ __forceinline__ void push_mirror(const PathQueue<INST, SHAPES>& q, const DevJob& J, const Frame& f, int job,
+                                            int view, int plane, D3 p, D3 wP, double dP, double a, double lam,
+                                            const double* cie, int pix) {
+    if (!queue_mirror(q.w, job, view, plane, p, wP, dP, a, lam, cie, pix))
+        mirror_now<INST, SHAPES>(J, f, view, plane, p, wP, dP, a, lam, cie[0], cie[1], cie[2], pix);
 }
 
 // connectSpecularPlane's geometry (render.h:1334-1366) for one plane and view: the vertex and
@@ -1206,39 +1252,15 @@ __device__ __forceinline__ bool mirror_geometry(const DevPlane& mp, const DevCam
 // camSpecularSplatAll / camSpecularSplatVolumeAll (render.h:1515-1585) over the planar
 // mirrors: a mirror record for k_shadow per plane and view that the geometry lets through.
 // `weight`: the vertex's albedo.
-__device__ __noinline__ void connect_mirrors(const DevScene& sc, const DevJob& J, const Wave& w, const Frame& f,
+template <class Q>
+__device__ __noinline__ void connect_mirrors(const DevScene& sc, const DevJob& J, const Q& w, const Frame& f,
                                              int job, D3 p, bool volume, D3 nw, double g, double lam,
                                              const double* cie, double beta, double weight) {
     for (int k = 0; k < sc.n_planes; ++k) {
         for (int v = 0; v < view_count(J); ++v) {
             D3 wP; double dP, shape; int pix;
             if (!mirror_geometry(sc.planes[k], view_cam(J, v), p, volume, nw, g, wP, dP, shape, pix)) continue;
-            push_mirror(w, f, job, v, k, p, wP, dP, beta * (weight * shape), lam, cie, pix);
-        }
-    }
-}
-
-// The same for a bundle's live wavelengths (camSpecularSplatAllHero, render.h:1570-1576): a
-// record carries (lambda_i, beta_i x (rho_i x shape)) per wavelength, as the bundle's camera
-// connections do; k_shadow_hero evaluates the mirror's reflectance per wavelength.
-__device__ __noinline__ void connect_mirrors_hero(const DevScene& sc, const DevJob& J, const Wave& w, const Frame& f,
-                                                  int job, D3 p, D3 n, const double* lam, const double* beta,
-                                                  const double* rho, int nup) {
-    for (int k = 0; k < sc.n_planes; ++k) {
-        for (int v = 0; v < view_count(J); ++v) {
-            D3 wP; double dP, shape; int pix;
-            if (!mirror_geometry(sc.planes[k], view_cam(J, v), p, false, n, 0.0, wP, dP, shape, pix)) continue;
-            const int i = agg_inc(&w.counts[kShadowCount]);
-            if (i >= w.S) { atomicOr(f.status, ST_QUEUE_OVERFLOW); continue; }
-            w.sox[i] = p.x; w.soy[i] = p.y; w.soz[i] = p.z;
-            w.sdx[i] = wP.x; w.sdy[i] = wP.y; w.sdz[i] = wP.z;
-            w.smax[i] = dP; w.spix[i] = ~pix; w.sjob[i] = job; w.sview[i] = v | (k << 16);
-            w.slam[i] = lam[0]; w.sval[i] = beta[0] * (rho[0] * shape);
-            for (int q = 1; q < nup; ++q) {
-                w.xlam[(size_t)(q - 1) * w.S + i] = lam[q];
-                w.xval[(size_t)(q - 1) * w.S + i] = beta[q] * (rho[q] * shape);
-            }
-            w.snup[i] = nup;
+            push_mirror(w, J, f, job, v, k, p, wP, dP, beta * (weight * shape), lam, cie, pix);
         }
     }
 }
@@ -1532,8 +1554,8 @@ __global__ void __launch_bounds__(128, FTB_EMIT_MINB) k_emit(Wave w, const DevJo
         if (J.lambda_mode == FTB_LAMBDA_UNIFORM_380_780) beta *= wl;
         tally_add(acc, jobs, multi, j, T_EMIT, to_fixed(beta, J.tally_scale_inv, f.status));
         const double cie[3] = {cie_x(lam), cie_y(lam), cie_z(lam)};
-        connect_surface<MEDIA>(sc, J, w, f, j, origin, emit_n, emit_n, emit_n, lam, cie, beta, 1.0);
-        if (MIRROR && sc.n_planes > 0) connect_mirrors(sc, J, w, f, j, origin, false, emit_n, 0.0, lam, cie, beta, 1.0);
+        connect_surface<MEDIA>(sc, J, WaveQueue{w}, f, j, origin, emit_n, emit_n, emit_n, lam, cie, beta, 1.0);
+        if (MIRROR && sc.n_planes > 0) connect_mirrors(sc, J, WaveQueue{w}, f, j, origin, false, emit_n, 0.0, lam, cie, beta, 1.0);
         D3 ro = origin + dir * 1e-6;
         if (J.max_bounce <= 0) {
             tally_add(acc, jobs, multi, j, T_RES, to_fixed(beta, J.tally_scale_inv, f.status));
@@ -1719,7 +1741,162 @@ __device__ void refract_or_reflect(const DevScene& sc, const DevMat& m, const Hi
     d_out = out;
 }
 
-// One bounce of Renderer::tracePhoton's loop body (render.h:2013-2238).
+// One bounce of Renderer::tracePhoton's loop body (render.h:2013-2238): media, interior
+// absorption and the interaction at the closest hit (record rec at distance ht, BLAS record
+// sub), connections queued.  Returns -1 when the path goes on from (no, nd), 0 absorbed, 1
+// escaped; `costly`: the next ray starts among curves.  cie() yields the path's CIE values.
+template <bool MEDIA, bool INST, bool SHAPES, bool MIRROR, class Q, class Cie>
+__device__ __forceinline__ int shade_bounce(const DevScene& sc, const DevJob& J, const Q& w, const Frame& f, int j,
+                                            Pcg& rng, D3 ro, D3 rd, double lam, double& beta, Stk& stk, double ht,
+                                            int rec, int sub, const Cie& cie, D3& no, D3& nd, bool& costly) {
+    int fate = -1;
+    bool valid = rec >= 0;
+    double d_surf = valid ? ht : 1e30;
+    double d_event = d_surf;
+    bool medium_event = false;
+    int scatter_med = -1;
+    D3 mp = mk(0, 0, 0);
+    if (MEDIA && sc.n_med > 0) {
+        double tm; int which;
+        if (sample_media_collision(sc, ro, rd, d_surf, lam, rng, tm, which)) {
+            d_event = tm; medium_event = true; scatter_med = which; mp = ro + rd * tm;
+        }
+    }
+    {   // Beer-Lambert inside the current dielectric (render.h:2063-2066)
+        int mi = stk_top_mat(stk);
+        double a = (mi >= 0) ? spec_slot(sc, sc.mats[mi].absorb, lam, 0.0) : 0.0;
+        if (a > 0.0) beta *= exp(-a * d_event);
+    }
+    no = ro; nd = rd;
+    if (medium_event) {   // render.h:2105-2115
+        const DevMed& sm = sc.med[scatter_med];
+        connect_volume(sc, J, w, f, j, sm, mp, rd, lam, cie(), beta);
+        if (MIRROR && sc.n_planes > 0)
+            connect_mirrors(sc, J, w, f, j, mp, true, rd, sm.g, lam, cie(), beta, med_albedo(sc, sm, lam));
+        if (uniform(rng) >= med_albedo(sc, sm, lam)) fate = 0;
+        else { nd = sample_hg(rd, sm.g, rng); no = mp; }
+    } else if (!valid) {
+        fate = 1;
+    } else {
+        Rec r;
+        load_rec(sc.recs, rec, r);
+        if (SHAPES && rec_type(r) == REC_CURVE) costly = true;
+        Hit h;
+        if (INST && rec_type(r) == REC_INST) {
+            instance_hit(sc.inst[rec_inst(r)], sub, ro, rd, h);
+            h.prim = r.prim;
+        } else {
+            RayCtx R = make_ray(ro, rd);
+            hit_attributes<SHAPES>(sc.tri_n, R, sc.recs, rec, r, h);
+        }
+        const DevMat& m = sc.mats[h.mat];
+        switch (m.type) {
+        case FTB_MAT_DIELECTRIC: {   // render.h:1612-1660
+            bool entering = dot(rd, h.ng) < 0.0;
+            int mi = h.mat, pr = m.priority;
+            bool has_pri = pr != INT_MIN;
+            bool transmitted = false;
+            if (entering) {
+                int out_mat = stk_top_mat(stk), out_pri = stk_top_pri(stk);
+                bool ranked = has_pri && (stk.n == 0 || (out_mat >= 0 && sc.mats[out_mat].priority != INT_MIN));
+                if (ranked && stk.n != 0 && pr <= out_pri) {
+                    stk_push(stk, mi, pr, f.status);
+                    no = h.p + rd * 1e-6;
+                } else {
+                    double ext = (ranked && out_mat >= 0) ? mat_ior(sc, sc.mats[out_mat], lam) : 1.0;
+                    refract_or_reflect(sc, m, h, rd, lam, rng, transmitted, ext, no, nd);
+                    if (transmitted) stk_push(stk, mi, pr, f.status);
+                }
+            } else {
+                Stk after = stk;
+                stk_pop_mat(after, mi);
+                int new_mat = stk_top_mat(after), new_pri = stk_top_pri(after);
+                bool ranked = has_pri && (after.n == 0 || (new_mat >= 0 && sc.mats[new_mat].priority != INT_MIN));
+                if (ranked && new_mat >= 0 && pr <= new_pri) {
+                    stk_pop_mat(stk, mi);
+                    no = h.p + rd * 1e-6;
+                } else {
+                    double ext = (ranked && new_mat >= 0) ? mat_ior(sc, sc.mats[new_mat], lam) : 1.0;
+                    refract_or_reflect(sc, m, h, rd, lam, rng, transmitted, ext, no, nd);
+                    if (transmitted) stk_pop_mat(stk, mi);
+                }
+            }
+            break;
+        }
+        case FTB_MAT_GLOSSY: {   // render.h:1725-1733
+            double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
+            if (uniform(rng) >= rr) { fate = 0; break; }
+            D3 o = sample_glossy(reflect(rd, h.n), m.roughness, rng);
+            if (dot(o, h.n) <= 0) { fate = 0; break; }
+            no = h.p + h.n * 1e-6; nd = o;
+            break;
+        }
+        case FTB_MAT_MIRROR: {   // render.h:1680-1688
+            double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
+            if (uniform(rng) >= rr) { fate = 0; break; }
+            nd = reflect(rd, h.n);
+            no = h.p + h.n * 1e-6;
+            break;
+        }
+        case FTB_MAT_HALF_MIRROR: {   // render.h:1702-1711
+            double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
+            if (uniform(rng) < rr) {
+                nd = reflect(rd, h.n);
+                no = h.p + h.n * 1e-6;
+            } else {
+                no = h.p + rd * 1e-6;
+            }
+            break;
+        }
+        case FTB_MAT_FILTER: {   // render.h:1711-1723
+            double tt = clamp01(spec_slot(sc, m.transmit, lam, 0.0));
+            if (uniform(rng) >= tt) { fate = 0; break; }
+            no = h.p + rd * 1e-6;
+            break;
+        }
+        case FTB_MAT_DIFFUSE_TRANSMIT: {   // render.h:2180-2212
+            double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
+            double rt = clamp01(spec_slot(sc, m.transmit, lam, 0.0));
+            double sum = rr + rt;
+            if (sum > 1.0) { rr /= sum; rt /= sum; sum = 1.0; }
+            D3 ngo = oriented_geo_n(h);
+            D3 wi = mk(-rd.x, -rd.y, -rd.z);
+            connect_surface<MEDIA>(sc, J, w, f, j, h.p, h.n, ngo, wi, lam, cie(), beta, rr);
+            connect_surface<MEDIA>(sc, J, w, f, j, h.p, neg(h.n), neg(ngo), wi, lam, cie(), beta, rt);
+            if (MIRROR && sc.n_planes > 0) {
+                connect_mirrors(sc, J, w, f, j, h.p, false, h.n, 0.0, lam, cie(), beta, rr);
+                connect_mirrors(sc, J, w, f, j, h.p, false, neg(h.n), 0.0, lam, cie(), beta, rt);
+            }
+            double u = uniform(rng);
+            if (u < rr) {
+                D3 wo = cosine_hemisphere(h.n, rng);
+                beta *= shading_adjoint_corr(wi, wo, h.n, ngo);
+                no = h.p + h.n * 1e-6; nd = wo;
+            } else if (u < sum) {
+                D3 wo = cosine_hemisphere(mk(-h.n.x, -h.n.y, -h.n.z), rng);
+                beta *= shading_adjoint_corr(wi, wo, h.n, ngo);
+                no = h.p - h.n * 1e-6; nd = wo;
+            } else fate = 0;
+            break;
+        }
+        default: {   // Diffuse (render.h:2215-2236)
+            double rho = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
+            D3 ngo = oriented_geo_n(h);
+            D3 wi = mk(-rd.x, -rd.y, -rd.z);
+            connect_surface<MEDIA>(sc, J, w, f, j, h.p, h.n, ngo, wi, lam, cie(), beta, rho);
+            if (MIRROR && sc.n_planes > 0) connect_mirrors(sc, J, w, f, j, h.p, false, h.n, 0.0, lam, cie(), beta, rho);
+            if (uniform(rng) >= rho) { fate = 0; break; }
+            D3 wo = cosine_hemisphere(h.n, rng);
+            beta *= shading_adjoint_corr(wi, wo, h.n, ngo);
+            no = h.p + h.n * 1e-6; nd = wo;
+            break;
+        }
+        }
+    }
+    return fate;
+}
+
+// One bounce of every queued path; the survivors are copied into the other path buffer.
 template <bool MEDIA, bool INST, bool SHAPES, bool MIRROR>
 __global__ void __launch_bounds__(128, MEDIA ? FTB_SHADE_MEDIA_MINB : FTB_SHADE_MINB) k_shade(Wave w, const DevJob* __restrict__ jobs,
                                                                Frame f, PathState in, const int32_t* in_count,
@@ -1739,164 +1916,21 @@ __global__ void __launch_bounds__(128, MEDIA ? FTB_SHADE_MEDIA_MINB : FTB_SHADE_
         double lam = in.lam[i], beta = in.beta[i];
         double cie[3];   // read by the paths that connect or survive
         bool have_cie = false;
-        auto load_cie = [&]() {
-            if (have_cie) return;
+        auto load_cie = [&]() -> const double* {
+            if (have_cie) return cie;
             cie[0] = in.cie[i]; cie[1] = in.cie[w.W + i]; cie[2] = in.cie[2 * (size_t)w.W + i];
             have_cie = true;
+            return cie;
         };
         double ht = w.hit_t[i];
         int rec = w.hit_rec[i];
         Stk stk; stk.n = in.stk_n[i];
         for (int k = 0; k < stk.n; ++k) stk.e[k] = in.stk[k * w.W + i];
         log_hit<INST>(w, in, i, sc, rec);
-        int fate = -1;   // -1 continue, 0 absorbed, 1 escaped
-        bool costly = false;   // the next ray starts among curves: back end of the queue
-        bool valid = rec >= 0;
-        double d_surf = valid ? ht : 1e30;
-        double d_event = d_surf;
-        bool medium_event = false;
-        int scatter_med = -1;
-        D3 mp = mk(0, 0, 0);
-        if (MEDIA && sc.n_med > 0) {
-            double tm; int which;
-            if (sample_media_collision(sc, ro, rd, d_surf, lam, rng, tm, which)) {
-                d_event = tm; medium_event = true; scatter_med = which; mp = ro + rd * tm;
-            }
-        }
-        {   // Beer-Lambert inside the current dielectric (render.h:2063-2066)
-            int mi = stk_top_mat(stk);
-            double a = (mi >= 0) ? spec_slot(sc, sc.mats[mi].absorb, lam, 0.0) : 0.0;
-            if (a > 0.0) beta *= exp(-a * d_event);
-        }
-        D3 no = ro, nd = rd;
-        if (medium_event) {   // render.h:2105-2115
-            const DevMed& sm = sc.med[scatter_med];
-            load_cie();
-            connect_volume(sc, J, w, f, j, sm, mp, rd, lam, cie, beta);
-            if (MIRROR && sc.n_planes > 0)
-                connect_mirrors(sc, J, w, f, j, mp, true, rd, sm.g, lam, cie, beta, med_albedo(sc, sm, lam));
-            if (uniform(rng) >= med_albedo(sc, sm, lam)) fate = 0;
-            else { nd = sample_hg(rd, sm.g, rng); no = mp; }
-        } else if (!valid) {
-            fate = 1;
-        } else {
-            Rec r;
-            load_rec(sc.recs, rec, r);
-            if (SHAPES && rec_type(r) == REC_CURVE) costly = true;
-            Hit h;
-            if (INST && rec_type(r) == REC_INST) {
-                instance_hit(sc.inst[rec_inst(r)], w.hit_sub[i], ro, rd, h);
-                h.prim = r.prim;
-            } else {
-                RayCtx R = make_ray(ro, rd);
-                hit_attributes<SHAPES>(sc.tri_n, R, sc.recs, rec, r, h);
-            }
-            const DevMat& m = sc.mats[h.mat];
-            switch (m.type) {
-            case FTB_MAT_DIELECTRIC: {   // render.h:1612-1660
-                bool entering = dot(rd, h.ng) < 0.0;
-                int mi = h.mat, pr = m.priority;
-                bool has_pri = pr != INT_MIN;
-                bool transmitted = false;
-                if (entering) {
-                    int out_mat = stk_top_mat(stk), out_pri = stk_top_pri(stk);
-                    bool ranked = has_pri && (stk.n == 0 || (out_mat >= 0 && sc.mats[out_mat].priority != INT_MIN));
-                    if (ranked && stk.n != 0 && pr <= out_pri) {
-                        stk_push(stk, mi, pr, f.status);
-                        no = h.p + rd * 1e-6;
-                    } else {
-                        double ext = (ranked && out_mat >= 0) ? mat_ior(sc, sc.mats[out_mat], lam) : 1.0;
-                        refract_or_reflect(sc, m, h, rd, lam, rng, transmitted, ext, no, nd);
-                        if (transmitted) stk_push(stk, mi, pr, f.status);
-                    }
-                } else {
-                    Stk after = stk;
-                    stk_pop_mat(after, mi);
-                    int new_mat = stk_top_mat(after), new_pri = stk_top_pri(after);
-                    bool ranked = has_pri && (after.n == 0 || (new_mat >= 0 && sc.mats[new_mat].priority != INT_MIN));
-                    if (ranked && new_mat >= 0 && pr <= new_pri) {
-                        stk_pop_mat(stk, mi);
-                        no = h.p + rd * 1e-6;
-                    } else {
-                        double ext = (ranked && new_mat >= 0) ? mat_ior(sc, sc.mats[new_mat], lam) : 1.0;
-                        refract_or_reflect(sc, m, h, rd, lam, rng, transmitted, ext, no, nd);
-                        if (transmitted) stk_pop_mat(stk, mi);
-                    }
-                }
-                break;
-            }
-            case FTB_MAT_GLOSSY: {   // render.h:1725-1733
-                double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
-                if (uniform(rng) >= rr) { fate = 0; break; }
-                D3 o = sample_glossy(reflect(rd, h.n), m.roughness, rng);
-                if (dot(o, h.n) <= 0) { fate = 0; break; }
-                no = h.p + h.n * 1e-6; nd = o;
-                break;
-            }
-            case FTB_MAT_MIRROR: {   // render.h:1680-1688
-                double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
-                if (uniform(rng) >= rr) { fate = 0; break; }
-                nd = reflect(rd, h.n);
-                no = h.p + h.n * 1e-6;
-                break;
-            }
-            case FTB_MAT_HALF_MIRROR: {   // render.h:1702-1711
-                double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
-                if (uniform(rng) < rr) {
-                    nd = reflect(rd, h.n);
-                    no = h.p + h.n * 1e-6;
-                } else {
-                    no = h.p + rd * 1e-6;
-                }
-                break;
-            }
-            case FTB_MAT_FILTER: {   // render.h:1711-1723
-                double tt = clamp01(spec_slot(sc, m.transmit, lam, 0.0));
-                if (uniform(rng) >= tt) { fate = 0; break; }
-                no = h.p + rd * 1e-6;
-                break;
-            }
-            case FTB_MAT_DIFFUSE_TRANSMIT: {   // render.h:2180-2212
-                double rr = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
-                double rt = clamp01(spec_slot(sc, m.transmit, lam, 0.0));
-                double sum = rr + rt;
-                if (sum > 1.0) { rr /= sum; rt /= sum; sum = 1.0; }
-                D3 ngo = oriented_geo_n(h);
-                D3 wi = mk(-rd.x, -rd.y, -rd.z);
-                load_cie();
-                connect_surface<MEDIA>(sc, J, w, f, j, h.p, h.n, ngo, wi, lam, cie, beta, rr);
-                connect_surface<MEDIA>(sc, J, w, f, j, h.p, neg(h.n), neg(ngo), wi, lam, cie, beta, rt);
-                if (MIRROR && sc.n_planes > 0) {
-                    connect_mirrors(sc, J, w, f, j, h.p, false, h.n, 0.0, lam, cie, beta, rr);
-                    connect_mirrors(sc, J, w, f, j, h.p, false, neg(h.n), 0.0, lam, cie, beta, rt);
-                }
-                double u = uniform(rng);
-                if (u < rr) {
-                    D3 wo = cosine_hemisphere(h.n, rng);
-                    beta *= shading_adjoint_corr(wi, wo, h.n, ngo);
-                    no = h.p + h.n * 1e-6; nd = wo;
-                } else if (u < sum) {
-                    D3 wo = cosine_hemisphere(mk(-h.n.x, -h.n.y, -h.n.z), rng);
-                    beta *= shading_adjoint_corr(wi, wo, h.n, ngo);
-                    no = h.p - h.n * 1e-6; nd = wo;
-                } else fate = 0;
-                break;
-            }
-            default: {   // Diffuse (render.h:2215-2236)
-                double rho = clamp01(spec_slot(sc, m.reflect, lam, 0.5));
-                D3 ngo = oriented_geo_n(h);
-                D3 wi = mk(-rd.x, -rd.y, -rd.z);
-                load_cie();
-                connect_surface<MEDIA>(sc, J, w, f, j, h.p, h.n, ngo, wi, lam, cie, beta, rho);
-                if (MIRROR && sc.n_planes > 0) connect_mirrors(sc, J, w, f, j, h.p, false, h.n, 0.0, lam, cie, beta, rho);
-                if (uniform(rng) >= rho) { fate = 0; break; }
-                D3 wo = cosine_hemisphere(h.n, rng);
-                beta *= shading_adjoint_corr(wi, wo, h.n, ngo);
-                no = h.p + h.n * 1e-6; nd = wo;
-                break;
-            }
-            }
-        }
+        bool costly = false;
+        D3 no, nd;
+        const int fate = shade_bounce<MEDIA, INST, SHAPES, MIRROR>(sc, J, WaveQueue{w}, f, j, rng, ro, rd, lam, beta, stk, ht, rec,
+                                                                   INST ? w.hit_sub[i] : -1, load_cie, no, nd, costly);
         if (fate == 0) {
             tally_add(acc, jobs, multi, j, T_ABS, to_fixed(beta, J.tally_scale_inv, f.status));
             log_finish(w, in, i, 0, beta);
@@ -1974,14 +2008,11 @@ struct MirrorSeen {
     D3 R, wRE;
 };
 template <bool COUNT, bool INST, bool SHAPES>
-__device__ __forceinline__ bool mirror_seen(const DevJob& J, const Wave& w, const Frame& f, int i, TravCount& cnt,
-                                            MirrorSeen& ms) {
+__device__ __forceinline__ bool mirror_seen(const DevJob& J, const Frame& f, int view, int plane, D3 p, D3 wP,
+                                            double dP, TravCount& cnt, MirrorSeen& ms) {
     const DevScene& sc = J.sc;
-    const int view = w.sview[i] & 0xffff, plane = w.sview[i] >> 16;
     const DevPlane& mp = sc.planes[plane];
     const D3 pn = ld3(mp.n);
-    const D3 p = mk(w.sox[i], w.soy[i], w.soz[i]), wP = mk(w.sdx[i], w.sdy[i], w.sdz[i]);
-    const double dP = w.smax[i];
     {
         const RayCtx L = make_ray(p + wP * 1e-6, wP);
         if (traverse_any<COUNT, INST, SHAPES>(sc, L, EPS_RAY, (dP - 2e-6) - EPS_RAY, f.status, cnt)) return false;
@@ -2019,22 +2050,43 @@ __device__ __forceinline__ bool mirror_seen(const DevJob& J, const Wave& w, cons
 // the mirror the eye sees: (beta * (weight * shape)) * refl / (D^2 Omega), times the two legs'
 // transmittance in media.
 template <bool COUNT, bool INST, bool SHAPES>
-__device__ __noinline__ void mirror_splat(const DevJob& J, const Wave& w, const Frame& f, int i, TravCount& cnt) {
+__device__ __forceinline__ void mirror_splat(const DevJob& J, const Frame& f, int view, int plane, D3 p, D3 wP, double dP,
+                                             double a, double lam, double X, double Y, double Z, int pix,
+                                             TravCount& cnt) {
     MirrorSeen ms;
-    if (!mirror_seen<COUNT, INST, SHAPES>(J, w, f, i, cnt, ms)) return;
+    if (!mirror_seen<COUNT, INST, SHAPES>(J, f, view, plane, p, wP, dP, cnt, ms)) return;
     const DevScene& sc = J.sc;
     const double inv_d2_omega = 1.0 / (ms.D * ms.D * ms.omega);
-    const double lam = w.slam[i];
     const double refl = clamp01(spec_slot(sc, sc.mats[ms.mat].reflect, lam, 0.5));
-    double contrib = w.sval[i] * refl * inv_d2_omega;
+    double contrib = a * refl * inv_d2_omega;
     if (contrib <= 0.0) return;
     if (sc.n_med > 0) {
-        const D3 p = mk(w.sox[i], w.soy[i], w.soz[i]), wP = mk(w.sdx[i], w.sdy[i], w.sdz[i]);
-        contrib *= media_transmittance(sc, p, wP, w.smax[i], lam);
+        contrib *= media_transmittance(sc, p, wP, dP, lam);
         contrib *= media_transmittance(sc, ms.R, ms.wRE, ms.dE, lam);
     }
-    splat(J, w.sview[i] & 0xffff, ~w.spix[i], w.sxyz[i] * contrib, w.sxyz[w.S + i] * contrib,
-          w.sxyz[2 * (size_t)w.S + i] * contrib, f.status);
+    splat(J, view, pix, X * contrib, Y * contrib, Z * contrib, f.status);
+}
+template <bool COUNT, bool INST, bool SHAPES>
+__device__ __noinline__ void mirror_record(const DevJob& J, const Wave& w, const Frame& f, int i, TravCount& cnt) {
+    mirror_splat<COUNT, INST, SHAPES>(J, f, w.sview[i] & 0xffff, w.sview[i] >> 16, mk(w.sox[i], w.soy[i], w.soz[i]),
+                                      mk(w.sdx[i], w.sdy[i], w.sdz[i]), w.smax[i], w.sval[i], w.slam[i], w.sxyz[i],
+                                      w.sxyz[w.S + i], w.sxyz[2 * (size_t)w.S + i], ~w.spix[i], cnt);
+}
+
+// A connection that found the queue full: the same test and splat, by the lane that made it.
+template <bool INST, bool SHAPES>
+__device__ __noinline__ void connect_now(const DevJob& J, const Frame& f, int view, D3 o, D3 d, double tmax, double X,
+                                         double Y, double Z, int pix) {
+    TravCount cnt{0, 0, 0};
+    const RayCtx R = make_ray(o, d);
+    if (traverse_any<false, INST, SHAPES>(J.sc, R, EPS_RAY, tmax - EPS_RAY, f.status, cnt)) return;
+    splat(J, view, pix, X, Y, Z, f.status);
+}
+template <bool INST, bool SHAPES>
+__device__ __noinline__ void mirror_now(const DevJob& J, const Frame& f, int view, int plane, D3 p, D3 wP, double dP,
+                                        double a, double lam, double X, double Y, double Z, int pix) {
+    TravCount cnt{0, 0, 0};
+    mirror_splat<false, INST, SHAPES>(J, f, view, plane, p, wP, dP, a, lam, X, Y, Z, pix, cnt);
 }
 
 // Camera connections: occlusion (Scene::occluded, default tmin 1e-6) then Film::add.
@@ -2052,7 +2104,7 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow(Wave w, const Dev
         const DevScene& sc = J.sc;
         if (COUNT) rays++;
         if (MIRROR && w.spix[i] < 0) {
-            mirror_splat<COUNT, INST, SHAPES>(J, w, f, i, cnt);
+            mirror_record<COUNT, INST, SHAPES>(J, w, f, i, cnt);
             continue;
         }
         D3 o = mk(w.sox[i], w.soy[i], w.soz[i]), d = mk(w.sdx[i], w.sdy[i], w.sdz[i]);
@@ -2078,10 +2130,12 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow(Wave w, const Dev
 // in scenes without media, and so does this path (the host sends such jobs to the scalar
 // kernels).
 
-__device__ __forceinline__ void push_shadow_hero(const Wave& w, const Frame& f, int job, int view, D3 o, D3 d,
-                                                 double tmax, int nup, const double* lam, const double* val, int pix) {
+// A bundle's connection, plain (pix >= 0: val per wavelength is the contribution) or through
+// mirror `view >> 16` (pix < 0).  Returns false when the queue is full.
+__device__ __forceinline__ bool queue_hero(const Wave& w, int job, int view, D3 o, D3 d, double tmax, int nup,
+                                           const double* lam, const double* val, int pix) {
     int i = agg_inc(&w.counts[kShadowCount]);
-    if (i >= w.S) { atomicOr(f.status, ST_QUEUE_OVERFLOW); return; }
+    if (i >= w.S) return false;
     w.sox[i] = o.x; w.soy[i] = o.y; w.soz[i] = o.z;
     w.sdx[i] = d.x; w.sdy[i] = d.y; w.sdz[i] = d.z;
     w.smax[i] = tmax; w.spix[i] = pix; w.sjob[i] = job; w.sview[i] = view;
@@ -2091,10 +2145,26 @@ __device__ __forceinline__ void push_shadow_hero(const Wave& w, const Frame& f, 
         w.xval[(size_t)(k - 1) * w.S + i] = val[k];
     }
     w.snup[i] = nup;
+    return true;
+}
+template <bool INST, bool SHAPES>
+__device__ __noinline__ void connect_now_hero(const DevJob& J, const Frame& f, int view, D3 o, D3 d, double tmax,
+                                              int nup, const double* lam, const double* val, int pix);
+__device__ __forceinline__ void push_hero(const WaveQueue& q, const DevJob&, const Frame& f, int job, int view, D3 o,
+                                          D3 d, double tmax, int nup, const double* lam, const double* val, int pix) {
+    if (!queue_hero(q.w, job, view, o, d, tmax, nup, lam, val, pix)) atomicOr(f.status, ST_QUEUE_OVERFLOW);
+}
+template <bool INST, bool SHAPES>
+__device__ __forceinline__ void push_hero(const PathQueue<INST, SHAPES>& q, const DevJob& J, const Frame& f, int job,
+                                          int view, D3 o, D3 d, double tmax, int nup, const double* lam,
+                                          const double* val, int pix) {
+    if (!queue_hero(q.w, job, view, o, d, tmax, nup, lam, val, pix))
+        connect_now_hero<INST, SHAPES>(J, f, view, o, d, tmax, nup, lam, val, pix);
 }
 
 // connectHero (render.h:564-577): one connectGeom, a contribution per live wavelength
-__device__ void connect_surface_hero(const DevJob& J, const Wave& w, const Frame& f, int job, D3 p, D3 n,
+template <class Q>
+__device__ void connect_surface_hero(const DevJob& J, const Q& w, const Frame& f, int job, D3 p, D3 n,
                                      D3 ng, D3 wi, const double* lam, const double* beta, const double* rho,
                                      int nup) {
     for (int v = 0; v < view_count(J); ++v) {
@@ -2116,7 +2186,25 @@ __device__ void connect_surface_hero(const DevJob& J, const Wave& w, const Frame
             double fr = rho[i] / PI_D;
             val[i] = beta[i] * fr * cos_surf * corr / denom * stg;
         }
-        push_shadow_hero(w, f, job, v, p + ng * 1e-6, wdir, dist - 2e-6, nup, lam, val, py * cam.rx + px);
+        push_hero(w, J, f, job, v, p + ng * 1e-6, wdir, dist - 2e-6, nup, lam, val, py * cam.rx + px);
+    }
+}
+
+// connect_mirrors for a bundle's live wavelengths (camSpecularSplatAllHero, render.h:
+// 1570-1576): a record carries (lambda_i, beta_i x (rho_i x shape)) per wavelength, as the
+// bundle's camera connections do; k_shadow_hero evaluates the mirror's reflectance for each.
+template <class Q>
+__device__ __noinline__ void connect_mirrors_hero(const DevScene& sc, const DevJob& J, const Q& w, const Frame& f,
+                                                  int job, D3 p, D3 n, const double* lam, const double* beta,
+                                                  const double* rho, int nup) {
+    for (int k = 0; k < sc.n_planes; ++k) {
+        for (int v = 0; v < view_count(J); ++v) {
+            D3 wP; double dP, shape; int pix;
+            if (!mirror_geometry(sc.planes[k], view_cam(J, v), p, false, n, 0.0, wP, dP, shape, pix)) continue;
+            double val[kHeroMax];
+            for (int q = 0; q < nup; ++q) val[q] = beta[q] * (rho[q] * shape);
+            push_hero(w, J, f, job, v | (k << 16), p, wP, dP, nup, lam, val, ~pix);
+        }
     }
 }
 
@@ -2172,8 +2260,8 @@ __global__ void __launch_bounds__(128, FTB_EMIT_MINB) k_emit_hero(Wave w, const 
             one[i] = 1.0;
         }
         tally_add(acc, jobs, multi, j, T_EMIT, to_fixed(sum_of(beta, C), J.tally_scale_inv, f.status));
-        connect_surface_hero(J, w, f, j, origin, emit_n, emit_n, emit_n, lam, beta, one, C);
-        if (MIRROR && sc.n_planes > 0) connect_mirrors_hero(sc, J, w, f, j, origin, emit_n, lam, beta, one, C);
+        connect_surface_hero(J, WaveQueue{w}, f, j, origin, emit_n, emit_n, emit_n, lam, beta, one, C);
+        if (MIRROR && sc.n_planes > 0) connect_mirrors_hero(sc, J, WaveQueue{w}, f, j, origin, emit_n, lam, beta, one, C);
         D3 ro = origin + dir * 1e-6;
         if (J.max_bounce <= 0) {
             tally_add(acc, jobs, multi, j, T_RES, to_fixed(sum_of(beta, C), J.tally_scale_inv, f.status));
@@ -2194,6 +2282,176 @@ __global__ void __launch_bounds__(128, FTB_EMIT_MINB) k_emit_hero(Wave w, const 
     tally_finish(acc, jobs, multi, n_jobs);
 }
 
+// One bounce of a bundle (tracePhotonHeroLoop): as shade_bounce, over the nup live
+// wavelengths; `absorbed`: the reweights booked as absorption (fixed point, per add).
+template <bool INST, bool SHAPES, bool MIRROR, class Q>
+__device__ __forceinline__ int shade_bounce_hero(const DevScene& sc, const DevJob& J, const Q& w, const Frame& f, int j,
+                                                 Pcg& rng, D3 ro, D3 rd, double (&lam)[kHeroMax],
+                                                 double (&beta)[kHeroMax], int& nup, Stk& stk, double ht, int rec,
+                                                 int sub, D3& no, D3& nd, bool& costly, long long& absorbed) {
+    const int C = J.hero_c;
+    const bool valid = rec >= 0;
+    const double d_event = valid ? ht : 1e30;
+    {   // Beer-Lambert per live wavelength (render.h:2389-2398)
+        int mi = stk_top_mat(stk);
+        if (mi >= 0)
+            for (int i = 0; i < nup; ++i) {
+                double a = spec_slot(sc, sc.mats[mi].absorb, lam[i], 0.0);
+                if (a > 0.0) beta[i] *= exp(-a * d_event);
+            }
+    }
+    int fate = -1;
+    no = ro; nd = rd;
+    absorbed = 0;
+    if (!valid) {
+        fate = 1;
+    } else {
+        Rec r;
+        load_rec(sc.recs, rec, r);
+        if (SHAPES && rec_type(r) == REC_CURVE) costly = true;
+        Hit h;
+        if (INST && rec_type(r) == REC_INST) {
+            instance_hit(sc.inst[rec_inst(r)], sub, ro, rd, h);
+            h.prim = r.prim;
+        } else {
+            RayCtx R = make_ray(ro, rd);
+            hit_attributes<SHAPES>(sc.tri_n, R, sc.recs, rec, r, h);
+        }
+        const DevMat& m = sc.mats[h.mat];
+        switch (m.type) {
+        case FTB_MAT_DIFFUSE_TRANSMIT: {   // render.h:2454-2503
+            double rr[kHeroMax], rt[kHeroMax];
+            for (int i = 0; i < nup; ++i) {
+                double a = clamp01(spec_slot(sc, m.reflect, lam[i], 0.5));
+                double b = clamp01(spec_slot(sc, m.transmit, lam[i], 0.0));
+                double s = a + b;
+                if (s > 1.0) { a /= s; b /= s; }
+                rr[i] = a; rt[i] = b;
+            }
+            D3 ngo = oriented_geo_n(h);
+            D3 wi = mk(-rd.x, -rd.y, -rd.z);
+            connect_surface_hero(J, w, f, j, h.p, h.n, ngo, wi, lam, beta, rr, nup);
+            connect_surface_hero(J, w, f, j, h.p, neg(h.n), neg(ngo), wi, lam, beta, rt, nup);
+            if (MIRROR && sc.n_planes > 0) {
+                connect_mirrors_hero(sc, J, w, f, j, h.p, h.n, lam, beta, rr, nup);
+                connect_mirrors_hero(sc, J, w, f, j, h.p, neg(h.n), lam, beta, rt, nup);
+            }
+            double q_r = max_of(rr, nup), q_t = max_of(rt, nup);
+            double sum_h = q_r + q_t;
+            if (nup > 1 && sum_h > 1.0) { q_r /= sum_h; q_t /= sum_h; sum_h = q_r + q_t; }
+            double uu = uniform(rng);
+            if (uu < q_r || uu < sum_h) {
+                const bool front = uu < q_r;
+                for (int i = 0; i < nup; ++i) {
+                    double wgt = (front ? rr[i] : rt[i]) / (front ? q_r : q_t);
+                    absorbed += to_fixed(beta[i] * (1.0 - wgt), J.tally_scale_inv, f.status);
+                    beta[i] *= wgt;
+                }
+                D3 wo = cosine_hemisphere(front ? h.n : mk(-h.n.x, -h.n.y, -h.n.z), rng);
+                double corr = shading_adjoint_corr(wi, wo, h.n, ngo);
+                for (int i = 0; i < nup; ++i) beta[i] *= corr;
+                no = front ? h.p + h.n * 1e-6 : h.p - h.n * 1e-6;
+                nd = wo;
+            } else {
+                fate = 0;
+            }
+            break;
+        }
+        case FTB_MAT_MIRROR:
+        case FTB_MAT_FILTER:
+        case FTB_MAT_GLOSSY: {   // achromatic lobes (render.h:2509-2537)
+            double cc[kHeroMax];
+            for (int i = 0; i < nup; ++i)
+                cc[i] = (m.type == FTB_MAT_FILTER) ? clamp01(spec_slot(sc, m.transmit, lam[i], 0.0))
+                                                   : clamp01(spec_slot(sc, m.reflect, lam[i], 0.5));
+            double q = max_of(cc, nup);
+            if (uniform(rng) >= q) { fate = 0; break; }
+            for (int i = 0; i < nup; ++i) {
+                double wgt = cc[i] / q;
+                absorbed += to_fixed(beta[i] * (1.0 - wgt), J.tally_scale_inv, f.status);
+                beta[i] *= wgt;
+            }
+            if (m.type == FTB_MAT_MIRROR) {
+                no = h.p + h.n * 1e-6; nd = reflect(rd, h.n);
+            } else if (m.type == FTB_MAT_FILTER) {
+                no = h.p + rd * 1e-6;
+            } else {
+                D3 o = sample_glossy(reflect(rd, h.n), m.roughness, rng);
+                if (dot(o, h.n) <= 0) { fate = 0; break; }
+                no = h.p + h.n * 1e-6; nd = o;
+            }
+            break;
+        }
+        case FTB_MAT_HALF_MIRROR: {   // de-hero, then the scalar half mirror (render.h:2546-2589, 1702-1711)
+            if (nup > 1) { beta[0] *= (double)C; nup = 1; }
+            const double rr = clamp01(spec_slot(sc, m.reflect, lam[0], 0.5));
+            if (uniform(rng) < rr) {
+                nd = reflect(rd, h.n);
+                no = h.p + h.n * 1e-6;
+            } else {
+                no = h.p + rd * 1e-6;
+            }
+            break;
+        }
+        case FTB_MAT_DIELECTRIC: {   // de-hero, then the scalar interaction (render.h:2539-2589)
+            if (nup > 1) { beta[0] *= (double)C; nup = 1; }
+            const double lam0 = lam[0];
+            bool entering = dot(rd, h.ng) < 0.0;
+            int mi = h.mat, pr = m.priority;
+            bool has_pri = pr != INT_MIN;
+            bool transmitted = false;
+            if (entering) {
+                int out_mat = stk_top_mat(stk), out_pri = stk_top_pri(stk);
+                bool ranked = has_pri && (stk.n == 0 || (out_mat >= 0 && sc.mats[out_mat].priority != INT_MIN));
+                if (ranked && stk.n != 0 && pr <= out_pri) {
+                    stk_push(stk, mi, pr, f.status);
+                    no = h.p + rd * 1e-6;
+                } else {
+                    double ext = (ranked && out_mat >= 0) ? mat_ior(sc, sc.mats[out_mat], lam0) : 1.0;
+                    refract_or_reflect(sc, m, h, rd, lam0, rng, transmitted, ext, no, nd);
+                    if (transmitted) stk_push(stk, mi, pr, f.status);
+                }
+            } else {
+                Stk after = stk;
+                stk_pop_mat(after, mi);
+                int new_mat = stk_top_mat(after), new_pri = stk_top_pri(after);
+                bool ranked = has_pri && (after.n == 0 || (new_mat >= 0 && sc.mats[new_mat].priority != INT_MIN));
+                if (ranked && new_mat >= 0 && pr <= new_pri) {
+                    stk_pop_mat(stk, mi);
+                    no = h.p + rd * 1e-6;
+                } else {
+                    double ext = (ranked && new_mat >= 0) ? mat_ior(sc, sc.mats[new_mat], lam0) : 1.0;
+                    refract_or_reflect(sc, m, h, rd, lam0, rng, transmitted, ext, no, nd);
+                    if (transmitted) stk_pop_mat(stk, mi);
+                }
+            }
+            break;
+        }
+        default: {   // Diffuse (render.h:2591-2625)
+            double rho[kHeroMax];
+            for (int i = 0; i < nup; ++i) rho[i] = clamp01(spec_slot(sc, m.reflect, lam[i], 0.5));
+            D3 ngo = oriented_geo_n(h);
+            D3 wi = mk(-rd.x, -rd.y, -rd.z);
+            connect_surface_hero(J, w, f, j, h.p, h.n, ngo, wi, lam, beta, rho, nup);
+            if (MIRROR && sc.n_planes > 0) connect_mirrors_hero(sc, J, w, f, j, h.p, h.n, lam, beta, rho, nup);
+            double q = max_of(rho, nup);
+            if (uniform(rng) >= q) { fate = 0; break; }
+            for (int i = 0; i < nup; ++i) {
+                double wgt = rho[i] / q;
+                absorbed += to_fixed(beta[i] * (1.0 - wgt), J.tally_scale_inv, f.status);
+                beta[i] *= wgt;
+            }
+            D3 wo = cosine_hemisphere(h.n, rng);
+            double corr = shading_adjoint_corr(wi, wo, h.n, ngo);
+            for (int i = 0; i < nup; ++i) beta[i] *= corr;
+            no = h.p + h.n * 1e-6; nd = wo;
+            break;
+        }
+        }
+    }
+    return fate;
+}
+
 template <bool INST, bool SHAPES, bool MIRROR>
 __global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, const DevJob* __restrict__ jobs,
                                                                     Frame f, PathState in, const int32_t* in_count,
@@ -2208,7 +2466,6 @@ __global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, cons
         const int j = multi ? in.job[p] : 0;
         const DevJob& J = jobs[j];
         const DevScene& sc = J.sc;
-        const int C = J.hero_c;
         Pcg rng; rng.s = in.rng_s[p]; rng.inc = in.rng_i[p];
         D3 ro = mk(in.ox[p], in.oy[p], in.oz[p]), rd = mk(in.dx[p], in.dy[p], in.dz[p]);
         int nup = in.hlive[p];
@@ -2222,166 +2479,12 @@ __global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, cons
         Stk stk; stk.n = in.stk_n[p];
         for (int k = 0; k < stk.n; ++k) stk.e[k] = in.stk[k * w.W + p];
         log_hit<INST>(w, in, p, sc, rec);
-        const bool valid = rec >= 0;
-        const double d_event = valid ? ht : 1e30;
-        {   // Beer-Lambert per live wavelength (render.h:2389-2398)
-            int mi = stk_top_mat(stk);
-            if (mi >= 0)
-                for (int i = 0; i < nup; ++i) {
-                    double a = spec_slot(sc, sc.mats[mi].absorb, lam[i], 0.0);
-                    if (a > 0.0) beta[i] *= exp(-a * d_event);
-                }
-        }
-        int fate = -1;   // -1 continue, 0 absorbed, 1 escaped
-        bool costly = false;   // the next ray starts among curves: back end of the queue
-        D3 no = ro, nd = rd;
-        long long absorbed = 0;   // reweights booked as absorption (fixed point, per add)
-        if (!valid) {
-            fate = 1;
-        } else {
-            Rec r;
-            load_rec(sc.recs, rec, r);
-            if (SHAPES && rec_type(r) == REC_CURVE) costly = true;
-            Hit h;
-            if (INST && rec_type(r) == REC_INST) {
-                instance_hit(sc.inst[rec_inst(r)], w.hit_sub[p], ro, rd, h);
-                h.prim = r.prim;
-            } else {
-                RayCtx R = make_ray(ro, rd);
-                hit_attributes<SHAPES>(sc.tri_n, R, sc.recs, rec, r, h);
-            }
-            const DevMat& m = sc.mats[h.mat];
-            switch (m.type) {
-            case FTB_MAT_DIFFUSE_TRANSMIT: {   // render.h:2454-2503
-                double rr[kHeroMax], rt[kHeroMax];
-                for (int i = 0; i < nup; ++i) {
-                    double a = clamp01(spec_slot(sc, m.reflect, lam[i], 0.5));
-                    double b = clamp01(spec_slot(sc, m.transmit, lam[i], 0.0));
-                    double s = a + b;
-                    if (s > 1.0) { a /= s; b /= s; }
-                    rr[i] = a; rt[i] = b;
-                }
-                D3 ngo = oriented_geo_n(h);
-                D3 wi = mk(-rd.x, -rd.y, -rd.z);
-                connect_surface_hero(J, w, f, j, h.p, h.n, ngo, wi, lam, beta, rr, nup);
-                connect_surface_hero(J, w, f, j, h.p, neg(h.n), neg(ngo), wi, lam, beta, rt, nup);
-                if (MIRROR && sc.n_planes > 0) {
-                    connect_mirrors_hero(sc, J, w, f, j, h.p, h.n, lam, beta, rr, nup);
-                    connect_mirrors_hero(sc, J, w, f, j, h.p, neg(h.n), lam, beta, rt, nup);
-                }
-                double q_r = max_of(rr, nup), q_t = max_of(rt, nup);
-                double sum_h = q_r + q_t;
-                if (nup > 1 && sum_h > 1.0) { q_r /= sum_h; q_t /= sum_h; sum_h = q_r + q_t; }
-                double uu = uniform(rng);
-                if (uu < q_r || uu < sum_h) {
-                    const bool front = uu < q_r;
-                    for (int i = 0; i < nup; ++i) {
-                        double wgt = (front ? rr[i] : rt[i]) / (front ? q_r : q_t);
-                        absorbed += to_fixed(beta[i] * (1.0 - wgt), J.tally_scale_inv, f.status);
-                        beta[i] *= wgt;
-                    }
-                    D3 wo = cosine_hemisphere(front ? h.n : mk(-h.n.x, -h.n.y, -h.n.z), rng);
-                    double corr = shading_adjoint_corr(wi, wo, h.n, ngo);
-                    for (int i = 0; i < nup; ++i) beta[i] *= corr;
-                    no = front ? h.p + h.n * 1e-6 : h.p - h.n * 1e-6;
-                    nd = wo;
-                } else {
-                    fate = 0;
-                }
-                break;
-            }
-            case FTB_MAT_MIRROR:
-            case FTB_MAT_FILTER:
-            case FTB_MAT_GLOSSY: {   // achromatic lobes (render.h:2509-2537)
-                double cc[kHeroMax];
-                for (int i = 0; i < nup; ++i)
-                    cc[i] = (m.type == FTB_MAT_FILTER) ? clamp01(spec_slot(sc, m.transmit, lam[i], 0.0))
-                                                       : clamp01(spec_slot(sc, m.reflect, lam[i], 0.5));
-                double q = max_of(cc, nup);
-                if (uniform(rng) >= q) { fate = 0; break; }
-                for (int i = 0; i < nup; ++i) {
-                    double wgt = cc[i] / q;
-                    absorbed += to_fixed(beta[i] * (1.0 - wgt), J.tally_scale_inv, f.status);
-                    beta[i] *= wgt;
-                }
-                if (m.type == FTB_MAT_MIRROR) {
-                    no = h.p + h.n * 1e-6; nd = reflect(rd, h.n);
-                } else if (m.type == FTB_MAT_FILTER) {
-                    no = h.p + rd * 1e-6;
-                } else {
-                    D3 o = sample_glossy(reflect(rd, h.n), m.roughness, rng);
-                    if (dot(o, h.n) <= 0) { fate = 0; break; }
-                    no = h.p + h.n * 1e-6; nd = o;
-                }
-                break;
-            }
-            case FTB_MAT_HALF_MIRROR: {   // de-hero, then the scalar half mirror (render.h:2546-2589, 1702-1711)
-                if (nup > 1) { beta[0] *= (double)C; nup = 1; }
-                const double rr = clamp01(spec_slot(sc, m.reflect, lam[0], 0.5));
-                if (uniform(rng) < rr) {
-                    nd = reflect(rd, h.n);
-                    no = h.p + h.n * 1e-6;
-                } else {
-                    no = h.p + rd * 1e-6;
-                }
-                break;
-            }
-            case FTB_MAT_DIELECTRIC: {   // de-hero, then the scalar interaction (render.h:2539-2589)
-                if (nup > 1) { beta[0] *= (double)C; nup = 1; }
-                const double lam0 = lam[0];
-                bool entering = dot(rd, h.ng) < 0.0;
-                int mi = h.mat, pr = m.priority;
-                bool has_pri = pr != INT_MIN;
-                bool transmitted = false;
-                if (entering) {
-                    int out_mat = stk_top_mat(stk), out_pri = stk_top_pri(stk);
-                    bool ranked = has_pri && (stk.n == 0 || (out_mat >= 0 && sc.mats[out_mat].priority != INT_MIN));
-                    if (ranked && stk.n != 0 && pr <= out_pri) {
-                        stk_push(stk, mi, pr, f.status);
-                        no = h.p + rd * 1e-6;
-                    } else {
-                        double ext = (ranked && out_mat >= 0) ? mat_ior(sc, sc.mats[out_mat], lam0) : 1.0;
-                        refract_or_reflect(sc, m, h, rd, lam0, rng, transmitted, ext, no, nd);
-                        if (transmitted) stk_push(stk, mi, pr, f.status);
-                    }
-                } else {
-                    Stk after = stk;
-                    stk_pop_mat(after, mi);
-                    int new_mat = stk_top_mat(after), new_pri = stk_top_pri(after);
-                    bool ranked = has_pri && (after.n == 0 || (new_mat >= 0 && sc.mats[new_mat].priority != INT_MIN));
-                    if (ranked && new_mat >= 0 && pr <= new_pri) {
-                        stk_pop_mat(stk, mi);
-                        no = h.p + rd * 1e-6;
-                    } else {
-                        double ext = (ranked && new_mat >= 0) ? mat_ior(sc, sc.mats[new_mat], lam0) : 1.0;
-                        refract_or_reflect(sc, m, h, rd, lam0, rng, transmitted, ext, no, nd);
-                        if (transmitted) stk_pop_mat(stk, mi);
-                    }
-                }
-                break;
-            }
-            default: {   // Diffuse (render.h:2591-2625)
-                double rho[kHeroMax];
-                for (int i = 0; i < nup; ++i) rho[i] = clamp01(spec_slot(sc, m.reflect, lam[i], 0.5));
-                D3 ngo = oriented_geo_n(h);
-                D3 wi = mk(-rd.x, -rd.y, -rd.z);
-                connect_surface_hero(J, w, f, j, h.p, h.n, ngo, wi, lam, beta, rho, nup);
-                if (MIRROR && sc.n_planes > 0) connect_mirrors_hero(sc, J, w, f, j, h.p, h.n, lam, beta, rho, nup);
-                double q = max_of(rho, nup);
-                if (uniform(rng) >= q) { fate = 0; break; }
-                for (int i = 0; i < nup; ++i) {
-                    double wgt = rho[i] / q;
-                    absorbed += to_fixed(beta[i] * (1.0 - wgt), J.tally_scale_inv, f.status);
-                    beta[i] *= wgt;
-                }
-                D3 wo = cosine_hemisphere(h.n, rng);
-                double corr = shading_adjoint_corr(wi, wo, h.n, ngo);
-                for (int i = 0; i < nup; ++i) beta[i] *= corr;
-                no = h.p + h.n * 1e-6; nd = wo;
-                break;
-            }
-            }
-        }
+        bool costly = false;
+        D3 no, nd;
+        long long absorbed;
+        const int fate = shade_bounce_hero<INST, SHAPES, MIRROR>(sc, J, WaveQueue{w}, f, j, rng, ro, rd, lam, beta, nup,
+                                                                 stk, ht, rec, INST ? w.hit_sub[p] : -1, no, nd, costly,
+                                                                 absorbed);
         if (absorbed) tally_add(acc, jobs, multi, j, T_ABS, absorbed);
         if (fate >= 0) {
             tally_add(acc, jobs, multi, j, fate == 0 ? T_ABS : T_ESC,
@@ -2416,19 +2519,19 @@ __global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, cons
 // A bundle's mirror record: every live wavelength is its own splat with its own reflectance
 // (splatMirrorLegs, render.h:1321-1330; bundles run without media); a wavelength whose
 // contribution is not positive adds nothing, not even to the hit count.
-template <bool COUNT, bool INST, bool SHAPES>
-__device__ __noinline__ void mirror_splat_hero(const DevJob& J, const Wave& w, const Frame& f, int i, TravCount& cnt) {
+template <bool COUNT, bool INST, bool SHAPES, class Lam, class Val>
+__device__ __forceinline__ void mirror_splat_hero(const DevJob& J, const Frame& f, int view, int plane, D3 p, D3 wP,
+                                                  double dP, int nup, const Lam& lam_of, const Val& val_of, int pix,
+                                                  TravCount& cnt) {
     MirrorSeen ms;
-    if (!mirror_seen<COUNT, INST, SHAPES>(J, w, f, i, cnt, ms)) return;
+    if (!mirror_seen<COUNT, INST, SHAPES>(J, f, view, plane, p, wP, dP, cnt, ms)) return;
     const DevScene& sc = J.sc;
     const double inv_d2_omega = 1.0 / (ms.D * ms.D * ms.omega);
-    const int nup = w.snup[i];
     long long sx = 0, sy = 0, sz = 0, hits = 0;
     for (int k = 0; k < nup; ++k) {
-        const double lam = k == 0 ? w.slam[i] : w.xlam[(size_t)(k - 1) * w.S + i];
-        const double a = k == 0 ? w.sval[i] : w.xval[(size_t)(k - 1) * w.S + i];
+        const double lam = lam_of(k);
         const double refl = clamp01(spec_slot(sc, sc.mats[ms.mat].reflect, lam, 0.5));
-        const double contrib = a * refl * inv_d2_omega;
+        const double contrib = val_of(k) * refl * inv_d2_omega;
         if (contrib <= 0.0) continue;
         sx += to_fixed(cie_x(lam) * contrib, J.film_scale_inv, f.status);
         sy += to_fixed(cie_y(lam) * contrib, J.film_scale_inv, f.status);
@@ -2436,7 +2539,47 @@ __device__ __noinline__ void mirror_splat_hero(const DevJob& J, const Wave& w, c
         ++hits;
     }
     if (!hits) return;
-    film_add(view_film(J, w.sview[i] & 0xffff), ~w.spix[i], sx, sy, sz, hits);
+    film_add(view_film(J, view), pix, sx, sy, sz, hits);
+}
+template <bool COUNT, bool INST, bool SHAPES>
+__device__ __noinline__ void mirror_record_hero(const DevJob& J, const Wave& w, const Frame& f, int i, TravCount& cnt) {
+    auto lam_of = [&](int k) { return k == 0 ? w.slam[i] : w.xlam[(size_t)(k - 1) * w.S + i]; };
+    auto val_of = [&](int k) { return k == 0 ? w.sval[i] : w.xval[(size_t)(k - 1) * w.S + i]; };
+    mirror_splat_hero<COUNT, INST, SHAPES>(J, f, w.sview[i] & 0xffff, w.sview[i] >> 16,
+                                           mk(w.sox[i], w.soy[i], w.soz[i]), mk(w.sdx[i], w.sdy[i], w.sdz[i]), w.smax[i],
+                                           w.snup[i], lam_of, val_of, ~w.spix[i], cnt);
+}
+
+// A bundle's connection that was not occluded: every wavelength is one Film::add, each rounded
+// to fixed point on its own; their integer sum goes to the pixel at once (integer sums are
+// exact).
+template <class Lam, class Val>
+__device__ __forceinline__ void splat_hero(const DevJob& J, const Frame& f, int view, int pix, int nup,
+                                           const Lam& lam_of, const Val& val_of) {
+    long long sx = 0, sy = 0, sz = 0;
+    for (int k = 0; k < nup; ++k) {
+        const double lam = lam_of(k), c = val_of(k);
+        double X = cie_x(lam) * c, Y = cie_y(lam) * c, Z = cie_z(lam) * c;
+        sx += to_fixed(X, J.film_scale_inv, f.status);
+        sy += to_fixed(Y, J.film_scale_inv, f.status);
+        sz += to_fixed(Z, J.film_scale_inv, f.status);
+    }
+    film_add(view_film(J, view), pix, sx, sy, sz, nup);
+}
+// A bundle's connection that found the queue full: the same test and splat at once.
+template <bool INST, bool SHAPES>
+__device__ __noinline__ void connect_now_hero(const DevJob& J, const Frame& f, int view, D3 o, D3 d, double tmax,
+                                              int nup, const double* lam, const double* val, int pix) {
+    TravCount cnt{0, 0, 0};
+    auto lam_of = [&](int k) { return lam[k]; };
+    auto val_of = [&](int k) { return val[k]; };
+    if (pix < 0) {
+        mirror_splat_hero<false, INST, SHAPES>(J, f, view & 0xffff, view >> 16, o, d, tmax, nup, lam_of, val_of, ~pix, cnt);
+        return;
+    }
+    const RayCtx R = make_ray(o, d);
+    if (traverse_any<false, INST, SHAPES>(J.sc, R, EPS_RAY, tmax - EPS_RAY, f.status, cnt)) return;
+    splat_hero(J, f, view, pix, nup, lam_of, val_of);
 }
 
 // Connections of bundles: one occlusion test, then a splat per wavelength.  MIRROR: the queue
@@ -2454,32 +2597,172 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow_hero(Wave w, cons
         const DevScene& sc = J.sc;
         if (COUNT) rays++;
         if (MIRROR && w.spix[i] < 0) {
-            mirror_splat_hero<COUNT, INST, SHAPES>(J, w, f, i, cnt);
+            mirror_record_hero<COUNT, INST, SHAPES>(J, w, f, i, cnt);
             continue;
         }
         D3 o = mk(w.sox[i], w.soy[i], w.soz[i]), d = mk(w.sdx[i], w.sdy[i], w.sdz[i]);
         double max_dist = w.smax[i];
         RayCtx R = make_ray(o, d);
         if (traverse_any<COUNT, INST, SHAPES>(sc, R, EPS_RAY, max_dist - EPS_RAY, f.status, cnt)) continue;
-        const int nup = w.snup[i];
-        // every wavelength is one Film::add, each rounded to fixed point on its own; their
-        // integer sum goes to the pixel at once (integer sums are exact)
-        long long sx = 0, sy = 0, sz = 0;
-        for (int k = 0; k < nup; ++k) {
-            double lam = k == 0 ? w.slam[i] : w.xlam[(size_t)(k - 1) * w.S + i];
-            double c = k == 0 ? w.sval[i] : w.xval[(size_t)(k - 1) * w.S + i];
-            double X = cie_x(lam) * c, Y = cie_y(lam) * c, Z = cie_z(lam) * c;
-            sx += to_fixed(X, J.film_scale_inv, f.status);
-            sy += to_fixed(Y, J.film_scale_inv, f.status);
-            sz += to_fixed(Z, J.film_scale_inv, f.status);
-        }
-        film_add(view_film(J, w.sview[i]), w.spix[i], sx, sy, sz, nup);
+        splat_hero(J, f, w.sview[i], w.spix[i], w.snup[i],
+                   [&](int k) { return k == 0 ? w.slam[i] : w.xlam[(size_t)(k - 1) * w.S + i]; },
+                   [&](int k) { return k == 0 ? w.sval[i] : w.xval[(size_t)(k - 1) * w.S + i]; });
     }
     film_finish();
     if (COUNT) {
         block_add3(f.stats + 3, rays, cnt.nodes, cnt.recs);
         block_add1(f.stats + 7, cnt.exact);
     }
+}
+
+// ------------------------------------------------------------------ whole paths --------
+// The queue's paths, each traced to its end by one lane: closest hit and shading alternate
+// until the path ends, its state stays in the lane, and the connections are queued for
+// k_shadow.  For queues of at most trace_limit() paths -- the tail of a streaming pass, and
+// passes and renders that small from the start -- where launches per bounce mostly wait for
+// the slowest warp of each: bound by the latency of one path's chain of bounces, not by
+// throughput, so with fewer paths than lanes they are spread over all warps (a warp of few
+// paths diverges less).  B200: preview of 2^16 photons 0.45 -> 0.26 ms, three renders of
+// 23,334 photons through glass without allocation 5.06 -> 1.62 ms, fog + strands frame (32
+// bounces) 117.2 -> 116.1, session of 4 views 23.6 -> 22.5.  The line lies at one path per
+// resident lane: tails of 50,000, 150,000 and 500,000 paths took the same time on whole
+// frames, and above it the kernel loses to the launches per bounce (all of a Cornell frame
+// traced this way: 16.1 against 13.6 ms; glass 580-650 against 235 ms), since its warps run
+// closest hits and materials of all kinds side by side at half the resident warps.
+template <class Load, class Step>
+__device__ __forceinline__ void trace_lanes(const Wave& w, int n, const Load& load, const Step& step) {
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    const int share = (n + warps - 1) / warps;
+    bool more = lane < share, alive = false;   // this lane takes paths; it has one
+    for (;;) {
+        const unsigned want = __ballot_sync(0xffffffffu, more && !alive);
+        if (want) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&w.counts[kFetchExtend], __popc(want));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (more && !alive) {
+                const int q = base + __popc(want & ((1u << lane) - 1u));
+                if (q < n) { load(q); alive = true; }
+                else more = false;
+            }
+        }
+        if (!__any_sync(0xffffffffu, alive)) return;
+        if (alive) alive = step();
+    }
+}
+
+template <bool MEDIA, bool INST, bool SHAPES, bool MIRROR>
+__global__ void __launch_bounds__(128, FTB_TRACE_MINB) k_trace(Wave w, const DevJob* __restrict__ jobs, Frame f,
+                                                              PathState in, const int32_t* in_count) {
+    const int32_t n_jobs = w.params[0];
+    const bool multi = n_jobs > 1;
+    TallyAcc acc;
+    tally_init(acc, multi, n_jobs);
+    const int front = in_count[0];
+    const PathQueue<INST, SHAPES> queue{w};
+    TravCount cnt{0, 0, 0};
+    int i = 0, j = 0, bounce = 0;
+    Pcg rng{0, 0};
+    D3 ro = mk(0, 0, 0), rd = mk(0, 0, 1);
+    double lam = 0.0, beta = 0.0, cie[3] = {0.0, 0.0, 0.0};
+    Stk stk;
+    stk.n = 0;
+    auto load = [&](int q) {
+        i = queue_entry(w, front, q);
+        j = multi ? in.job[i] : 0;
+        rng.s = in.rng_s[i]; rng.inc = in.rng_i[i];
+        ro = mk(in.ox[i], in.oy[i], in.oz[i]); rd = mk(in.dx[i], in.dy[i], in.dz[i]);
+        lam = in.lam[i]; beta = in.beta[i];
+        cie[0] = in.cie[i]; cie[1] = in.cie[w.W + i]; cie[2] = in.cie[2 * (size_t)w.W + i];
+        stk.n = in.stk_n[i];
+        for (int e = 0; e < stk.n; ++e) stk.e[e] = in.stk[e * w.W + i];
+        bounce = in.nbounce[i];
+    };
+    auto step = [&]() -> bool {
+        const DevJob& J = jobs[j];
+        const DevScene& sc = J.sc;
+        double t;
+        int sub = -1;
+        const int rec = traverse_closest<false, INST, SHAPES>(sc, make_ray(ro, rd), EPS_RAY, t, &sub, f.status, cnt);
+        if (w.logs) {
+            if (INST) w.hit_sub[i] = sub;
+            log_hit<INST>(w, in, i, sc, rec);
+        }
+        bool costly = false;
+        D3 no, nd;
+        int fate = shade_bounce<MEDIA, INST, SHAPES, MIRROR>(sc, J, queue, f, j, rng, ro, rd, lam, beta, stk, t, rec,
+                                                            sub, [&]() -> const double* { return cie; }, no, nd, costly);
+        if (fate < 0 && ++bounce >= J.max_bounce) fate = 2;
+        ro = no; rd = nd;
+        if (fate < 0) return true;
+        tally_add(acc, jobs, multi, j, fate == 0 ? T_ABS : (fate == 1 ? T_ESC : T_RES),
+                  to_fixed(beta, J.tally_scale_inv, f.status));
+        log_finish(w, in, i, fate, beta);
+        return false;
+    };
+    trace_lanes(w, queue_len(in_count), load, step);
+    film_finish();
+    tally_finish(acc, jobs, multi, n_jobs);
+}
+
+template <bool INST, bool SHAPES, bool MIRROR>
+__global__ void __launch_bounds__(128, FTB_TRACE_MINB) k_trace_hero(Wave w, const DevJob* __restrict__ jobs, Frame f,
+                                                                   PathState in, const int32_t* in_count) {
+    const int32_t n_jobs = w.params[0];
+    const bool multi = n_jobs > 1;
+    TallyAcc acc;
+    tally_init(acc, multi, n_jobs);
+    const int front = in_count[0];
+    const PathQueue<INST, SHAPES> queue{w};
+    TravCount cnt{0, 0, 0};
+    int i = 0, j = 0, bounce = 0, nup = 0;
+    Pcg rng{0, 0};
+    D3 ro = mk(0, 0, 0), rd = mk(0, 0, 1);
+    double lam[kHeroMax], beta[kHeroMax];
+    Stk stk;
+    stk.n = 0;
+    auto load = [&](int q) {
+        i = queue_entry(w, front, q);
+        j = multi ? in.job[i] : 0;
+        rng.s = in.rng_s[i]; rng.inc = in.rng_i[i];
+        ro = mk(in.ox[i], in.oy[i], in.oz[i]); rd = mk(in.dx[i], in.dy[i], in.dz[i]);
+        nup = in.hlive[i];
+        for (int k = 0; k < nup; ++k) {
+            lam[k] = in.hlam[(size_t)k * w.W + i];
+            beta[k] = in.hbeta[(size_t)k * w.W + i];
+        }
+        stk.n = in.stk_n[i];
+        for (int e = 0; e < stk.n; ++e) stk.e[e] = in.stk[e * w.W + i];
+        bounce = in.nbounce[i];
+    };
+    auto step = [&]() -> bool {
+        const DevJob& J = jobs[j];
+        const DevScene& sc = J.sc;
+        double t;
+        int sub = -1;
+        const int rec = traverse_closest<false, INST, SHAPES>(sc, make_ray(ro, rd), EPS_RAY, t, &sub, f.status, cnt);
+        if (w.logs) {
+            if (INST) w.hit_sub[i] = sub;
+            log_hit<INST>(w, in, i, sc, rec);
+        }
+        bool costly = false;
+        D3 no, nd;
+        long long absorbed;
+        int fate = shade_bounce_hero<INST, SHAPES, MIRROR>(sc, J, queue, f, j, rng, ro, rd, lam, beta, nup, stk, t, rec,
+                                                          sub, no, nd, costly, absorbed);
+        if (absorbed) tally_add(acc, jobs, multi, j, T_ABS, absorbed);
+        if (fate < 0 && ++bounce >= J.max_bounce) fate = 2;
+        ro = no; rd = nd;
+        if (fate < 0) return true;
+        tally_add(acc, jobs, multi, j, fate == 0 ? T_ABS : (fate == 1 ? T_ESC : T_RES),
+                  to_fixed(sum_of(beta, nup), J.tally_scale_inv, f.status));
+        log_finish(w, in, i, fate, beta[0]);
+        return false;
+    };
+    trace_lanes(w, queue_len(in_count), load, step);
+    film_finish();
+    tally_finish(acc, jobs, multi, n_jobs);
 }
 
 // ------------------------------------------------------------------ host side ----------
@@ -2552,11 +2835,12 @@ __global__ void k_stream_init(Wave w) {
 
 // End of a half-iteration (one thread): the refill's photons are booked and its paths join
 // the queue for the next half-iteration, the consumed queue is emptied (the connection queue
-// is by the launch that traces it), and whether work is left -- paths queued or photons not yet handed out -- goes to
-// the progress word and, inside a graph, to the loop condition.  A pass that reaches its
-// half-iteration cap with work left stops with ST_LOOP_CAP.
+// is by the launch that traces it), and whether work is left for another half-iteration --
+// photons not yet handed out, or more than `tail` paths queued -- goes to the progress word
+// and, inside a graph, to the loop condition.  A pass that reaches its half-iteration cap
+// with such work left stops with ST_LOOP_CAP.
 __global__ void k_stream_advance(Wave w, Frame f, int32_t* consumed, int32_t* next_q,
-                                 cudaGraphConditionalHandle loop, int32_t set_loop) {
+                                 int32_t tail, cudaGraphConditionalHandle loop, int32_t set_loop) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     StreamCtl& c = *w.ctl;
     const int64_t total = reinterpret_cast<const int64_t*>(w.params)[1];
@@ -2571,7 +2855,7 @@ __global__ void k_stream_advance(Wave w, Frame f, int32_t* consumed, int32_t* ne
     consumed[1] = 0;
     w.counts[kFetchExtend] = 0;
     w.counts[kFetchShade] = 0;
-    int32_t more = (queue_len(next_q) > 0 || c.next < total) ? 1 : 0;
+    int32_t more = (queue_len(next_q) > tail || c.next < total) ? 1 : 0;
     if (more && c.half >= cap) {
         atomicOr(f.status, ST_LOOP_CAP);
         more = 0;
@@ -2623,7 +2907,11 @@ struct Issue {
     bool sorted;
     cudaStream_t st;
     LaunchSink* sink;
+    int32_t sms;
     static constexpr int T = 128;
+
+    // paths left to the whole-path kernels, which have no counting variant
+    int32_t tail() const { return f.stats ? 0 : trace_limit(sms); }
 
     void mark(int k, bool end) { if (sink) sink->mark(k, end, st); }
     void emit(bool stream, const PathState& out, int32_t* co) {
@@ -2666,6 +2954,29 @@ struct Issue {
         else if (kind.mirrors) trav<LaunchShadowMirror>(w, (const DevJob*)w.jobs, f);
         else trav<LaunchShadow>(w, (const DevJob*)w.jobs, f);
         mark(K_SHADOW, true);
+    }
+    void trace(const PathState& in, const int32_t* c) {   // whole paths (booked with closest hit)
+        const bool inst = kind.instances, shp = kind.shapes;
+        const DevJob* jobs = w.jobs;
+        const int g = sms * FTB_TRACE_MINB;
+        mark(K_EXTEND, false);
+#define FTB_TRACE(...) __VA_ARGS__<<<g, T, 0, st>>>(w, jobs, f, in, c)
+#define FTB_TRACE_SET(...) \
+    if (inst) { if (shp) FTB_TRACE(__VA_ARGS__ true, true, false>); else FTB_TRACE(__VA_ARGS__ true, false, false>); } \
+    else { if (shp) FTB_TRACE(__VA_ARGS__ false, true, false>); else FTB_TRACE(__VA_ARGS__ false, false, false>); }
+        // scenes with planar mirrors share one variant for every kind of record (three builds
+        // of the heaviest kernels rather than twelve); the others' exact variants are 15-20 %
+        // faster than it on a preview of 2^16 photons (0.26 against 0.31 ms)
+        if (kind.mirrors) {
+            if (kind.bundles) FTB_TRACE(k_trace_hero<true, true, true>);
+            else if (kind.media) FTB_TRACE(k_trace<true, true, true, true>);
+            else FTB_TRACE(k_trace<false, true, true, true>);
+        } else if (kind.bundles) { FTB_TRACE_SET(k_trace_hero<) }
+        else if (kind.media) { FTB_TRACE_SET(k_trace<true,) }
+        else { FTB_TRACE_SET(k_trace<false,) }
+#undef FTB_TRACE_SET
+#undef FTB_TRACE
+        mark(K_EXTEND, true);
     }
     void extend(const PathState& in, int32_t* c) {
         mark(K_EXTEND, false);
@@ -2730,6 +3041,15 @@ void issue_wave(Issue& I, int32_t max_bounce) {
     }
 }
 
+// A wave of at most trace_limit() slots: emission, then every path to its end.
+void issue_wave_paths(Issue& I) {
+    Wave& w = I.w;
+    cudaMemsetAsync(w.counts, 0, 64, I.st);
+    I.emit(false, w.ps[0], queue_counts(w, 0));
+    I.trace(w.ps[0], queue_counts(w, 0));
+    I.shadow();
+}
+
 // A streaming pass: the prologue fills the first queue (ps[0]); a half-iteration traces queue
 // `a` and leaves the next one in queue a ^ 1 (the survivors of shading, then the refill).  The
 // connections a half-iteration queues are traced by the next one, beside its closest-hit
@@ -2742,7 +3062,7 @@ void stream_prologue(Issue& I) {
     Wave& w = I.w;
     k_stream_init<<<1, 32, 0, I.st>>>(w);
     I.emit(true, w.ps[0], queue_counts(w, 0));
-    k_stream_advance<<<1, 32, 0, I.st>>>(w, I.f, queue_counts(w, 1), queue_counts(w, 0), 0, 0);
+    k_stream_advance<<<1, 32, 0, I.st>>>(w, I.f, queue_counts(w, 1), queue_counts(w, 0), I.tail(), 0, 0);
 }
 void stream_connections(Issue& I) {
     I.shadow();
@@ -2781,13 +3101,30 @@ void stream_half(Issue& I, int a, cudaGraphConditionalHandle loop, int32_t set_l
     if (side) cudaStreamWaitEvent(I.st, side->join, 0);
     I.shade(w.ps[a], queue_counts(w, a), w.ps[a ^ 1], queue_counts(w, a ^ 1));
     I.emit(true, w.ps[a ^ 1], queue_counts(w, a ^ 1));
-    k_stream_advance<<<1, 32, 0, I.st>>>(w, I.f, queue_counts(w, a), queue_counts(w, a ^ 1), loop, set_loop);
+    k_stream_advance<<<1, 32, 0, I.st>>>(w, I.f, queue_counts(w, a), queue_counts(w, a ^ 1), I.tail(), loop, set_loop);
+}
+// After the loop: the last half-iteration's connections, the paths still queued (in ps[0]) to
+// their ends, and the connections those made.
+void stream_tail(Issue& I) {
+    stream_connections(I);
+    I.trace(I.w.ps[0], queue_counts(I.w, 0));
+    I.shadow();
+}
+// A pass of few photons: all of them emitted (their stream positions are the queue's), then
+// every path to its end.
+void stream_paths(Issue& I) {
+    Wave& w = I.w;
+    k_stream_init<<<1, 32, 0, I.st>>>(w);
+    I.emit(true, w.ps[0], queue_counts(w, 0));
+    k_stream_advance<<<1, 32, 0, I.st>>>(w, I.f, queue_counts(w, 1), queue_counts(w, 0), I.tail(), 0, 0);
+    I.trace(w.ps[0], queue_counts(w, 0));
+    I.shadow();
 }
 }  // namespace
 
 struct WaveGraphs {
     struct Entry {
-        int32_t max_bounce, grid;   // max_bounce -1: a streaming pass
+        int32_t max_bounce, grid;   // max_bounce -1: a streaming pass, -2: one of few photons, -3: a wave of few
         bool inst, hero, media, shapes, mirrors, sorted;
         int32_t* status;
         cudaGraphExec_t exec;
@@ -2820,24 +3157,30 @@ int launch_grid(const Wave& w, int32_t sms, const LaunchShape& shape) {
 }
 }  // namespace
 
+int32_t trace_limit(int32_t sms) { return sms * FTB_TRACE_MINB * Issue::T; }
+
 cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const Frame& f, int32_t sms,
-                        const LaunchShape& shape, cudaStream_t st, LaunchSink* sink, WaveGraphs* graphs) {
+                        const LaunchShape& shape, cudaStream_t st, LaunchSink* sink, WaveGraphs* graphs,
+                        bool whole_paths) {
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;   // the buffer carries no bundles
     const int grid = launch_grid(w, sms, shape);
     // A graph bakes the kernel arguments: the wave's buffers and status word are fixed for the
     // life of its cache, but a log buffer changes per call, so logging waves launch directly.
     if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
-        Issue I{w, kind, f, grid, shape.sort_rays, st, sink};
-        issue_wave(I, max_bounce);
+        Issue I{w, kind, f, grid, shape.sort_rays, st, sink, sms};
+        if (whole_paths) issue_wave_paths(I);
+        else issue_wave(I, max_bounce);
         return cudaGetLastError();
     }
+    if (whole_paths) max_bounce = -3;
     if (cudaGraphExec_t ex = graphs->find(max_bounce, grid, kind, shape.sort_rays, f.status))
         return cudaGraphLaunch(ex, st);
     cudaGraph_t g = nullptr;
     cudaError_t err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (err != cudaSuccess) return err;
-    Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr};
-    issue_wave(I, max_bounce);
+    Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr, sms};
+    if (whole_paths) issue_wave_paths(I);
+    else issue_wave(I, max_bounce);
     err = cudaStreamEndCapture(st, &g);
     if (err != cudaSuccess) return err;
     WaveGraphs::Entry e{max_bounce, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors,
@@ -2849,39 +3192,56 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
     return cudaGraphLaunch(e.exec, st);
 }
 
-cudaError_t launch_stream(Wave& w, const WaveKind& kind, const Frame& f, int32_t sms, const LaunchShape& shape,
-                          cudaStream_t st, LaunchSink* sink, WaveGraphs* graphs) {
+cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKind& kind, const Frame& f, int32_t sms,
+                          const LaunchShape& shape, cudaStream_t st, LaunchSink* sink, WaveGraphs* graphs) {
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;
     const int grid = launch_grid(w, sms, shape);
+    const bool few = !f.stats && photons <= std::min(slots, trace_limit(sms));
     if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
         // host-driven: the graph's loop body (two half-iterations) at a time, the progress
         // word read after each, so the launches are the ones a graph replay makes
-        Issue I{w, kind, f, grid, shape.sort_rays, st, sink};
+        Issue I{w, kind, f, grid, shape.sort_rays, st, sink, sms};
+        if (few) {
+            stream_paths(I);
+            return cudaGetLastError();
+        }
         stream_prologue(I);
         for (;;) {
-            stream_half(I, 0, 0, 0, nullptr);
-            stream_half(I, 1, 0, 0, nullptr);
             cudaError_t e = cudaGetLastError();
             int32_t more = 0;
             if (e == cudaSuccess) e = cudaMemcpyAsync(&more, &w.ctl->more, sizeof more, cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) return e;
             if (!more) {
-                I.shadow();
+                stream_tail(I);
                 return cudaGetLastError();
             }
+            stream_half(I, 0, 0, 0, nullptr);
+            stream_half(I, 1, 0, 0, nullptr);
         }
     }
-    if (cudaGraphExec_t ex = graphs->find(-1, grid, kind, shape.sort_rays, f.status)) return cudaGraphLaunch(ex, st);
+    const int32_t key = few ? -2 : -1;
+    if (cudaGraphExec_t ex = graphs->find(key, grid, kind, shape.sort_rays, f.status)) return cudaGraphLaunch(ex, st);
     // prologue, then a conditional while node whose body is two half-iterations (the queues
     // swap roles between them; the last advance of the body sets the loop condition), then the
-    // connections of the last one
-    Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr};
+    // paths still queued and the connections
+    Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr, sms};
+    WaveGraphs::Entry entry{key, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors,
+                            shape.sort_rays, f.status, nullptr};
     cudaGraph_t g = nullptr;
     cudaError_t err = graphs->side.init();
     if (err != cudaSuccess) return err;
     err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (err != cudaSuccess) return err;
+    if (few) {
+        stream_paths(I);
+        err = cudaStreamEndCapture(st, &g);
+        if (err == cudaSuccess) err = cudaGraphInstantiate(&entry.exec, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (err != cudaSuccess) return err;
+        graphs->entries.push_back(entry);
+        return cudaGraphLaunch(entry.exec, st);
+    }
     stream_prologue(I);
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t* deps = nullptr;
@@ -2899,7 +3259,7 @@ cudaError_t launch_stream(Wave& w, const WaveKind& kind, const Frame& f, int32_t
         err = cudaGraphAddNode(&node, g, deps, n_deps, &p);
     }
     if (err == cudaSuccess) err = cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies);
-    if (err == cudaSuccess) I.shadow();
+    if (err == cudaSuccess) stream_tail(I);
     cudaGraph_t captured = nullptr;
     cudaError_t end = cudaStreamEndCapture(st, &captured);
     if (err == cudaSuccess) err = end;
@@ -2915,13 +3275,11 @@ cudaError_t launch_stream(Wave& w, const WaveKind& kind, const Frame& f, int32_t
         cudaGraph_t b2 = nullptr;
         err = cudaStreamEndCapture(st, &b2);
     }
-    WaveGraphs::Entry e{-1, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors,
-                        shape.sort_rays, f.status, nullptr};
-    if (err == cudaSuccess) err = cudaGraphInstantiate(&e.exec, captured, 0);
+    if (err == cudaSuccess) err = cudaGraphInstantiate(&entry.exec, captured, 0);
     cudaGraphDestroy(captured);
     if (err != cudaSuccess) return err;
-    graphs->entries.push_back(e);
-    return cudaGraphLaunch(e.exec, st);
+    graphs->entries.push_back(entry);
+    return cudaGraphLaunch(entry.exec, st);
 }
 
 }  // namespace ftb

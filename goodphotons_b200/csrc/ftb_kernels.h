@@ -207,9 +207,16 @@ inline bool scene_has_shapes(const DevScene& sc) { return (int64_t)sc.n_recs > s
 // counting (f.stats) and logging (w.logs) launches are issued directly.  A cache's graphs
 // hold the addresses of its wave buffer and status word: destroy the cache when either
 // changes.
+// With `whole_paths`, every path is traced to its end by one launch instead (for waves of at
+// most trace_limit() slots: three kernels rather than three per bounce).
 cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const Frame& f, int32_t sms,
                         const LaunchShape& shape, cudaStream_t stream, LaunchSink* sink = nullptr,
-                        WaveGraphs* graphs = nullptr);
+                        WaveGraphs* graphs = nullptr, bool whole_paths = false);
+
+// Paths that the whole-path kernels hold at once, one per resident lane.  A streaming pass
+// whose queue is no longer than this, with no photon left to refill, ends with one whole-path
+// launch; a pass of no more photons is emission, that launch and its connections.
+int32_t trace_limit(int32_t sms);
 
 // Trace a streaming pass on `stream`: the caller has written the table of photon ranges to
 // w.jobs (g0 consecutive from 0) and w.params = {ranges, slots, photons (int64 at [1]),
@@ -217,11 +224,13 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
 // half-iteration runs closest hit beside the connections queued so far, shading (the
 // survivors are compacted into the other path buffer) and a refill that appends the next
 // photons of the pass up to `slots` paths, until every photon is done; then the last
-// connections.  With `graphs` and shape.graph the loop is one
+// connections.  The last trace_limit() paths are traced to their ends by one launch; a pass
+// of no more `photons` than that and `slots` is only that.  With `graphs` and shape.graph the loop is one
 // graph launch (a conditional while node whose condition the device sets); otherwise the
 // host issues half-iterations in groups and reads the progress word between groups.
-cudaError_t launch_stream(Wave& w, const WaveKind& kind, const Frame& f, int32_t sms, const LaunchShape& shape,
-                          cudaStream_t stream, LaunchSink* sink = nullptr, WaveGraphs* graphs = nullptr);
+cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKind& kind, const Frame& f, int32_t sms,
+                          const LaunchShape& shape, cudaStream_t stream, LaunchSink* sink = nullptr,
+                          WaveGraphs* graphs = nullptr);
 
 // Half-iterations a streaming pass of `photons` with `slots` paths in flight can need: a
 // path ends within max_bounce half-iterations and its place is refilled in the one it ends

@@ -157,7 +157,8 @@ extern "C" ftb_status ftb_render_forward_noalloc(ftb_scene* scene, const ftb_cam
     kind.media = dev.n_med > 0;
     kind.shapes = ftb::scene_has_shapes(dev);
     kind.mirrors = dev.n_planes > 0;
-    if (e == cudaSuccess && p->n_photons > 0) e = ftb::launch_wave(w, p->max_bounce, kind, f, sms, shape, st);
+    if (e == cudaSuccess && p->n_photons > 0)
+        e = ftb::launch_wave(w, p->max_bounce, kind, f, sms, shape, st, nullptr, nullptr, true);
     if (e != cudaSuccess) out = na_fail(FTB_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     if (out == FTB_OK && info) {
         info->frac_bits = frac;

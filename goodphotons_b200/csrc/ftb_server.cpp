@@ -419,7 +419,8 @@ void scheduler(ftb_server* s) {
         f.stats = nullptr;
         f.status = s->d_status + 16 * b;
         if (e == cudaSuccess)
-            e = stream ? ftb::launch_stream(w.wave, kind, f, s->sms, s->shape, w.stream, nullptr, w.graphs)
+            e = stream ? ftb::launch_stream(w.wave, photons, slots, kind, f, s->sms, s->shape, w.stream, nullptr,
+                                            w.graphs)
                        : ftb::launch_wave(w.wave, mb, kind, f, s->sms, s->shape, w.stream, nullptr, w.graphs);
         if (e == cudaSuccess) e = cudaEventRecord(w.done, w.stream);
         {
