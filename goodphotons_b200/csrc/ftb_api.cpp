@@ -807,6 +807,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
+        kind.multi = table.size() > 1;
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                s->eng->graphs[k & 1]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
@@ -857,6 +858,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
+        kind.multi = table.size() > 1;
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                              s->eng->graphs[k & 1]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");

@@ -1304,15 +1304,20 @@ enum { T_EMIT = 0, T_ABS = 1, T_SENSOR = 2, T_ESC = 3, T_RES = 4 };
 // in shared memory (one row of five per job of the table) whenever the job of the path it
 // books changes -- often, in a streaming pass, where the paths of neighbouring jobs share
 // the queues -- and the block adds the table's nonzero entries to the jobs' tallies once
-// at the end, so the global atomics per launch do not grow with the job changes.
+// at the end, so the global atomics per launch do not grow with the job changes.  The table
+// is dynamic shared memory, given to launches of many jobs only: eight resident blocks' tables
+// take 82 KB of the SM's storage from the L1 that holds these kernels' spills (shading of a
+// frame of one job with the table / without it, B200: Cornell 4.67 / 4.34 ms, glass 54.7 /
+// 52.4, Cornell bundles 1.92 / 1.82).
+constexpr size_t kTallyBytes = sizeof(unsigned long long) * kWaveJobs * 5;
 struct TallyAcc {
     int job;
     bool multi;
     long long v[5];
 };
 __device__ __forceinline__ unsigned long long* tally_table() {
-    __shared__ unsigned long long tab[kWaveJobs * 5];
-    return tab;
+    extern __shared__ unsigned long long dyn_tally[];   // kTallyBytes, launches of many jobs only
+    return dyn_tally;
 }
 // Called by every thread of the block at the start of the kernel.
 __device__ __forceinline__ void tally_init(TallyAcc& a, bool multi, int n_jobs) {
@@ -2911,6 +2916,7 @@ struct Issue {
     static constexpr int T = 128;
 
     // paths left to the whole-path kernels, which have no counting variant
+    size_t tally() const { return kind.multi ? kTallyBytes : 0; }   // dynamic shared memory of the tally kernels
     int32_t tail() const { return f.stats ? 0 : trace_limit(sms); }
 
     void mark(int k, bool end) { if (sink) sink->mark(k, end, st); }
@@ -2918,11 +2924,11 @@ struct Issue {
         mark(K_EMIT, false);
         const DevJob* jobs = w.jobs;
 #define FTB_EMIT_HERO(S) \
-    (kind.mirrors ? k_emit_hero<S, true><<<grid, T, 0, st>>>(w, jobs, f, out, co) \
-                  : k_emit_hero<S, false><<<grid, T, 0, st>>>(w, jobs, f, out, co))
+    (kind.mirrors ? k_emit_hero<S, true><<<grid, T, tally(), st>>>(w, jobs, f, out, co) \
+                  : k_emit_hero<S, false><<<grid, T, tally(), st>>>(w, jobs, f, out, co))
 #define FTB_EMIT(M, S) \
-    (kind.mirrors ? k_emit<M, S, true><<<grid, T, 0, st>>>(w, jobs, f, out, co) \
-                  : k_emit<M, S, false><<<grid, T, 0, st>>>(w, jobs, f, out, co))
+    (kind.mirrors ? k_emit<M, S, true><<<grid, T, tally(), st>>>(w, jobs, f, out, co) \
+                  : k_emit<M, S, false><<<grid, T, tally(), st>>>(w, jobs, f, out, co))
         if (stream) {
             if (kind.bundles) FTB_EMIT_HERO(true);
             else if (kind.media) FTB_EMIT(true, true);
@@ -2960,7 +2966,7 @@ struct Issue {
         const DevJob* jobs = w.jobs;
         const int g = sms * FTB_TRACE_MINB;
         mark(K_EXTEND, false);
-#define FTB_TRACE(...) __VA_ARGS__<<<g, T, 0, st>>>(w, jobs, f, in, c)
+#define FTB_TRACE(...) __VA_ARGS__<<<g, T, tally(), st>>>(w, jobs, f, in, c)
 #define FTB_TRACE_SET(...) \
     if (inst) { if (shp) FTB_TRACE(__VA_ARGS__ true, true, false>); else FTB_TRACE(__VA_ARGS__ true, false, false>); } \
     else { if (shp) FTB_TRACE(__VA_ARGS__ false, true, false>); else FTB_TRACE(__VA_ARGS__ false, false, false>); }
@@ -2993,7 +2999,7 @@ struct Issue {
         const bool inst = kind.instances, shp = kind.shapes;
         const DevJob* jobs = w.jobs;
         mark(K_SHADE, false);
-#define FTB_SHADE(...) __VA_ARGS__<<<grid, T, 0, st>>>(w, jobs, f, in, ci, out, co)
+#define FTB_SHADE(...) __VA_ARGS__<<<grid, T, tally(), st>>>(w, jobs, f, in, ci, out, co)
         if (kind.bundles && kind.mirrors) {
             if (inst) { if (shp) FTB_SHADE(k_shade_hero<true, true, true>); else FTB_SHADE(k_shade_hero<true, false, true>); }
             else { if (shp) FTB_SHADE(k_shade_hero<false, true, true>); else FTB_SHADE(k_shade_hero<false, false, true>); }
@@ -3125,7 +3131,7 @@ void stream_paths(Issue& I) {
 struct WaveGraphs {
     struct Entry {
         int32_t max_bounce, grid;   // max_bounce -1: a streaming pass, -2: one of few photons, -3: a wave of few
-        bool inst, hero, media, shapes, mirrors, sorted;
+        bool inst, hero, media, shapes, mirrors, multi, sorted;
         int32_t* status;
         cudaGraphExec_t exec;
     };
@@ -3137,7 +3143,8 @@ struct WaveGraphs {
     cudaGraphExec_t find(int32_t max_bounce, int32_t grid, const WaveKind& kind, bool sorted, int32_t* status) const {
         for (auto& e : entries)
             if (e.max_bounce == max_bounce && e.grid == grid && e.inst == kind.instances && e.hero == kind.bundles &&
-                e.media == kind.media && e.shapes == kind.shapes && e.mirrors == kind.mirrors && e.sorted == sorted &&
+                e.media == kind.media && e.shapes == kind.shapes && e.mirrors == kind.mirrors &&
+                e.multi == kind.multi && e.sorted == sorted &&
                 e.status == status)
                 return e.exec;
         return nullptr;
@@ -3183,7 +3190,7 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
     else issue_wave(I, max_bounce);
     err = cudaStreamEndCapture(st, &g);
     if (err != cudaSuccess) return err;
-    WaveGraphs::Entry e{max_bounce, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors,
+    WaveGraphs::Entry e{max_bounce, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors, kind.multi,
                         shape.sort_rays, f.status, nullptr};
     err = cudaGraphInstantiate(&e.exec, g, 0);
     cudaGraphDestroy(g);
@@ -3226,7 +3233,7 @@ cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKin
     // swap roles between them; the last advance of the body sets the loop condition), then the
     // paths still queued and the connections
     Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr, sms};
-    WaveGraphs::Entry entry{key, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors,
+    WaveGraphs::Entry entry{key, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors, kind.multi,
                             shape.sort_rays, f.status, nullptr};
     cudaGraph_t g = nullptr;
     cudaError_t err = graphs->side.init();

@@ -191,6 +191,7 @@ struct WaveKind {
     bool media = false;       // some scene has participating media
     bool shapes = false;      // some scene has spheres or curves (not only triangles)
     bool mirrors = false;     // some scene has planar mirrors (mirror connections queued)
+    bool multi = false;       // the table holds more than one job (it must say so exactly)
 };
 // Connection records one path vertex of job J can queue: a camera connection and one per
 // planar mirror, for each of the job's views.  A wave or pass keeps its slots at most
