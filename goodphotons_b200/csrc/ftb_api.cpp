@@ -657,6 +657,7 @@ DevCam dev_cam(const ftb_camera* c) {
     DevCam d;
     for (int i = 0; i < 3; ++i) { d.eye[i] = c->eye[i]; d.u[i] = c->u[i]; d.v[i] = c->v[i]; d.w[i] = c->w[i]; }
     d.thx = c->tan_half_x; d.thy = c->tan_half_y; d.rx = c->res_x; d.ry = c->res_y;
+    cam_finish(d);
     return d;
 }
 
@@ -720,7 +721,7 @@ ftb::DevJob make_job(const ftb_scene* s, const ftb_camera* cam, int64_t* d_film,
     J.tally_scale_inv = std::ldexp(1.0, 32) / s->power;
     J.max_bounce = max_bounce;
     J.hero_c = effective_hero(s, hero_c);
-    J.lambda_mode = lambda_mode;
+    J.lambda_mode = (int16_t)lambda_mode;
     return J;
 }
 
@@ -780,7 +781,6 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             ftb::DevJob J = base[j];
             J.photon0 = seed[j] + (uint64_t)done_in_job;
             J.g0 = g;
-            J.slot0 = 0;
             J.n = (int32_t)m;
             table.push_back(J);
             max_bounce = std::max(max_bounce, J.max_bounce);
@@ -833,7 +833,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             int32_t m = (int32_t)std::min<int64_t>(left, (int64_t)(cap - slots));
             ftb::DevJob J = base[j];
             J.photon0 = seed[j] + (uint64_t)done_in_job;
-            J.slot0 = slots;
+            J.g0 = slots;
             J.n = m;
             table.push_back(J);
             max_bounce = std::max(max_bounce, J.max_bounce);
@@ -1914,7 +1914,7 @@ ftb_status ftb_session_batch(ftb_session* ss, int64_t n, uint64_t seed_base) {
     // path vertex connects to each camera; the paths are traced once.
     ftb::DevJob J = make_job(s, &ss->cams[0], ss->films[0], ss->tally, ss->frac_bits, ss->max_bounce, ss->hero_c);
     J.views = ss->views;
-    J.n_views = (int32_t)ss->cams.size();
+    J.n_views = (uint16_t)ss->cams.size();
     st = run_jobs(s, {J}, {n}, {seed_base}, false, nullptr, 0, nullptr);
     if (st != FTB_OK) return st;
     CK(cudaDeviceSynchronize(), "session batch");

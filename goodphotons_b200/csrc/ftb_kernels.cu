@@ -1025,9 +1025,34 @@ __device__ __forceinline__ bool cam_project(const DevCam& c, D3 p, int& px, int&
     return true;
 }
 __device__ __forceinline__ double cam_pixel_solid_angle(const DevCam& c, double cos_cam) {
-    double ipa = 4.0 * c.thx * c.thy;
-    double ppa = ipa / ((double)c.rx * (double)c.ry);
-    return ppa * cos_cam * cos_cam * cos_cam;
+    return c.ppa * cos_cam * cos_cam * cos_cam;
+}
+// The connection p -> eye (connectGeom, render.h:499-520): unit direction, distance and, if
+// the point projects into the image, its pixel and cosine.  Camera::project works on
+// p - eye, the exact negative of eye - p, so its squared length and distance are those of the
+// connection: one square root and four divisions fewer per connection than projecting afresh
+// (shading, B200: Cornell 4.19 -> 4.00 ms, glass 51.0 -> 49.2, showroom 15.6 -> 15.2).
+struct EyeRay { D3 to, dir; double dist2, dist; };
+__device__ __forceinline__ EyeRay eye_ray(const DevCam& c, D3 p) {
+    EyeRay e;
+    e.to = ld3(c.eye) - p;
+    e.dist2 = dot(e.to, e.to);
+    e.dist = sqrt(e.dist2);
+    e.dir = e.to / e.dist;
+    return e;
+}
+__device__ __forceinline__ bool eye_project(const DevCam& c, const EyeRay& e, int& px, int& py, double& cos_cam) {
+    const D3 d = neg(e.to);
+    const double cz = dot(d, ld3(c.w));
+    if (cz <= 1e-9) return false;
+    const double cx = dot(d, ld3(c.u)), cy = dot(d, ld3(c.v));
+    const double ix = (cx / cz) / c.thx - 0.0;
+    const double iy = (cy / cz) / c.thy;
+    if (ix < -1 || ix >= 1 || iy < -1 || iy >= 1) return false;
+    px = (int)((ix * 0.5 + 0.5) * c.rx);
+    py = (int)((iy * 0.5 + 0.5) * c.ry);
+    cos_cam = cz / e.dist;
+    return true;
 }
 
 // geometry.h:174-242
@@ -1138,15 +1163,15 @@ __device__ void connect_surface(const DevScene& sc, const DevJob& J, const Q& w,
                                 D3 p, D3 n, D3 ng, D3 wi, double lam, const double* cie, double beta, double rho) {
     for (int v = 0; v < view_count(J); ++v) {
         const DevCam& cam = view_cam(J, v);
-        D3 to_cam = ld3(cam.eye) - p;
-        double dist = len(to_cam);
-        D3 wdir = to_cam / dist;
+        const EyeRay er = eye_ray(cam, p);
+        const D3 wdir = er.dir;
+        const double dist = er.dist, dist2 = er.dist2;
         double cos_surf = dot(n, wdir);
         if (cos_surf <= 0) continue;
         double stg = shadow_terminator_g(wdir, n, ng);
         if (stg <= 0.0) continue;
-        int px, py; double cos_cam, dist2;
-        if (!cam_project(cam, p, px, py, cos_cam, dist2)) continue;
+        int px, py; double cos_cam;
+        if (!eye_project(cam, er, px, py, cos_cam)) continue;
         double omega = cam_pixel_solid_angle(cam, cos_cam);
         double corr = shading_adjoint_corr(wi, wdir, n, ng);
         double denom = dist2 * omega;
@@ -1162,11 +1187,11 @@ __device__ void connect_volume(const DevScene& sc, const DevJob& J, const Q& w, 
                                const DevMed& m, D3 p, D3 win, double lam, const double* cie, double beta) {
     for (int v = 0; v < view_count(J); ++v) {
         const DevCam& cam = view_cam(J, v);
-        D3 to_cam = ld3(cam.eye) - p;
-        double dist = len(to_cam);
-        D3 wdir = to_cam / dist;
-        int px, py; double cos_cam, dist2;
-        if (!cam_project(cam, p, px, py, cos_cam, dist2)) continue;
+        const EyeRay er = eye_ray(cam, p);
+        const D3 wdir = er.dir;
+        const double dist = er.dist, dist2 = er.dist2;
+        int px, py; double cos_cam;
+        if (!eye_project(cam, er, px, py, cos_cam)) continue;
         double ph = hg_phase(dot(win, wdir), m.g);
         double alb = med_albedo(sc, m, lam);
         double omega = cam_pixel_solid_angle(cam, cos_cam);
@@ -1416,7 +1441,7 @@ __device__ __forceinline__ void log_move(const Wave& w, const PathState& in, int
     for (int q = 0; q < 8; ++q) out.lprims[q * w.W + o] = in.lprims[q * w.W + i];
 }
 
-// Photon sources of the emission kernels.  A wave emits photon photon0 + (t - slot0) of the
+// Photon sources of the emission kernels.  A wave emits photon photon0 + (t - g0) of the
 // table range holding t, for t < params[1]; a streaming pass's refill emits stream indices
 // next .. next+F-1, F = the free places (slots less the survivors already queued, at most the
 // photons left), each mapped to its range's photon.
@@ -1458,10 +1483,10 @@ __device__ __forceinline__ int photon_job(const DevJob* __restrict__ jobs, int n
         const int slot = (int)t;
         if (n_jobs > 1) {
             int lo = 0, hi = n_jobs - 1;
-            while (lo < hi) { int mid = (lo + hi + 1) / 2; if (jobs[mid].slot0 <= slot) lo = mid; else hi = mid - 1; }
+            while (lo < hi) { int mid = (lo + hi + 1) / 2; if (jobs[mid].g0 <= slot) lo = mid; else hi = mid - 1; }
             j = lo;
         }
-        photon = jobs[j].photon0 + (uint64_t)(slot - jobs[j].slot0);
+        photon = jobs[j].photon0 + (uint64_t)(slot - jobs[j].g0);
     }
     return j;
 }
@@ -2174,15 +2199,15 @@ __device__ void connect_surface_hero(const DevJob& J, const Q& w, const Frame& f
                                      int nup) {
     for (int v = 0; v < view_count(J); ++v) {
         const DevCam& cam = view_cam(J, v);
-        D3 to_cam = ld3(cam.eye) - p;
-        double dist = len(to_cam);
-        D3 wdir = to_cam / dist;
+        const EyeRay er = eye_ray(cam, p);
+        const D3 wdir = er.dir;
+        const double dist = er.dist, dist2 = er.dist2;
         double cos_surf = dot(n, wdir);
         if (cos_surf <= 0) continue;
         double stg = shadow_terminator_g(wdir, n, ng);
         if (stg <= 0.0) continue;
-        int px, py; double cos_cam, dist2;
-        if (!cam_project(cam, p, px, py, cos_cam, dist2)) continue;
+        int px, py; double cos_cam;
+        if (!eye_project(cam, er, px, py, cos_cam)) continue;
         double omega = cam_pixel_solid_angle(cam, cos_cam);
         double corr = shading_adjoint_corr(wi, wdir, n, ng);
         double denom = dist2 * omega;

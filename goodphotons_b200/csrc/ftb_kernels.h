@@ -28,7 +28,7 @@ struct DevView {
 };
 
 // One job's share of a wave: its scene, camera(s) and film(s), and the slots
-// [slot0, slot0+n) of the wave that trace its photons photon0, photon0+1, ...  In a
+// [g0, g0+n) of the wave that trace its photons photon0, photon0+1, ...  In a
 // streaming pass the table is a list of photon ranges instead: the pass hands out photons
 // g = 0, 1, ... in order, and g in [g0, g0+n) is this job's photon photon0 + (g - g0).
 struct DevJob {
@@ -36,16 +36,16 @@ struct DevJob {
     DevCam cam;
     int64_t* film;             // 4 words per pixel
     const DevView* views;      // n_views > 1: every vertex connects to each view (shared splat)
-    int32_t n_views;
-    int32_t lambda_mode;       // ftb_lambda_mode of the job's photons
     unsigned long long* tally; // 5 fixed-point energy tallies
     double film_scale_inv;     // 2^frac / power_ref
     double tally_scale_inv;    // 2^32 / power_ref
     uint64_t photon0;
-    int64_t g0;                // streaming pass: first stream index of this range
-    int32_t slot0, n;
+    int64_t g0;                // first stream index of this range; in a wave, its first slot
+    int32_t n;
     int32_t max_bounce;
     int32_t hero_c;            // wavelengths per photon (1: the scalar tracer)
+    uint16_t n_views;          // at most 65535 (a connection's view field has 16 bits)
+    int16_t lambda_mode;       // ftb_lambda_mode of the job's photons
 };
 
 // Progress of a streaming pass (device memory, updated by k_stream_advance).

@@ -145,5 +145,11 @@ struct DevScene {
 struct DevCam {
     double eye[3], u[3], v[3], w[3];
     double thx, thy;
+    double ppa;               // image-plane area of a pixel, 4 thx thy / (rx ry)
     int32_t rx, ry;
 };
+// Camera::pixelSolidAngle's first two lines (camera.h), the same for every connection.
+static inline void cam_finish(DevCam& c) {
+    const double ipa = 4.0 * c.thx * c.thy;
+    c.ppa = ipa / ((double)c.rx * (double)c.ry);
+}

@@ -138,15 +138,16 @@ extern "C" ftb_status ftb_render_forward_noalloc(ftb_scene* scene, const ftb_cam
         J.cam.eye[i] = cam->eye[i]; J.cam.u[i] = cam->u[i]; J.cam.v[i] = cam->v[i]; J.cam.w[i] = cam->w[i];
     }
     J.cam.thx = cam->tan_half_x; J.cam.thy = cam->tan_half_y; J.cam.rx = cam->res_x; J.cam.ry = cam->res_y;
+    cam_finish(J.cam);
     J.film = d_film;
     J.tally = tally;
     J.film_scale_inv = std::ldexp(1.0, frac) / power;
     J.tally_scale_inv = std::ldexp(1.0, 32) / power;
     J.photon0 = p->seed_base;
-    J.slot0 = 0;
+    J.g0 = 0;
     J.n = (int32_t)p->n_photons;
     J.max_bounce = p->max_bounce;
-    J.lambda_mode = p->lambda_mode;
+    J.lambda_mode = (int16_t)p->lambda_mode;
     ftb_status out = FTB_OK;
     k_noalloc_stage<<<1, 32, 0, st>>>(J, w.jobs, w.params, tally, status);
     cudaError_t e = cudaGetLastError();

@@ -321,12 +321,11 @@ int64_t build_table_locked(ftb_server* s, std::vector<ftb::DevJob>& table, std::
         J.film_scale_inv = std::ldexp(1.0, j->frac) / j->power;
         J.tally_scale_inv = std::ldexp(1.0, 32) / j->power;
         J.photon0 = j->req.seed_base + (uint64_t)j->next;
-        J.g0 = photons;                // stream index of a streaming pass
-        J.slot0 = (int32_t)photons;    // first slot of a wave
+        J.g0 = photons;                // stream index of a streaming pass, or first slot of a wave
         J.n = (int32_t)give[i];
         J.max_bounce = j->req.max_bounce;
         J.hero_c = j->hero;
-        J.lambda_mode = j->req.lambda_mode;
+        J.lambda_mode = (int16_t)j->req.lambda_mode;
         table.push_back(J);
         members.push_back(j);
         j->next += give[i];
