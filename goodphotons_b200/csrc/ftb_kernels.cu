@@ -53,14 +53,23 @@ namespace cg = cooperative_groups;
 #ifndef FTB_TRAV_MINB
 #define FTB_TRAV_MINB 8
 #endif
+#ifndef FTB_EXTEND_TRI_MINB    // closest hit of triangles only, 72 registers (glass 126.5 ms at 7
+                               // blocks against 129.7 at 8 and at 6; curves 59.4 at 8, 61.1 at 7)
+#define FTB_EXTEND_TRI_MINB 7
+#endif
 #ifndef FTB_SHADE_MINB
 #define FTB_SHADE_MINB 8
+#endif
+#ifndef FTB_SHADE_HERO_MINB    // bundles: their wavelength arrays want the registers (Cornell 1.62 ms
+                               // at 6 blocks, 1.77 at 8, 1.72 at 5)
+#define FTB_SHADE_HERO_MINB 6
 #endif
 #ifndef FTB_TRACE_MINB         // whole paths: registers for traversal and shading at once
 #define FTB_TRACE_MINB 4
 #endif
-#ifndef FTB_SHADE_MEDIA_MINB   // shading with participating media: more registers pay off
-#define FTB_SHADE_MEDIA_MINB 4
+#ifndef FTB_SHADE_MEDIA_MINB   // shading with participating media: more registers pay off (fog +
+                               // strands 22.5 ms at 5 blocks, 23.6 at 4)
+#define FTB_SHADE_MEDIA_MINB 5
 #endif
 
 namespace ftb {
@@ -1622,7 +1631,7 @@ __device__ void block_add1(unsigned long long* dst, unsigned long long a) {
 
 
 template <bool COUNT, bool INST, bool SHAPES>
-__global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_extend(Wave w, const DevJob* __restrict__ jobs,
+__global__ void __launch_bounds__(128, INST || SHAPES ? FTB_TRAV_MINB : FTB_EXTEND_TRI_MINB) k_extend(Wave w, const DevJob* __restrict__ jobs,
                                                               PathState in, const int32_t* qcount,
                                                               const int32_t* __restrict__ order, Frame f) {
     const int32_t n_jobs = w.params[0];
@@ -2483,7 +2492,7 @@ __device__ __forceinline__ int shade_bounce_hero(const DevScene& sc, const DevJo
 }
 
 template <bool INST, bool SHAPES, bool MIRROR>
-__global__ void __launch_bounds__(128, FTB_SHADE_MINB) k_shade_hero(Wave w, const DevJob* __restrict__ jobs,
+__global__ void __launch_bounds__(128, FTB_SHADE_HERO_MINB) k_shade_hero(Wave w, const DevJob* __restrict__ jobs,
                                                                     Frame f, PathState in, const int32_t* in_count,
                                                                     PathState out, int32_t* out_count) {
     const int32_t n_jobs = w.params[0];
