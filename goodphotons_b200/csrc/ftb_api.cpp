@@ -763,7 +763,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         table.clear();
         int64_t g = 0;
         int32_t max_bounce = 0, slots = W;
-        bool inst = false, media = false, shapes = false, mirrors = false;
+        bool inst = false, media = false, shapes = false, mirrors = false, deep = false;
         int bundles = -1, views = -1;
         while (j < base.size() && (int)table.size() < ftb::kWaveJobs) {
             const int64_t left = count[j] - done_in_job;
@@ -788,6 +788,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             media |= J.sc.n_med > 0;
             shapes |= ftb::scene_has_shapes(J.sc);
             mirrors |= J.sc.n_planes > 0;
+            deep |= ftb::scene_is_deep(J.sc);
             g += m;
             done_in_job += m;
             if (done_in_job >= count[j]) { ++j; done_in_job = 0; }
@@ -807,6 +808,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
+        kind.deep = deep;
         kind.multi = table.size() > 1;
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                s->eng->graphs[k & 1]);
@@ -816,7 +818,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
     while (j < base.size()) {
         table.clear();
         int32_t slots = 0, max_bounce = 0;
-        bool inst = false, media = false, shapes = false, mirrors = false;
+        bool inst = false, media = false, shapes = false, mirrors = false, deep = false;
         int bundles = -1;   // a wave holds either one-wavelength jobs or bundles, not both
         // A path queues at most 2 connections per view (and per mirror) per bounce, so a wave
         // of jobs with a fan-out of F connections per vertex carries W / F slots.
@@ -841,6 +843,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             media |= J.sc.n_med > 0;
             shapes |= ftb::scene_has_shapes(J.sc);
             mirrors |= J.sc.n_planes > 0;
+            deep |= ftb::scene_is_deep(J.sc);
             slots += m;
             done_in_job += m;
             if (done_in_job >= count[j]) { ++j; done_in_job = 0; }
@@ -858,6 +861,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
+        kind.deep = deep;
         kind.multi = table.size() > 1;
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                              s->eng->graphs[k & 1]);

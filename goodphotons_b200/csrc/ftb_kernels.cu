@@ -3205,27 +3205,28 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
                         bool whole_paths) {
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;   // the buffer carries no bundles
     const int grid = launch_grid(w, sms, shape);
+    const bool sorted = shape.sort_rays || kind.deep;
     // A graph bakes the kernel arguments: the wave's buffers and status word are fixed for the
     // life of its cache, but a log buffer changes per call, so logging waves launch directly.
     if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
-        Issue I{w, kind, f, grid, shape.sort_rays, st, sink, sms};
+        Issue I{w, kind, f, grid, sorted, st, sink, sms};
         if (whole_paths) issue_wave_paths(I);
         else issue_wave(I, max_bounce);
         return cudaGetLastError();
     }
     if (whole_paths) max_bounce = -3;
-    if (cudaGraphExec_t ex = graphs->find(max_bounce, grid, kind, shape.sort_rays, f.status))
+    if (cudaGraphExec_t ex = graphs->find(max_bounce, grid, kind, sorted, f.status))
         return cudaGraphLaunch(ex, st);
     cudaGraph_t g = nullptr;
     cudaError_t err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (err != cudaSuccess) return err;
-    Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr, sms};
+    Issue I{w, kind, f, grid, sorted, st, nullptr, sms};
     if (whole_paths) issue_wave_paths(I);
     else issue_wave(I, max_bounce);
     err = cudaStreamEndCapture(st, &g);
     if (err != cudaSuccess) return err;
     WaveGraphs::Entry e{max_bounce, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors, kind.multi,
-                        shape.sort_rays, f.status, nullptr};
+                        sorted, f.status, nullptr};
     err = cudaGraphInstantiate(&e.exec, g, 0);
     cudaGraphDestroy(g);
     if (err != cudaSuccess) return err;
@@ -3237,11 +3238,12 @@ cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKin
                           const LaunchShape& shape, cudaStream_t st, LaunchSink* sink, WaveGraphs* graphs) {
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;
     const int grid = launch_grid(w, sms, shape);
+    const bool sorted = shape.sort_rays || kind.deep;
     const bool few = !f.stats && photons <= std::min(slots, trace_limit(sms));
     if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
         // host-driven: the graph's loop body (two half-iterations) at a time, the progress
         // word read after each, so the launches are the ones a graph replay makes
-        Issue I{w, kind, f, grid, shape.sort_rays, st, sink, sms};
+        Issue I{w, kind, f, grid, sorted, st, sink, sms};
         if (few) {
             stream_paths(I);
             return cudaGetLastError();
@@ -3262,13 +3264,13 @@ cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKin
         }
     }
     const int32_t key = few ? -2 : -1;
-    if (cudaGraphExec_t ex = graphs->find(key, grid, kind, shape.sort_rays, f.status)) return cudaGraphLaunch(ex, st);
+    if (cudaGraphExec_t ex = graphs->find(key, grid, kind, sorted, f.status)) return cudaGraphLaunch(ex, st);
     // prologue, then a conditional while node whose body is two half-iterations (the queues
     // swap roles between them; the last advance of the body sets the loop condition), then the
     // paths still queued and the connections
-    Issue I{w, kind, f, grid, shape.sort_rays, st, nullptr, sms};
+    Issue I{w, kind, f, grid, sorted, st, nullptr, sms};
     WaveGraphs::Entry entry{key, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors, kind.multi,
-                            shape.sort_rays, f.status, nullptr};
+                            sorted, f.status, nullptr};
     cudaGraph_t g = nullptr;
     cudaError_t err = graphs->side.init();
     if (err != cudaSuccess) return err;

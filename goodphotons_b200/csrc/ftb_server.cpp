@@ -337,6 +337,7 @@ int64_t build_table_locked(ftb_server* s, std::vector<ftb::DevJob>& table, std::
         kind.media |= J.sc.n_med > 0;
         kind.shapes |= ftb::scene_has_shapes(J.sc);
         kind.mirrors |= J.sc.n_planes > 0;
+        kind.deep |= ftb::scene_is_deep(J.sc);
         fanout = std::max(fanout, ftb::conn_fanout(J));
     }
     return photons;
