@@ -661,26 +661,38 @@ DevCam dev_cam(const ftb_camera* c) {
     return d;
 }
 
+// The first wave buffer, of at least W paths.  The second is made when a render has a second
+// wave or pass to put in it (ensure_second_wave).
 ftb_status ensure_waves(ftb_scene* s, int32_t W, bool log, int32_t hero = 1) {
-    if (s->eng->wave_W >= W && s->eng->wave_log == log && s->eng->waves[0].block && s->eng->waves[0].hero >= hero)
-        return FTB_OK;
-    hero = std::max(hero, s->eng->waves[0].block ? s->eng->waves[0].hero : 1);   // keep the bundle room
-    if (s->eng->wave_log == log) W = std::max(W, s->eng->wave_W);
-    for (auto& w : s->eng->waves) ftb::wave_free(w);
-    for (auto& g : s->eng->graphs) {   // captured graphs hold the old buffers' addresses
+    Engine& e = *s->eng;
+    if (e.wave_W >= W && e.wave_log == log && e.waves[0].block && e.waves[0].hero >= hero) return FTB_OK;
+    hero = std::max(hero, e.waves[0].block ? e.waves[0].hero : 1);   // keep the bundle room
+    if (e.wave_log == log) W = std::max(W, e.wave_W);
+    for (auto& w : e.waves) ftb::wave_free(w);
+    for (auto& g : e.graphs) {   // captured graphs hold the old buffers' addresses
         ftb::wave_graphs_destroy(g);
         g = ftb::wave_graphs_create();
     }
-    s->eng->wave_W = 0;
-    for (auto& w : s->eng->waves) {
-        cudaError_t e = ftb::wave_alloc(w, W, log, hero);
-        if (e != cudaSuccess) return cuda_fail(e, "wave allocation");
-    }
-    for (auto& st : s->eng->streams)
+    e.wave_W = 0;
+    cudaError_t err = ftb::wave_alloc(e.waves[0], W, log, hero);
+    if (err != cudaSuccess) return cuda_fail(err, "wave allocation");
+    for (auto& st : e.streams)
         if (!st) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream create");
-    for (auto& sg : s->eng->stage) CK(sg.init(), "job staging");
-    s->eng->wave_W = W;
-    s->eng->wave_log = log;
+    CK(e.stage[0].init(), "job staging");
+    e.wave_W = W;
+    e.wave_log = log;
+    return FTB_OK;
+}
+ftb_status ensure_second_wave(ftb_scene* s, int32_t W) {
+    Engine& e = *s->eng;
+    ftb::Wave& w = e.waves[1];
+    if (w.block && w.W >= W && w.hero >= e.waves[0].hero) return FTB_OK;
+    ftb::wave_free(w);
+    ftb::wave_graphs_destroy(e.graphs[1]);
+    e.graphs[1] = ftb::wave_graphs_create();
+    cudaError_t err = ftb::wave_alloc(w, W, e.wave_log, e.waves[0].hero);
+    if (err != cudaSuccess) return cuda_fail(err, "wave allocation");
+    CK(e.stage[1].init(), "job staging");
     return FTB_OK;
 }
 
@@ -728,6 +740,24 @@ ftb::DevJob make_job(const ftb_scene* s, const ftb_camera* cam, int64_t* d_film,
 // A piece of a job placed in one wave.
 struct Segment { int job; int64_t first; int32_t n; };
 
+constexpr int64_t kPieceMax = (int64_t)1 << 30;   // photons of one range of a streaming pass
+
+// Whether run_jobs makes one streaming pass of these jobs: few enough ranges, one class
+// (bundles or not) and one connection fan-out.
+bool one_pass(const ftb::LaunchShape& shape, const std::vector<ftb::DevJob>& base, const std::vector<int64_t>& count) {
+    if (!shape.regenerate) return false;
+    int64_t pieces = 0;
+    const ftb::DevJob* first = nullptr;
+    for (size_t j = 0; j < base.size(); ++j) {
+        if (count[j] <= 0) continue;
+        if (!first) first = &base[j];
+        if ((base[j].hero_c > 1) != (first->hero_c > 1) || ftb::conn_fanout(base[j]) != ftb::conn_fanout(*first))
+            return false;
+        pieces += (count[j] + kPieceMax - 1) / kPieceMax;
+    }
+    return pieces <= ftb::kWaveJobs;
+}
+
 // Pack jobs' photon ranges into waves of at most W slots and kWaveJobs segments, launch
 // them alternately on the scene's two streams (handing off from and back to `user_stream`).
 // `base[j]` is job j's DevJob template; each segment gets its photon0 / slot range.
@@ -741,9 +771,14 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         hero = std::max(hero, base[i].hero_c);
         fanout = std::max(fanout, ftb::conn_fanout(base[i]));
     }
-    // a pass keeps W / fanout paths in flight, so few photons of a large fan-out get more room
-    int32_t W = pick_wave(std::min<int64_t>(total, s->eng->wave_cap) * fanout, s->eng->wave_cap);
-    ftb_status st = ensure_waves(s, W, log, hero);   // may keep larger buffers; waves use W slots
+    // A render that is one streaming pass has no second wave beside it, so its buffer takes the
+    // room of both: with twice the paths in flight a frame has half as many launches that end
+    // on their slowest warps (glass, 2^27 photons, 2^22 against 2^23 paths: 220.8 / 214.1 ms).
+    // A pass keeps W / fanout paths in flight, so few photons of a large fan-out get more room.
+    const int64_t cap = s->eng->wave_cap, room = one_pass(s->eng->shape, base, count) ? 2 * cap : cap;
+    int32_t W = pick_wave(std::min(total, room) * fanout, (int32_t)room);
+    ftb_status st = ensure_waves(s, W, log, hero);   // may keep a larger buffer; waves use W slots
+    if (st == FTB_ERR_OOM && W > cap) st = ensure_waves(s, W = (int32_t)cap, log, hero);
     if (st != FTB_OK) return st;
     ftb::Frame f;
     f.stats = s->prof_mode == 2 ? s->stats : nullptr;
@@ -777,7 +812,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             // refilled slot one more; the shadow queue holds 3W records, so a fan-out of F
             // connections per vertex gets W / F slots
             slots = std::max(1, W / nv);
-            const int64_t m = std::min<int64_t>(left, (int64_t)1 << 30);
+            const int64_t m = std::min<int64_t>(left, kPieceMax);
             ftb::DevJob J = base[j];
             J.photon0 = seed[j] + (uint64_t)done_in_job;
             J.g0 = g;
@@ -795,6 +830,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         }
         if (table.empty()) break;
         slots = (int32_t)std::min<int64_t>(slots, std::max<int64_t>(1, g));
+        if ((k & 1) && (st = ensure_second_wave(s, W)) != FTB_OK) return st;
         ftb::Wave& w = s->eng->waves[k & 1];
         cudaStream_t ws = s->eng->streams[k & 1];
         w.logs = d_logs;
@@ -849,6 +885,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             if (done_in_job >= count[j]) { ++j; done_in_job = 0; }
         }
         if (table.empty()) break;
+        if ((k & 1) && (st = ensure_second_wave(s, W)) != FTB_OK) return st;
         ftb::Wave& w = s->eng->waves[k & 1];
         cudaStream_t ws = s->eng->streams[k & 1];
         w.logs = d_logs;
