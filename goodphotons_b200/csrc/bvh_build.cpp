@@ -201,8 +201,10 @@ bool build_wide_bvh(const std::vector<Box>& boxes_in, double margin, WideBvh& ou
     const int n = (int)boxes_in.size();
     if (n == 0) return true;
     std::vector<Box> boxes(boxes_in);
-    for (auto& b : boxes)
-        for (int a = 0; a < 3; ++a) { b.lo[a] -= margin; b.hi[a] += margin; }
+    parallel_for(boxes.size(), [&](size_t i0, size_t i1) {
+        for (size_t i = i0; i < i1; ++i)
+            for (int a = 0; a < 3; ++a) { boxes[i].lo[a] -= margin; boxes[i].hi[a] += margin; }
+    });
     if (method == BuildMethod::kDeviceLbvh) return build_wide_lbvh_device(boxes, kLeafSize, device, out, err);
     std::vector<BinNode> nodes;
     std::vector<int> idx;
@@ -308,39 +310,41 @@ std::vector<FNode> widen_nodes(const WideBvh& bvh) {
     const std::vector<WNode>& nodes = bvh.nodes;
     const bool tight = bvh.planes.size() == nodes.size() * FTB_PLANES;
     std::vector<FNode> out(nodes.size());
-    for (size_t i = 0; i < nodes.size(); ++i) {
-        const WNode& w = nodes[i];
-        FNode& f = out[i];
-        f.child_base = w.child_base;
-        f.prim_base = w.prim_base;
-        f.pad[0] = f.pad[1] = 0;
-        const float p[3] = {w.px, w.py, w.pz};
-        const int eb[3] = {w.ex, w.ey, w.ez};
-        float sc[3] = {0.0f, 0.0f, 0.0f};
-        if (!tight)
-            for (int a = 0; a < 3; ++a) sc[a] = std::ldexp(1.0f, eb[a] - 127);
-        const uint8_t* qlo[3] = {w.qlo_x, w.qlo_y, w.qlo_z};
-        const uint8_t* qhi[3] = {w.qhi_x, w.qhi_y, w.qhi_z};
-        for (int k = 0; k < FTB_WIDTH; ++k) {
-            const uint8_t m = w.meta[k];
-            const bool inner = m != 0 && ((w.imask >> k) & 1u);
-            f.meta[k] = inner ? (uint8_t)((FNODE_INNER << 5) | (m & 31u)) : m;
-            f.code[k] = inner || !m ? (uint8_t)(m & 31u) : (uint8_t)(128u | ((m & 31u) << 2) | ((m >> 5) - 1u));
-            for (int a = 0; a < 3; ++a) {
-                const float s = sc[a];
-                if (!m) {
-                    f.lo[a][k] = INFINITY;
-                    f.hi[a][k] = -INFINITY;
-                } else if (tight) {
-                    f.lo[a][k] = bvh.planes[i * FTB_PLANES + 8 * a + k];
-                    f.hi[a][k] = bvh.planes[i * FTB_PLANES + 24 + 8 * a + k];
-                } else {
-                    f.lo[a][k] = plane(qlo[a][k], s, p[a]);
-                    f.hi[a][k] = plane(qhi[a][k], s, p[a]);
+    parallel_for(nodes.size(), [&](size_t i0, size_t i1) {
+        for (size_t i = i0; i < i1; ++i) {
+            const WNode& w = nodes[i];
+            FNode& f = out[i];
+            f.child_base = w.child_base;
+            f.prim_base = w.prim_base;
+            f.pad[0] = f.pad[1] = 0;
+            const float p[3] = {w.px, w.py, w.pz};
+            const int eb[3] = {w.ex, w.ey, w.ez};
+            float sc[3] = {0.0f, 0.0f, 0.0f};
+            if (!tight)
+                for (int a = 0; a < 3; ++a) sc[a] = std::ldexp(1.0f, eb[a] - 127);
+            const uint8_t* qlo[3] = {w.qlo_x, w.qlo_y, w.qlo_z};
+            const uint8_t* qhi[3] = {w.qhi_x, w.qhi_y, w.qhi_z};
+            for (int k = 0; k < FTB_WIDTH; ++k) {
+                const uint8_t m = w.meta[k];
+                const bool inner = m != 0 && ((w.imask >> k) & 1u);
+                f.meta[k] = inner ? (uint8_t)((FNODE_INNER << 5) | (m & 31u)) : m;
+                f.code[k] = inner || !m ? (uint8_t)(m & 31u) : (uint8_t)(128u | ((m & 31u) << 2) | ((m >> 5) - 1u));
+                for (int a = 0; a < 3; ++a) {
+                    const float s = sc[a];
+                    if (!m) {
+                        f.lo[a][k] = INFINITY;
+                        f.hi[a][k] = -INFINITY;
+                    } else if (tight) {
+                        f.lo[a][k] = bvh.planes[i * FTB_PLANES + 8 * a + k];
+                        f.hi[a][k] = bvh.planes[i * FTB_PLANES + 24 + 8 * a + k];
+                    } else {
+                        f.lo[a][k] = plane(qlo[a][k], s, p[a]);
+                        f.hi[a][k] = plane(qhi[a][k], s, p[a]);
+                    }
                 }
             }
         }
-    }
+    });
     return out;
 }
 

@@ -1,12 +1,38 @@
 // bvh_build.h -- host builder of the compressed 8-wide BVH.
 #pragma once
+#include <algorithm>
 #include <cfloat>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "ftb_layout.h"
 
 namespace ftb {
+
+// f(begin, end) over [0, n) in contiguous pieces on up to eight threads, for the loops over
+// all primitives, records or nodes of a bake; small n, and pieces whose thread cannot be made,
+// run on the calling thread.  f must not throw.
+template <class F>
+void parallel_for(size_t n, const F& f) {
+    constexpr size_t kPiece = 8192;   // ~0.2 ms of such a loop: a thread costs ~0.03 ms
+    const size_t parts = std::min<size_t>({n / kPiece, (size_t)std::max(1u, std::thread::hardware_concurrency()), 8});
+    if (parts <= 1) { f((size_t)0, n); return; }
+    std::thread th[8];
+    size_t begin = n / parts;   // the first piece is the caller's
+    const size_t mine = begin;
+    for (size_t k = 1; k < parts; ++k) {
+        const size_t end = k + 1 == parts ? n : n / parts * (k + 1);
+        try {
+            th[k] = std::thread([&f, begin, end] { f(begin, end); });
+        } catch (...) {
+            f(begin, end);
+        }
+        begin = end;
+    }
+    f((size_t)0, mine);
+    for (auto& t : th) if (t.joinable()) t.join();
+}
 
 struct Box {
     double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX};

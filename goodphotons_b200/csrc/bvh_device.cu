@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "bvh_build.h"
@@ -264,15 +265,21 @@ __global__ void k_collapse_level(const DBin* __restrict__ bins, const int* __res
         }
 }
 
-struct DevBuf {
-    std::vector<void*> ptrs;
-    ~DevBuf() { for (void* p : ptrs) cudaFree(p); }
+// One device allocation handed out in pieces: a build's two dozen arrays cost one cudaMalloc
+// and one cudaFree.
+struct Arena {
+    char* base = nullptr;
+    size_t size = 0, used = 0;
+    ~Arena() { if (base) cudaFree(base); }
+    static size_t rounded(size_t bytes) { return (bytes + 16 + 255) & ~(size_t)255; }
     template <class T>
-    cudaError_t get(T** out, size_t n) {
-        void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, n * sizeof(T) + 16);
-        if (e == cudaSuccess) { ptrs.push_back(p); *out = (T*)p; }
-        return e;
+    void want(size_t n) { size += rounded(n * sizeof(T)); }
+    cudaError_t make() { return cudaMalloc((void**)&base, size); }
+    template <class T>
+    T* get(size_t n) {
+        T* p = (T*)(base + used);
+        used += rounded(n * sizeof(T));
+        return p;
     }
 };
 
@@ -297,39 +304,63 @@ bool build_wide_lbvh_device(const std::vector<Box>& boxes, int leaf_size, int de
     };
     // centre bounds on the host (one pass over the boxes)
     double clo[3] = {1e300, 1e300, 1e300}, chi[3] = {-1e300, -1e300, -1e300};
-    std::vector<DBox> hb((size_t)n);
-    for (int i = 0; i < n; ++i) {
+    std::mutex mu;
+    parallel_for((size_t)n, [&](size_t i0, size_t i1) {
+        double l[3] = {1e300, 1e300, 1e300}, h[3] = {-1e300, -1e300, -1e300};
+        for (size_t i = i0; i < i1; ++i)
+            for (int a = 0; a < 3; ++a) {
+                double c = 0.5 * (boxes[i].lo[a] + boxes[i].hi[a]);
+                l[a] = c < l[a] ? c : l[a];
+                h[a] = c > h[a] ? c : h[a];
+            }
+        std::lock_guard<std::mutex> lk(mu);
         for (int a = 0; a < 3; ++a) {
-            hb[i].lo[a] = boxes[i].lo[a];
-            hb[i].hi[a] = boxes[i].hi[a];
-            double c = 0.5 * (boxes[i].lo[a] + boxes[i].hi[a]);
-            clo[a] = c < clo[a] ? c : clo[a];
-            chi[a] = c > chi[a] ? c : chi[a];
+            clo[a] = l[a] < clo[a] ? l[a] : clo[a];
+            chi[a] = h[a] > chi[a] ? h[a] : chi[a];
         }
-    }
+    });
     double inv[3];
     for (int a = 0; a < 3; ++a) inv[a] = chi[a] > clo[a] ? 1.0 / (chi[a] - clo[a]) : 0.0;
     {
-        DevBuf buf;
-        DBox *d_boxes, *d_nb;
-        uint64_t *d_k, *d_ks;
-        int *d_id, *d_ids, *d_left, *d_right, *d_parent, *d_first, *d_count, *d_visit, *d_src, *d_order, *d_ctr;
-        DBin* d_bins;
-        WNode* d_nodes;
-        float* d_planes = nullptr;
         const size_t nn = (size_t)n;
-        if ((e = buf.get(&d_boxes, nn)) || (e = buf.get(&d_nb, 2 * nn)) || (e = buf.get(&d_k, nn)) ||
-            (e = buf.get(&d_ks, nn)) || (e = buf.get(&d_id, nn)) || (e = buf.get(&d_ids, nn)) ||
-            (e = buf.get(&d_left, nn)) || (e = buf.get(&d_right, nn)) || (e = buf.get(&d_parent, 2 * nn)) ||
-            (e = buf.get(&d_first, nn)) || (e = buf.get(&d_count, nn)) || (e = buf.get(&d_visit, nn)) ||
-            (e = buf.get(&d_bins, 2 * nn)) || (e = buf.get(&d_src, nn + 1)) || (e = buf.get(&d_order, nn)) ||
-            (e = buf.get(&d_nodes, nn + 1)) || (e = buf.get(&d_ctr, 4)))
-            return fail("allocation");
-        if ((e = cudaMemcpy(d_boxes, hb.data(), sizeof(DBox) * nn, cudaMemcpyHostToDevice))) return fail("upload");
+        size_t tmp_bytes = 0;
+        if (n > 1 && (e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint64_t*)nullptr, (uint64_t*)nullptr,
+                                                          (int*)nullptr, (int*)nullptr, n, 0, 63)))
+            return fail("sort sizing");
+        Arena mem;
+        mem.want<DBox>(nn); mem.want<DBox>(2 * nn); mem.want<uint64_t>(nn); mem.want<uint64_t>(nn);
+        for (int k = 0; k < 2; ++k) mem.want<int>(nn);          // ids, sorted ids
+        for (int k = 0; k < 2; ++k) mem.want<int>(nn);          // left, right
+        mem.want<int>(2 * nn);                                  // parent
+        for (int k = 0; k < 3; ++k) mem.want<int>(nn);          // first, count, visits
+        mem.want<DBin>(2 * nn); mem.want<int>(nn + 1); mem.want<int>(nn); mem.want<WNode>(nn + 1); mem.want<int>(4);
+        mem.want<char>(tmp_bytes);
+        if ((e = mem.make())) return fail("allocation");
+        DBox* d_boxes = mem.get<DBox>(nn);
+        DBox* d_nb = mem.get<DBox>(2 * nn);
+        uint64_t* d_k = mem.get<uint64_t>(nn);
+        uint64_t* d_ks = mem.get<uint64_t>(nn);
+        int* d_id = mem.get<int>(nn);
+        int* d_ids = mem.get<int>(nn);
+        int* d_left = mem.get<int>(nn);
+        int* d_right = mem.get<int>(nn);
+        int* d_parent = mem.get<int>(2 * nn);
+        int* d_first = mem.get<int>(nn);
+        int* d_count = mem.get<int>(nn);
+        int* d_visit = mem.get<int>(nn);
+        DBin* d_bins = mem.get<DBin>(2 * nn);
+        int* d_src = mem.get<int>(nn + 1);
+        int* d_order = mem.get<int>(nn);
+        WNode* d_nodes = mem.get<WNode>(nn + 1);
+        int* d_ctr = mem.get<int>(4);
+        char* d_tmp = mem.get<char>(tmp_bytes);
+        float* d_planes = nullptr;
+        static_assert(sizeof(DBox) == sizeof(Box), "boxes are uploaded as they are");
+        if ((e = cudaMemcpy(d_boxes, boxes.data(), sizeof(DBox) * nn, cudaMemcpyHostToDevice))) return fail("upload");
         const int T = 256, G = (n + T - 1) / T, G2 = (2 * n - 1 + T - 1) / T;
         if (n == 1) {   // one leaf: the root of the collapse is leaf 0
             DBin leaf;
-            for (int a = 0; a < 3; ++a) { leaf.lo[a] = hb[0].lo[a]; leaf.hi[a] = hb[0].hi[a]; }
+            for (int a = 0; a < 3; ++a) { leaf.lo[a] = boxes[0].lo[a]; leaf.hi[a] = boxes[0].hi[a]; }
             leaf.left = leaf.right = -1; leaf.first = 0; leaf.count = 1;
             const int zero = 0;
             if ((e = cudaMemcpy(d_bins, &leaf, sizeof leaf, cudaMemcpyHostToDevice)) ||
@@ -339,11 +370,6 @@ bool build_wide_lbvh_device(const std::vector<Box>& boxes, int leaf_size, int de
             k_morton<<<G, T>>>(d_boxes, n, make_double3(clo[0], clo[1], clo[2]), make_double3(inv[0], inv[1], inv[2]),
                                d_k, d_id);
             if ((e = cudaGetLastError())) return fail("morton codes");
-            size_t tmp_bytes = 0;
-            if ((e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_k, d_ks, d_id, d_ids, n, 0, 63)))
-                return fail("sort sizing");
-            char* d_tmp = nullptr;
-            if ((e = buf.get(&d_tmp, tmp_bytes))) return fail("sort scratch");
             if ((e = cub::DeviceRadixSort::SortPairs(d_tmp, tmp_bytes, d_k, d_ks, d_id, d_ids, n, 0, 63)))
                 return fail("sort");
             if ((e = cudaMemset(d_parent, 0xff, sizeof(int) * 2 * nn))) return fail("memset");

@@ -1213,8 +1213,8 @@ ftb_status ftb_scene_create(const ftb_scene_desc* d, int32_t device, ftb_scene**
     s->tables->device = device;
     s->eng = engine_for(device);
     {
-        cudaDeviceProp p;
-        if (cudaGetDeviceProperties(&p, device) == cudaSuccess) s->sms = p.multiProcessorCount;
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) s->sms = sms;
     }
     // BLAS assets: shared handles or baked here
     for (int b = 0; b < d->n_blas; ++b) {
@@ -1236,28 +1236,42 @@ ftb_status ftb_scene_create(const ftb_scene_desc* d, int32_t device, ftb_scene**
     std::vector<ftb::Box> boxes((size_t)np);
     double maxabs = 1.0;
     auto see = [&](double v) { double a = std::fabs(v); if (a > maxabs) maxabs = a; };
-    for (int64_t i = 0; i < nt; ++i) {
-        const double* v = d->tri_v + 9 * i;
-        ftb::Box b;
-        for (int k = 0; k < 3; ++k) { b.grow_point(v + 3 * k); see(v[3 * k]); see(v[3 * k + 1]); see(v[3 * k + 2]); }
-        boxes[(size_t)i] = b;
-    }
+    std::mutex see_mu;
+    ftb::parallel_for((size_t)nt, [&](size_t i0, size_t i1) {
+        double m = 1.0;
+        for (size_t i = i0; i < i1; ++i) {
+            const double* v = d->tri_v + 9 * i;
+            ftb::Box b;
+            for (int k = 0; k < 3; ++k) b.grow_point(v + 3 * k);
+            for (int k = 0; k < 9; ++k) { const double a = std::fabs(v[k]); if (a > m) m = a; }
+            boxes[i] = b;
+        }
+        std::lock_guard<std::mutex> lk(see_mu);
+        see(m);
+    });
     for (int64_t i = 0; i < ns; ++i) {
         const double* sp = d->sph + 4 * i;
         ftb::Box b;
         for (int a = 0; a < 3; ++a) { b.lo[a] = sp[a] - sp[3]; b.hi[a] = sp[a] + sp[3]; see(b.lo[a]); see(b.hi[a]); }
         boxes[(size_t)(nt + i)] = b;
     }
-    for (int64_t i = 0; i < nc; ++i) {
-        const double* c = d->curve + 10 * i;
-        ftb::Box b;   // curveSegBounds (curve.h:99-104)
-        for (int a = 0; a < 3; ++a) {
-            b.lo[a] = std::min(c[a] - c[6], c[3 + a] - c[7]);
-            b.hi[a] = std::max(c[a] + c[6], c[3 + a] + c[7]);
-            see(b.lo[a]); see(b.hi[a]);
+    ftb::parallel_for((size_t)nc, [&](size_t i0, size_t i1) {
+        double m = 1.0;
+        for (size_t i = i0; i < i1; ++i) {
+            const double* c = d->curve + 10 * i;
+            ftb::Box b;   // curveSegBounds (curve.h:99-104)
+            for (int a = 0; a < 3; ++a) {
+                b.lo[a] = std::min(c[a] - c[6], c[3 + a] - c[7]);
+                b.hi[a] = std::max(c[a] + c[6], c[3 + a] + c[7]);
+                const double l = std::fabs(b.lo[a]), h = std::fabs(b.hi[a]);
+                if (l > m) m = l;
+                if (h > m) m = h;
+            }
+            boxes[(size_t)(nt + ns) + i] = b;
         }
-        boxes[(size_t)(nt + ns + i)] = b;
-    }
+        std::lock_guard<std::mutex> lk(see_mu);
+        see(m);
+    });
     for (int i = 0; i < d->n_emitters; ++i) {
         const ftb_emitter& e = d->emitters[i];
         for (int a = 0; a < 3; ++a) { see(e.origin[a] + std::fabs(e.u[a]) + std::fabs(e.v[a]) + e.radius); }
@@ -1371,38 +1385,40 @@ ftb_status ftb_scene_create(const ftb_scene_desc* d, int32_t device, ftb_scene**
     }
     // records in leaf order
     std::vector<PrimRec> recs(bvh.order.size());
-    bool any_smooth = false;
-    for (size_t r = 0; r < bvh.order.size(); ++r) {
-        int p = bvh.order[r];
-        PrimRec& R = recs[r];
-        std::memset(&R, 0, sizeof R);
-        int ty, mat, smooth = 0;
-        if (p < nt) {
-            rec_triangle(R, d->tri_v + 9 * (size_t)p);
-            ty = REC_TRI; mat = d->tri_mat[p];
-            if (d->tri_n) {
-                const double* n = d->tri_n + 9 * (size_t)p;
-                for (int k = 0; k < 9; ++k) if (n[k] != 0.0) smooth = 1;
+    std::atomic<bool> any_smooth{false};
+    ftb::parallel_for(bvh.order.size(), [&](size_t r0, size_t r1) {
+        for (size_t r = r0; r < r1; ++r) {
+            int p = bvh.order[r];
+            PrimRec& R = recs[r];
+            std::memset(&R, 0, sizeof R);
+            int ty, mat, smooth = 0;
+            if (p < nt) {
+                rec_triangle(R, d->tri_v + 9 * (size_t)p);
+                ty = REC_TRI; mat = d->tri_mat[p];
+                if (d->tri_n) {
+                    const double* n = d->tri_n + 9 * (size_t)p;
+                    for (int k = 0; k < 9; ++k) if (n[k] != 0.0) smooth = 1;
+                }
+            } else if (p < nt + ns) {
+                const double* sp = d->sph + 4 * (size_t)(p - nt);
+                std::memcpy(R.row[0], sp, 3 * sizeof(double));
+                R.row[1][0] = sp[3];
+                ty = REC_SPHERE; mat = d->sph_mat[p - nt];
+            } else if (p < nt + ns + nc) {
+                const double* c = d->curve + 10 * (size_t)(p - nt - ns);
+                std::memcpy(R.row[0], c, 3 * sizeof(double));
+                std::memcpy(R.row[1], c + 3, 3 * sizeof(double));
+                std::memcpy(R.row[2], c + 6, 2 * sizeof(double));
+                ty = REC_CURVE; mat = d->curve_mat[p - nt - ns];
+            } else {
+                int64_t k = p - nt - ns - nc;
+                std::memcpy(&R.row[0][0], &k, sizeof k);
+                ty = REC_INST; mat = 0;
             }
-        } else if (p < nt + ns) {
-            const double* sp = d->sph + 4 * (size_t)(p - nt);
-            std::memcpy(R.row[0], sp, 3 * sizeof(double));
-            R.row[1][0] = sp[3];
-            ty = REC_SPHERE; mat = d->sph_mat[p - nt];
-        } else if (p < nt + ns + nc) {
-            const double* c = d->curve + 10 * (size_t)(p - nt - ns);
-            std::memcpy(R.row[0], c, 3 * sizeof(double));
-            std::memcpy(R.row[1], c + 3, 3 * sizeof(double));
-            std::memcpy(R.row[2], c + 6, 2 * sizeof(double));
-            ty = REC_CURVE; mat = d->curve_mat[p - nt - ns];
-        } else {
-            int64_t k = p - nt - ns - nc;
-            std::memcpy(&R.row[0][0], &k, sizeof k);
-            ty = REC_INST; mat = 0;
+            if (smooth) any_smooth = true;
+            rec_tail(R, p, mat | (ty << 24) | (smooth << 30));
         }
-        any_smooth |= smooth != 0;
-        rec_tail(R, p, mat | (ty << 24) | (smooth << 30));
-    }
+    });
     std::vector<DevSpec> spec((size_t)d->n_spectra);
     for (int i = 0; i < d->n_spectra; ++i) {
         spec[i].kind = d->spectra[i].kind; spec[i].n = d->spectra[i].n; spec[i].offset = d->spectra[i].offset;
