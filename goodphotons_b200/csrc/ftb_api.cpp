@@ -253,6 +253,7 @@ struct BlasDev {
     const PrimRec* recs = nullptr;
     const double* tri_n = nullptr;
     int64_t n_tris = 0;
+    int32_t n_nodes = 0;
     int32_t max_mat = -1;
     double lo[3], hi[3];   // localBounds: union of the triangle boxes padded by 1e-6
 };
@@ -638,6 +639,7 @@ ftb_status bake_blas(const ftb_blas_desc& d, int device, ftb::BuildMethod method
         rec_tail(R, p, d.tri_mat[p] | (REC_TRI << 24) | (smooth << 30));
     }
     const std::vector<FNode> fn = ftb::widen_nodes(bvh);
+    b->n_nodes = (int32_t)fn.size();
     ftb_status st = upload(b->mem, fn.data(), fn.size(), &b->nodes, "upload BLAS nodes");
     if (st == FTB_OK) st = upload(b->mem, recs.data(), recs.size(), &b->recs, "upload BLAS records");
     if (st == FTB_OK && any_smooth) st = upload(b->mem, d.tri_n, (size_t)nt * 9, &b->tri_n, "upload BLAS normals");
@@ -1498,7 +1500,8 @@ ftb_status ftb_scene_create(const ftb_scene_desc* d, int32_t device, ftb_scene**
     D.n_mats = d->n_mats;
     D.n_emit = d->n_emitters;
     D.n_med = d->n_media;
-    D.n_spec = d->n_spectra;
+    D.max_nodes = D.n_nodes;
+    for (auto& b : s->blas) D.max_nodes = std::max(D.max_nodes, b->n_nodes);
     D.n_tris = nt;
     D.total_power = tp;
     s->power = tp;

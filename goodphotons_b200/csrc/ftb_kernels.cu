@@ -1656,10 +1656,15 @@ __global__ void __launch_bounds__(128, INST || SHAPES ? FTB_TRAV_MINB : FTB_EXTE
     }
 }
 
-// Optional reordering of a closest-hit queue by ray direction: pieces of kSortChunk entries
-// are bucketed by an 8-bit direction key (an octahedral 16 x 16 grid in Morton order), so
-// the lanes of a warp head the same way.  The order of rays does not change any result.
-constexpr int kSortChunk = 1024;
+// Reordering of a closest-hit queue or of the connections before traversal (large scenes, or
+// when the tuning asks): the order of rays does not change any result.
+
+// 8-bit Morton code of two 4-bit coordinates.
+__device__ __forceinline__ uint32_t morton4(uint32_t u, uint32_t v) {
+    u = (u | (u << 2)) & 0x33u; u = (u | (u << 1)) & 0x55u;
+    v = (v | (v << 2)) & 0x33u; v = (v | (v << 1)) & 0x55u;
+    return u | (v << 1);
+}
 
 __device__ __forceinline__ uint32_t direction_key(D3 d) {
     float x = (float)d.x, y = (float)d.y, z = (float)d.z;
@@ -1672,52 +1677,112 @@ __device__ __forceinline__ uint32_t direction_key(D3 d) {
     }
     uint32_t u = (uint32_t)min(15, max(0, (int)((x * 0.5f + 0.5f) * 16.0f)));
     uint32_t v = (uint32_t)min(15, max(0, (int)((y * 0.5f + 0.5f) * 16.0f)));
-    u = (u | (u << 2)) & 0x33u; u = (u | (u << 1)) & 0x55u;   // 4-bit Morton interleave
-    v = (v | (v << 2)) & 0x33u; v = (v | (v << 1)) & 0x55u;
-    return u | (v << 1);
+    return morton4(u, v);
 }
 
-// Traversal order of a queue, each kSortChunk-position piece bucketed by direction key (one
-// block per piece, counting sort in shared memory): order[q] is the entry of the path the
-// closest-hit kernel's q-th lane takes, so a warp's 32 lanes head the same way.
-__global__ void __launch_bounds__(128) k_sort_queue(Wave w, PathState in, const int32_t* qcount,
-                                                    int32_t* order) {
-    __shared__ int32_t hist[256];
-    const int front = qcount[0], nq = queue_len(qcount);
-    constexpr int kPer = kSortChunk / 128;
-    for (int base = blockIdx.x * kSortChunk; base < nq; base += gridDim.x * kSortChunk) {
-        for (int t = threadIdx.x; t < 256; t += 128) hist[t] = 0;
+// The order of positions 0 .. n-1 in which each piece of CHUNK of them is bucketed by key in
+// [0, KEYS) (counting sort in shared memory, one piece per block at a time): order[q] =
+// entry_of(p) for the q-th position p of its piece.
+template <int CHUNK, int THREADS, int KEYS, class Key, class Entry>
+__device__ __forceinline__ void bucket_pieces(int n, int32_t* order, const Key& key_of, const Entry& entry_of) {
+    constexpr int kPer = CHUNK / THREADS, kSlice = KEYS / THREADS, kWarps = THREADS / 32;
+    static_assert(CHUNK % THREADS == 0 && KEYS % THREADS == 0 && kWarps <= 32, "whole rows");
+    __shared__ int32_t hist[KEYS];
+    __shared__ int32_t warp_sum[kWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int base = blockIdx.x * CHUNK; base < n; base += gridDim.x * CHUNK) {
+        for (int t = threadIdx.x; t < KEYS; t += THREADS) hist[t] = 0;
         __syncthreads();
-        int pos[kPer], key[kPer], off[kPer];
+        int key[kPer], off[kPer];
 #pragma unroll
         for (int r = 0; r < kPer; ++r) {
-            const int p = base + r * 128 + threadIdx.x;
-            const int i = p < nq ? queue_entry(w, front, p) : 0;
-            pos[r] = p < nq ? i : -1;
-            key[r] = pos[r] >= 0 ? (int)direction_key(mk(in.dx[i], in.dy[i], in.dz[i])) : 255;
-            off[r] = pos[r] >= 0 ? atomicAdd(&hist[key[r]], 1) : 0;
+            const int p = base + r * THREADS + threadIdx.x;
+            key[r] = p < n ? key_of(p) : -1;
+            off[r] = p < n ? atomicAdd(&hist[key[r]], 1) : 0;
         }
         __syncthreads();
-        if (threadIdx.x < 32) {   // exclusive scan of the 256 bucket counts by one warp
-            int v[8], run = 0;
+        // exclusive scan of the bucket counts: a slice per thread, then over threads and warps
+        int slice[kSlice], run = 0;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) { v[k] = hist[threadIdx.x * 8 + k]; run += v[k]; }
-            int incl = run;
+        for (int k = 0; k < kSlice; ++k) { slice[k] = hist[threadIdx.x * kSlice + k]; run += slice[k]; }
+        int incl = run;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)threadIdx.x >= o) incl += y;
-            }
-            int acc = incl - run;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) { hist[threadIdx.x * 8 + k] = acc; acc += v[k]; }
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
         }
+        if (lane == 31) warp_sum[wid] = incl;
+        __syncthreads();
+        int acc = incl - run;
+        for (int k = 0; k < wid; ++k) acc += warp_sum[k];
+#pragma unroll
+        for (int k = 0; k < kSlice; ++k) { hist[threadIdx.x * kSlice + k] = acc; acc += slice[k]; }
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kPer; ++r)
-            if (pos[r] >= 0) order[base + hist[key[r]] + off[r]] = pos[r];
+            if (key[r] >= 0) order[base + hist[key[r]] + off[r]] = entry_of(base + r * THREADS + threadIdx.x);
         __syncthreads();   // before the next piece reuses the histogram
     }
+}
+
+// Traversal order of a queue: order[q] is the entry of the path the closest-hit kernel's q-th
+// lane takes.  Pieces of 8192 paths are bucketed by the cell of the ray's origin on a 4 x 4 x 4
+// grid over the scene's root box, then by its direction on an 8 x 8 octahedral grid, so a
+// warp's 32 lanes start near each other and head the same way.  Closest hit of a frame (B200),
+// against pieces of 1024 by direction alone (16 x 16): glass 117.0 -> 112.5 ms, fog + strands
+// 55.7 -> 51.9, animation batch 34.9 -> 33.2; a sort of the whole queue by 9 bits of cell and
+// 8 of direction gains as much again in traversal and costs more than that.
+constexpr int kRayChunk = 8192, kRayThreads = 512, kRayKeys = 4096;
+__global__ void __launch_bounds__(kRayThreads) k_sort_queue(Wave w, const DevJob* __restrict__ jobs, PathState in,
+                                                            const int32_t* qcount, int32_t* order) {
+    __shared__ float grid[kWaveJobs][6];   // per job: the root box's low corner, cells per unit
+    const int32_t n_jobs = w.params[0];
+    for (int t = threadIdx.x; t < 3 * n_jobs; t += kRayThreads) {
+        const int j = t / 3, a = t % 3;
+        const FNode& root = jobs[j].sc.nodes[0];
+        float lo = root.lo[a][0], hi = root.hi[a][0];
+        for (int k = 1; k < FTB_WIDTH; ++k) { lo = fminf(lo, root.lo[a][k]); hi = fmaxf(hi, root.hi[a][k]); }
+        const float ext = hi - lo;   // not positive in an empty scene
+        grid[j][a] = lo;
+        grid[j][3 + a] = ext > 0.0f && ext < FLT_MAX ? 4.0f / ext : 0.0f;
+    }
+    __syncthreads();
+    const int front = qcount[0];
+    bucket_pieces<kRayChunk, kRayThreads, kRayKeys>(
+        queue_len(qcount), order,
+        [&](int p) {
+            const int i = queue_entry(w, front, p);
+            const float* g = grid[n_jobs > 1 ? in.job[i] : 0];
+            const int cx = min(3, max(0, (int)(((float)in.ox[i] - g[0]) * g[3])));
+            const int cy = min(3, max(0, (int)(((float)in.oy[i] - g[1]) * g[4])));
+            const int cz = min(3, max(0, (int)(((float)in.oz[i] - g[2]) * g[5])));
+            const uint32_t d = direction_key(mk(in.dx[i], in.dy[i], in.dz[i]));
+            return ((cx | (cy << 2) | (cz << 4)) << 6) | (int)(d >> 2);
+        },
+        [&](int p) { return queue_entry(w, front, p); });
+}
+
+// Traversal order of the queued connections: all of a view's rays end at its eye, so those of
+// one tile of the image (a 16 x 16 grid in Morton order) cross the same nodes.  In large scenes
+// only, as for the closest-hit rays.  Whole frames (B200): fog + strands 110.7 -> 103.7 ms
+// (the connections alone 29.1 -> 24.0), glass 205.6 -> 202.7, animation batch 68.5 -> 66.1,
+// served jobs 83.0 -> 79.1; Cornell, where it does not run, would take 0.4 ms more.  Pieces of
+// 4096 gain 1 ms more on the strands and lose 1.2 on glass.
+constexpr int kConnChunk = 1024, kConnThreads = 128, kConnKeys = 256;
+__global__ void __launch_bounds__(kConnThreads) k_sort_connections(Wave w, const DevJob* __restrict__ jobs,
+                                                                   int32_t* order) {
+    const int32_t n_jobs = w.params[0];
+    int n = w.counts[kShadowCount];
+    if (n > w.S) n = w.S;
+    bucket_pieces<kConnChunk, kConnThreads, kConnKeys>(
+        n, order,
+        [&](int p) {
+            const DevCam& c = view_cam(jobs[n_jobs > 1 ? w.sjob[p] : 0], w.sview[p]);
+            const int pix = w.spix[p];
+            const int py = pix / c.rx, px = pix - py * c.rx;
+            return (int)morton4((uint32_t)((int64_t)px * 16 / c.rx), (uint32_t)((int64_t)py * 16 / c.ry));
+        },
+        [&](int p) { return p; });
 }
 
 struct Stk { int n; int2 e[kStkCap]; };
@@ -2132,13 +2197,14 @@ __device__ __noinline__ void mirror_now(const DevJob& J, const Frame& f, int vie
 // MIRROR: the queue may also hold mirror connections (scenes with planar mirrors).
 template <bool COUNT, bool INST, bool SHAPES, bool MIRROR>
 __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow(Wave w, const DevJob* __restrict__ jobs,
-                                                              Frame f) {
+                                                              Frame f, const int32_t* __restrict__ order) {
     const int32_t n_jobs = w.params[0];
     int n = w.counts[kShadowCount];
     if (n > w.S) n = w.S;
     TravCount cnt{0, 0, 0};
     unsigned long long rays = 0;
-    FTB_FOR_WARP_CHUNKS(i, n, &w.counts[kFetchShadow]) {
+    FTB_FOR_WARP_CHUNKS(q, n, &w.counts[kFetchShadow]) {
+        const int i = order ? order[q] : q;
         const DevJob& J = jobs[n_jobs > 1 ? w.sjob[i] : 0];
         const DevScene& sc = J.sc;
         if (COUNT) rays++;
@@ -2913,14 +2979,14 @@ struct LaunchExtend {
 };
 template <bool C, bool I, bool S>
 struct LaunchShadow {
-    static void go(int grid, cudaStream_t st, Wave w, const DevJob* jobs, Frame f) {
-        k_shadow<C, I, S, false><<<grid, 128, 0, st>>>(w, jobs, f);
+    static void go(int grid, cudaStream_t st, Wave w, const DevJob* jobs, Frame f, const int32_t* order) {
+        k_shadow<C, I, S, false><<<grid, 128, 0, st>>>(w, jobs, f, order);
     }
 };
 template <bool C, bool I, bool S>
 struct LaunchShadowMirror {
     static void go(int grid, cudaStream_t st, Wave w, const DevJob* jobs, Frame f) {
-        k_shadow<C, I, S, true><<<grid, 128, 0, st>>>(w, jobs, f);
+        k_shadow<C, I, S, true><<<grid, 128, 0, st>>>(w, jobs, f, nullptr);
     }
 };
 template <bool C, bool I, bool S>
@@ -2950,6 +3016,9 @@ struct Issue {
     static constexpr int T = 128;
 
     // paths left to the whole-path kernels, which have no counting variant
+    int sort_grid(int entries, int chunk, int per_sm) const {
+        return std::max(1, std::min(sms * per_sm, (entries + chunk - 1) / chunk));
+    }
     size_t tally() const { return kind.multi ? kTallyBytes : 0; }   // dynamic shared memory of the tally kernels
     int32_t tail() const { return f.stats ? 0 : trace_limit(sms); }
 
@@ -2992,7 +3061,17 @@ struct Issue {
         if (kind.bundles && kind.mirrors) trav<LaunchShadowHeroMirror>(w, (const DevJob*)w.jobs, f);
         else if (kind.bundles) trav<LaunchShadowHero>(w, (const DevJob*)w.jobs, f);
         else if (kind.mirrors) trav<LaunchShadowMirror>(w, (const DevJob*)w.jobs, f);
-        else trav<LaunchShadow>(w, (const DevJob*)w.jobs, f);
+        else {
+            const int32_t* order = nullptr;
+            if (kind.deep) {
+                // 4-byte positions in an array of 8-byte values that only bundles and mirror
+                // connections use
+                int32_t* o = reinterpret_cast<int32_t*>(w.slam);
+                k_sort_connections<<<sort_grid(w.S, kConnChunk, 16), kConnThreads, 0, st>>>(w, w.jobs, o);
+                order = o;
+            }
+            trav<LaunchShadow>(w, (const DevJob*)w.jobs, f, order);
+        }
         mark(K_SHADOW, true);
     }
     void trace(const PathState& in, const int32_t* c) {   // whole paths (booked with closest hit)
@@ -3022,8 +3101,7 @@ struct Issue {
         mark(K_EXTEND, false);
         const int32_t* order = nullptr;
         if (sorted) {
-            const int gs = std::max(1, std::min(grid, (w.W + kSortChunk - 1) / kSortChunk));
-            k_sort_queue<<<gs, T, 0, st>>>(w, in, c, w.perm);
+            k_sort_queue<<<sort_grid(w.W, kRayChunk, 4), kRayThreads, 0, st>>>(w, w.jobs, in, c, w.perm);
             order = w.perm;
         }
         trav<LaunchExtend>(w, (const DevJob*)w.jobs, in, (const int32_t*)c, order, f);
@@ -3165,7 +3243,8 @@ void stream_paths(Issue& I) {
 struct WaveGraphs {
     struct Entry {
         int32_t max_bounce, grid;   // max_bounce -1: a streaming pass, -2: one of few photons, -3: a wave of few
-        bool inst, hero, media, shapes, mirrors, multi, sorted;
+        WaveKind kind;
+        bool sorted;
         int32_t* status;
         cudaGraphExec_t exec;
     };
@@ -3176,10 +3255,7 @@ struct WaveGraphs {
     }
     cudaGraphExec_t find(int32_t max_bounce, int32_t grid, const WaveKind& kind, bool sorted, int32_t* status) const {
         for (auto& e : entries)
-            if (e.max_bounce == max_bounce && e.grid == grid && e.inst == kind.instances && e.hero == kind.bundles &&
-                e.media == kind.media && e.shapes == kind.shapes && e.mirrors == kind.mirrors &&
-                e.multi == kind.multi && e.sorted == sorted &&
-                e.status == status)
+            if (e.max_bounce == max_bounce && e.grid == grid && e.kind == kind && e.sorted == sorted && e.status == status)
                 return e.exec;
         return nullptr;
     }
@@ -3225,8 +3301,7 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
     else issue_wave(I, max_bounce);
     err = cudaStreamEndCapture(st, &g);
     if (err != cudaSuccess) return err;
-    WaveGraphs::Entry e{max_bounce, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors, kind.multi,
-                        sorted, f.status, nullptr};
+    WaveGraphs::Entry e{max_bounce, grid, kind, sorted, f.status, nullptr};
     err = cudaGraphInstantiate(&e.exec, g, 0);
     cudaGraphDestroy(g);
     if (err != cudaSuccess) return err;
@@ -3269,8 +3344,7 @@ cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKin
     // swap roles between them; the last advance of the body sets the loop condition), then the
     // paths still queued and the connections
     Issue I{w, kind, f, grid, sorted, st, nullptr, sms};
-    WaveGraphs::Entry entry{key, grid, kind.instances, kind.bundles, kind.media, kind.shapes, kind.mirrors, kind.multi,
-                            sorted, f.status, nullptr};
+    WaveGraphs::Entry entry{key, grid, kind, sorted, f.status, nullptr};
     cudaGraph_t g = nullptr;
     cudaError_t err = graphs->side.init();
     if (err != cudaSuccess) return err;

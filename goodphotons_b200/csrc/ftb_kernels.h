@@ -88,7 +88,7 @@ struct Wave {
     double* hit_t;             // closest hit of path i (indexed like the queue being traced)
     int32_t* hit_rec;          // world record of the closest hit, or -1
     int32_t* hit_sub;          // BLAS record when hit_rec is an instance
-    int32_t* perm;             // optional traversal order of a queue (bucketed by direction)
+    int32_t* perm;             // optional traversal order of a queue (k_sort_queue)
     int32_t* counts;           // [2a], [2a+1]: the two ends of the queue in ps[a]; [4] shadow records;
                                // [5..7] per-launch work counters (kFetch*)
     int32_t* sjob;             // job of each shadow record
@@ -169,12 +169,12 @@ struct LaunchSink {
 };
 
 // Launch shape chosen by the autotuner: blocks per SM of the queue-driven kernels, whether a
-// wave is replayed from a captured CUDA graph, and whether closest-hit rays are reordered by
-// direction within each block.
+// wave is replayed from a captured CUDA graph, and whether closest-hit rays are always
+// reordered by origin and direction.
 struct LaunchShape {
     int32_t grid_mult = 16;
     bool graph = true;
-    bool sort_rays = false;   // reorder each block's closest-hit rays by direction first
+    bool sort_rays = false;   // order closest-hit rays in every scene (large ones always do)
     bool regenerate = true;   // streaming passes: freed slots are refilled with new photons
 };
 
@@ -193,18 +193,24 @@ struct WaveKind {
     bool mirrors = false;     // some scene has planar mirrors (mirror connections queued)
     bool deep = false;        // some scene's hierarchy is large (scene_is_deep)
     bool multi = false;       // the table holds more than one job (it must say so exactly)
+    bool operator==(const WaveKind& o) const {
+        return instances == o.instances && bundles == o.bundles && media == o.media && shapes == o.shapes &&
+               mirrors == o.mirrors && deep == o.deep && multi == o.multi;
+    }
 };
 // Connection records one path vertex of job J can queue: a camera connection and one per
 // planar mirror, for each of the job's views.  A wave or pass keeps its slots at most
 // W / fanout so that the shadow queue (kShadowPerSlot records per slot) cannot overflow.
 inline int conn_fanout(const DevJob& J) { return (J.n_views > 1 ? J.n_views : 1) * (1 + J.sc.n_planes); }
-// Whether ordering a scene's closest-hit rays by direction pays for itself (launches do it
-// then, whatever the tuning says): the hierarchy has to be large enough that rays of one
-// direction share nodes that others do not.  Whole frames with / without it (B200): glass of
-// 327,680 triangles (37 k nodes) 220.8 / 225.4 ms, fog + 250 k strands 113.2 / 116.1;
-// showroom (2 k nodes) 27.75 / 27.75, Cornell (9 nodes) 11.9 / 11.4.
+// Whether ordering a scene's closest-hit rays (by origin and direction) and its connections
+// (by image tile) before traversal pays for itself; launches do it then, whatever the tuning
+// says: the hierarchy has to be large enough that rays near each other share nodes that others
+// do not.  Whole frames with / without the order of the rays, by direction alone (B200): glass
+// of 327,680 triangles (37 k nodes) 220.8 / 225.4 ms, fog + 250 k strands 113.2 / 116.1, glass
+// of 81,920 triangles (9 k nodes) 25.8 / 25.8, showroom (2 k nodes) 27.75 / 27.75, Cornell (9
+// nodes) 11.9 / 11.4.
 constexpr int32_t kSortNodes = 8192;
-inline bool scene_is_deep(const DevScene& sc) { return sc.n_nodes >= kSortNodes; }
+inline bool scene_is_deep(const DevScene& sc) { return sc.max_nodes >= kSortNodes; }
 // Whether a scene's world records include spheres or curves.
 inline bool scene_has_shapes(const DevScene& sc) { return (int64_t)sc.n_recs > sc.n_tris + sc.n_inst; }
 
