@@ -847,7 +847,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.shapes = shapes;
         kind.mirrors = mirrors;
         kind.deep = deep;
-        kind.multi = table.size() > 1;
+        kind.multi = ftb::table_class(table.size());
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                s->eng->graphs[k & 1]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
@@ -901,7 +901,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.shapes = shapes;
         kind.mirrors = mirrors;
         kind.deep = deep;
-        kind.multi = table.size() > 1;
+        kind.multi = ftb::table_class(table.size());
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                              s->eng->graphs[k & 1]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");

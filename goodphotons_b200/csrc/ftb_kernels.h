@@ -192,12 +192,16 @@ struct WaveKind {
     bool shapes = false;      // some scene has spheres or curves (not only triangles)
     bool mirrors = false;     // some scene has planar mirrors (mirror connections queued)
     bool deep = false;        // some scene's hierarchy is large (scene_is_deep)
-    bool multi = false;       // the table holds more than one job (it must say so exactly)
+    int32_t multi = 0;        // table_class() of the table's jobs (it must be exactly that)
     bool operator==(const WaveKind& o) const {
         return instances == o.instances && bundles == o.bundles && media == o.media && shapes == o.shapes &&
                mirrors == o.mirrors && deep == o.deep && multi == o.multi;
     }
 };
+// Tables by size: 0 one job, 1 at most kSmallTable, 2 more.  The tally kernels hold a row per
+// job in shared memory, and what they hold is taken from L1.
+constexpr int32_t kSmallTable = 32;
+inline int32_t table_class(size_t jobs) { return jobs <= 1 ? 0 : (jobs <= (size_t)kSmallTable ? 1 : 2); }
 // Connection records one path vertex of job J can queue: a camera connection and one per
 // planar mirror, for each of the job's views.  A wave or pass keeps its slots at most
 // W / fanout so that the shadow queue (kShadowPerSlot records per slot) cannot overflow.

@@ -398,7 +398,7 @@ void scheduler(ftb_server* s) {
         }
         retire(s, b);   // the buffer's previous wave
         WaveSlot& w = s->ws[b];
-        kind.multi = table.size() > 1;
+        kind.multi = ftb::table_class(table.size());
         std::memcpy(w.table, table.data(), sizeof(ftb::DevJob) * table.size());
         // streaming pass: {ranges, paths in flight, photons (int64), half-iteration cap (int64)};
         // wave: {jobs, slots}
