@@ -60,6 +60,7 @@ def test_passes_equal_whole_paths(gpu, tuning, slots, heroes):
 @pytest.mark.parametrize("name,build", [
     ("glass", lambda L: scenes.make_glass(L, freq=90)),                # ~18 k nodes: rays ordered by direction
     ("fog_strands", lambda L: scenes.make_fog_strands(L, n_strands=40_000)),
+    ("instanced", lambda L: scenes.make_glass_instanced(L, level=6)),   # the large hierarchy is the BLAS's
 ])
 def test_ordered_queues_of_large_scenes(gpu, tuning, name, build):
     torch = pytest.importorskip("torch")
@@ -75,3 +76,27 @@ def test_ordered_queues_of_large_scenes(gpu, tuning, name, build):
         np.testing.assert_array_equal(film.cpu().numpy(), ref)
         np.testing.assert_array_equal(np.array(list(en.fx), dtype=np.int64), fx)
     sc.close()
+
+
+@pytest.mark.parametrize("n_jobs", [3, 40])   # job tables of up to 32 rows, and of more
+def test_ordered_queues_of_mixed_scenes(gpu, tuning, n_jobs):
+    """Each path is put on the grid of its own job's scene, and tallied to its own job."""
+    torch = pytest.importorskip("torch")
+    scs = [lib.Scene(scenes.make_cornell(gpu), 0, gpu), lib.Scene(scenes.make_glass(gpu, freq=90), 0, gpu),
+           lib.Scene(scenes.make_fog_strands(gpu, n_strands=40_000), 0, gpu)]
+    cam = scenes.default_camera(gpu, 20)
+    jobs, films = [], []
+    for k in range(n_jobs):
+        film = torch.zeros((20, 20, 4), dtype=torch.int64, device="cuda:0")
+        films.append(film)
+        jobs.append(dict(scene=scs[k % 3], cam=cam, d_film=film.data_ptr(), n=120_000 // n_jobs + k,
+                         seed_base=10_000 * k, max_bounce=6 + k % 5, frac_bits=24))
+    tuning(wave_slots=20_000)
+    _, ens = gpu.render_batch(jobs, stream=torch.cuda.current_stream().cuda_stream)
+    tuning(wave_slots=1 << 22)
+    for job, film, en in zip(jobs, films, ens):
+        ref, fx = _solo(gpu, torch, job["scene"], cam, job["n"], job["seed_base"], job["max_bounce"], 1)
+        np.testing.assert_array_equal(film.cpu().numpy(), ref)
+        np.testing.assert_array_equal(np.array(list(en.fx), dtype=np.int64), fx)
+    for sc in scs:
+        sc.close()
