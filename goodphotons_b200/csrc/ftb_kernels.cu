@@ -1116,13 +1116,23 @@ __device__ __forceinline__ int queue_entry(const Wave& w, int front, int p) {
     return p < front ? p : w.W - 1 - (p - front);
 }
 
+// A place in the connection queue, or -1 when it is full.  A place that was not there is given
+// back, so the count stays at most the queue plus one per lane in flight however many
+// connections a whole-path launch makes, and never falls below the places taken.
+__device__ __forceinline__ int queue_slot(const Wave& w) {
+    const int i = agg_inc(&w.counts[kShadowCount]);
+    if (i < w.S) return i;
+    atomicSub(&w.counts[kShadowCount], 1);
+    return -1;
+}
+
 // A one-wavelength connection: the film increments cieX/Y/Z(lambda) * contribution in the
 // order Film::add forms them (scene_film.h:12), from the matching functions evaluated once
 // per path at emission.  Returns false when the connection queue is full.
 __device__ __forceinline__ bool queue_shadow(const Wave& w, int job, int view, D3 o, D3 d, double tmax, double val,
                                              const double* cie, int pix) {
-    int i = agg_inc(&w.counts[kShadowCount]);
-    if (i >= w.S) return false;
+    const int i = queue_slot(w);
+    if (i < 0) return false;
     w.sox[i] = o.x; w.soy[i] = o.y; w.soz[i] = o.z;
     w.sdx[i] = d.x; w.sdy[i] = d.y; w.sdz[i] = d.z;
     w.smax[i] = tmax; w.spix[i] = pix;
@@ -1218,8 +1228,8 @@ __device__ void connect_volume(const DevScene& sc, const DevJob& J, const Q& w, 
 // mirror's reflectance is known only once k_shadow has seen which mirror the eye meets.
 __device__ __forceinline__ bool queue_mirror(const Wave& w, int job, int view, int plane, D3 p, D3 wP, double dP,
                                              double a, double lam, const double* cie, int pix) {
-    int i = agg_inc(&w.counts[kShadowCount]);
-    if (i >= w.S) return false;
+    const int i = queue_slot(w);
+    if (i < 0) return false;
     w.sox[i] = p.x; w.soy[i] = p.y; w.soz[i] = p.z;
     w.sdx[i] = wP.x; w.sdy[i] = wP.y; w.sdz[i] = wP.z;
     w.smax[i] = dP; w.spix[i] = ~pix;
@@ -2239,8 +2249,8 @@ __global__ void __launch_bounds__(128, FTB_TRAV_MINB) k_shadow(Wave w, const Dev
 // mirror `view >> 16` (pix < 0).  Returns false when the queue is full.
 __device__ __forceinline__ bool queue_hero(const Wave& w, int job, int view, D3 o, D3 d, double tmax, int nup,
                                            const double* lam, const double* val, int pix) {
-    int i = agg_inc(&w.counts[kShadowCount]);
-    if (i >= w.S) return false;
+    const int i = queue_slot(w);
+    if (i < 0) return false;
     w.sox[i] = o.x; w.soy[i] = o.y; w.soz[i] = o.z;
     w.sdx[i] = d.x; w.sdy[i] = d.y; w.sdz[i] = d.z;
     w.smax[i] = tmax; w.spix[i] = pix; w.sjob[i] = job; w.sview[i] = view;
