@@ -18,12 +18,13 @@
 // out work to warps 32 entries at a time from a per-launch counter.  A streaming pass
 // (launch_stream) refills the room freed by finished paths with the next photons every
 // half-iteration and runs as one CUDA graph with a device-driven while loop; a wave
-// (launch_wave) traces W photons to their last bounce.
+// (launch_wave) traces W photons to their last bounce.  Small passes and renders, and the last
+// paths of larger passes, are traced to their ends by one launch (k_trace, k_trace_hero).
 //
 // Variants: k_emit_hero / k_shade_hero / k_shadow_hero trace hero-wavelength bundles (one
 // path carries up to kHeroMax wavelengths), and the kernels are templated on whether the
 // scenes have instances, participating media or spheres/curves, so a launch runs only the
-// code its scenes need.  k_sort_queue optionally orders a closest-hit queue by direction.
+// code its scenes need.  k_sort_queue and k_sort_connections order the rays of large scenes.
 //
 // Numerics.  Everything that decides a path -- triangle/sphere/curve tests, hit points,
 // normals, BSDF sampling, Russian roulette, the camera projection -- is computed in fp64
