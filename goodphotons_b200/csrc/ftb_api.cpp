@@ -33,7 +33,11 @@ ftb_status fail(ftb_status s, const std::string& m) {
     g_err = m;
     return s;
 }
+// The status of a failed CUDA call.  The error is taken off the thread: it is reported by the
+// call that met it, and a render that goes on without the allocation, or the host's own next
+// launch, must not find it there.
 ftb_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();
     g_err = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? FTB_ERR_OOM : FTB_ERR_CUDA;
 }

@@ -1,0 +1,213 @@
+// Device memory and stream order of the render entry points (ftb_api.cpp) against a CUDA
+// runtime made of host memory (test infrastructure, built and run by
+// tests/test_render_memory.py).  cudaMalloc fails past a limit, launches of the wave buffers
+// are recorded instead of run, and the runtime knows which launches each stream, event and
+// synchronization is ordered after, so a render that runs out of memory can be looked at
+// without a device: what it launched, what is still in flight when it returns, and whether a
+// CUDA error is left on the thread.
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include <set>
+
+#include "../goodphotons_b200/csrc/ftb_api.cpp"
+
+// ---- the runtime ------------------------------------------------------------------------
+namespace fake {
+struct Launch { const char *lo, *hi; int64_t photons; };
+std::vector<Launch> launches;
+std::map<cudaStream_t, std::set<int>> after;         // launches a stream's next work runs after
+std::map<cudaEvent_t, std::set<int>> recorded;
+std::set<int> done;                                  // known to the host to have ended
+std::map<void*, size_t> blocks;
+size_t live = 0, peak = 0, limit = SIZE_MAX;
+int events = 0, overlaps = 0, launch_fails_at = -1;
+uintptr_t handles = 0;
+cudaError_t last = cudaSuccess;
+
+cudaError_t err(cudaError_t e) { if (e != cudaSuccess) last = e; return e; }
+cudaError_t take(void** p, size_t n) {
+    if (live + n > limit) return err(cudaErrorMemoryAllocation);
+    *p = std::calloc(1, n ? n : 1);
+    blocks[*p] = n;
+    live += n;
+    peak = std::max(peak, live);
+    return cudaSuccess;
+}
+void give(void* p) {
+    if (!p) return;
+    live -= blocks[p];
+    blocks.erase(p);
+    std::free(p);
+}
+void sync(cudaStream_t s) { done.insert(after[s].begin(), after[s].end()); }
+cudaError_t launch(const ftb::Wave& w, int64_t photons, cudaStream_t st) {
+    if ((int)launches.size() == launch_fails_at) return err(cudaErrorLaunchFailure);
+    const Launch l{(const char*)w.block, (const char*)w.block + w.bytes, photons};
+    for (int k = 0; k < (int)launches.size(); ++k)
+        if (launches[k].lo < l.hi && l.lo < launches[k].hi && !done.count(k) && !after[st].count(k)) ++overlaps;
+    after[st].insert((int)launches.size());
+    launches.push_back(l);
+    return cudaSuccess;
+}
+// launches that neither the host nor work issued next to `user` is ordered after
+int in_flight(cudaStream_t user) {
+    int n = 0;
+    for (int k = 0; k < (int)launches.size(); ++k) n += !done.count(k) && !after[user].count(k);
+    return n;
+}
+void reset() {
+    launches.clear(); after.clear(); recorded.clear(); done.clear();
+    overlaps = 0; launch_fails_at = -1; last = cudaSuccess; limit = SIZE_MAX; peak = live;
+}
+}  // namespace fake
+
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) { return fake::take(p, n); }
+cudaError_t cudaFree(void* p) { fake::give(p); return cudaSuccess; }
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return fake::take(p, n); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { fake::give(p); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::calloc(1, n); return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemset(void* d, int v, size_t n) { std::memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { std::memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = *t = 0; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) { std::memset(p, 0, sizeof *p); return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+const char* cudaGetErrorString(cudaError_t) { return "error"; }
+cudaError_t cudaGetLastError() { cudaError_t e = fake::last; fake::last = cudaSuccess; return e; }
+cudaError_t cudaPeekAtLastError() { return fake::last; }
+cudaError_t cudaDeviceSynchronize() {
+    for (int k = 0; k < (int)fake::launches.size(); ++k) fake::done.insert(k);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)(++fake::handles); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { fake::sync(s); return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+    fake::after[s].insert(fake::recorded[e].begin(), fake::recorded[e].end());
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t* e) { ++fake::events; *e = (cudaEvent_t)(++fake::handles); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t) { --fake::events; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { fake::recorded[e] = fake::after[s]; return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    fake::done.insert(fake::recorded[e].begin(), fake::recorded[e].end());
+    return cudaSuccess;
+}
+cudaError_t cudaEventElapsedTime(float* t, cudaEvent_t, cudaEvent_t) { *t = 1.0f; return cudaSuccess; }
+}
+
+namespace ftb {
+void wave_carve(Wave& w, void* block, int32_t W, bool log, int32_t hero) {
+    w = Wave{};
+    w.W = W;
+    w.hero = hero > 1 ? hero : 1;
+    w.bytes = wave_bytes(W, log, hero);
+    w.block = block;
+    w.jobs = (DevJob*)block;
+    w.params = (int32_t*)((char*)block + sizeof(DevJob) * kWaveJobs);
+}
+cudaError_t wave_alloc(Wave& w, int32_t W, bool log, int32_t hero) {
+    void* block = nullptr;
+    cudaError_t e = cudaMalloc(&block, wave_bytes(W, log, hero));
+    if (e != cudaSuccess) { w = Wave{}; return e; }
+    wave_carve(w, block, W, log, hero);
+    return cudaSuccess;
+}
+void wave_free(Wave& w) {
+    if (w.block) cudaFree(w.block);
+    w.block = nullptr;
+}
+struct WaveGraphs {};
+WaveGraphs* wave_graphs_create() { return new WaveGraphs(); }
+void wave_graphs_destroy(WaveGraphs* g) { delete g; }
+int32_t trace_limit(int32_t) { return 75776; }
+// as the real ones: launches without a graph end in a look at the thread's last error
+cudaError_t launch_stream(Wave& w, int64_t photons, int32_t, const WaveKind&, const Frame&, int32_t,
+                          const LaunchShape& shape, cudaStream_t st, LaunchSink*, WaveGraphs*) {
+    cudaError_t e = fake::launch(w, photons, st);
+    return e != cudaSuccess || shape.graph ? e : cudaGetLastError();
+}
+cudaError_t launch_wave(Wave& w, int32_t, const WaveKind&, const Frame&, int32_t, const LaunchShape& shape,
+                        cudaStream_t st, LaunchSink*, WaveGraphs*, bool) {
+    cudaError_t e = fake::launch(w, w.params[1], st);
+    return e != cudaSuccess || shape.graph ? e : cudaGetLastError();
+}
+bool build_wide_lbvh_device(const std::vector<Box>&, int, int, WideBvh&, std::string& err) {
+    err = "no device";
+    return false;
+}
+}  // namespace ftb
+
+// ---- renders ----------------------------------------------------------------------------
+namespace {
+constexpr int32_t kSlots = 4096;
+int failures = 0;
+void check(bool ok, const char* what, const std::string& where) {
+    if (!ok) { std::printf("%s: %s\n", where.c_str(), what); ++failures; }
+}
+
+struct Host {   // a scene without geometry: nothing is launched for real
+    ftb_scene* s = new ftb_scene();
+    ftb_camera cam{};
+    std::vector<int64_t> film = std::vector<int64_t>(4 * 4 * 4);
+    Host(int regenerate, int graphs) {
+        ftb_tuning t{};
+        t.wave_slots = kSlots; t.grid_mult = 16; t.use_graphs = graphs; t.regenerate = regenerate;
+        ftb_set_tuning(0, &t);
+        s->eng = engine_for(0);
+        s->tables = std::make_shared<DevBlock>();
+        s->power = 1.0;
+        cam.res_x = cam.res_y = 4;
+    }
+    ~Host() { delete s; }
+    ftb_status batch(const std::vector<int>& heroes, int64_t n, cudaStream_t user) {
+        std::vector<ftb_job> jobs;
+        for (int h : heroes) {
+            ftb_job j{};
+            j.scene = s; j.cam = cam; j.d_film = film.data(); j.n_photons = n; j.max_bounce = 4; j.hero_c = h;
+            jobs.push_back(j);
+        }
+        return ftb_render_batch(jobs.data(), (int32_t)jobs.size(), nullptr, nullptr, user);
+    }
+};
+int64_t photons_launched(size_t from) {
+    int64_t n = 0;
+    for (size_t k = from; k < fake::launches.size(); ++k) n += fake::launches[k].photons;
+    return n;
+}
+
+// A buffer of twice the slots does not fit, one of the slots does: the render is whole and
+// leaves no error on the thread; and where neither fits, the error is the call's alone.
+void error_left_behind() {
+    for (int graphs : {1, 0})
+        for (bool fits : {true, false}) {
+            fake::reset();
+            Host h(1, graphs);
+            fake::limit = fake::live + 4096 + ftb::wave_bytes(kSlots, false) * (fits ? 3 : 1) / 2;
+            const std::string where = "graphs " + std::to_string(graphs) + (fits ? " fits" : " too large");
+            const ftb_status st = h.batch({1, 1}, 3 * kSlots, nullptr);
+            check(st == (fits ? FTB_OK : FTB_ERR_OOM), "status", where + " " + ftb_last_error());
+            check(photons_launched(0) == (fits ? 6 * kSlots : 0), "photons launched", where);
+            check(fake::last == cudaSuccess, "a CUDA error is left on the thread", where);
+        }
+}
+}  // namespace
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "error_left_behind") error_left_behind();
+    else return 2;
+    std::printf("%s: %s\n", what.c_str(), failures ? "wrong" : "ok");
+    return failures ? 1 : 0;
+}
