@@ -667,8 +667,8 @@ DevCam dev_cam(const ftb_camera* c) {
     return d;
 }
 
-// The first wave buffer, of at least W paths.  The second is made when a render has a second
-// wave or pass to put in it (ensure_second_wave).
+// The first wave buffer, of at least W paths.  The second is made before the first launch of a
+// render that has a second wave or pass to put in it (ensure_second_wave).
 ftb_status ensure_waves(ftb_scene* s, int32_t W, bool log, int32_t hero = 1) {
     Engine& e = *s->eng;
     if (e.wave_W >= W && e.wave_log == log && e.waves[0].block && e.waves[0].hero >= hero) return FTB_OK;
@@ -764,35 +764,31 @@ bool one_pass(const ftb::LaunchShape& shape, const std::vector<ftb::DevJob>& bas
     return pieces <= ftb::kWaveJobs;
 }
 
-// Pack jobs' photon ranges into waves of at most W slots and kWaveJobs segments, launch
-// them alternately on the scene's two streams (handing off from and back to `user_stream`).
-// `base[j]` is job j's DevJob template; each segment gets its photon0 / slot range.
-ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const std::vector<int64_t>& count,
-                    const std::vector<uint64_t>& seed, bool log, ftb_photon_log* d_logs, int64_t log_base,
-                    cudaStream_t user_stream) {
-    int64_t total = 0;
-    int32_t hero = 1, fanout = 1;
-    for (size_t i = 0; i < count.size(); ++i) {
-        total += count[i];
-        hero = std::max(hero, base[i].hero_c);
-        fanout = std::max(fanout, ftb::conn_fanout(base[i]));
+// Whether run_jobs makes one wave of W slots of these jobs: few enough of them, one class, and
+// all their photons within the slots that the largest fan-out leaves.
+bool one_wave(int32_t W, const std::vector<ftb::DevJob>& base, const std::vector<int64_t>& count) {
+    int64_t total = 0, cap = W;
+    int jobs = 0;
+    const ftb::DevJob* first = nullptr;
+    for (size_t j = 0; j < base.size(); ++j) {
+        if (count[j] <= 0) continue;
+        if (!first) first = &base[j];
+        if ((base[j].hero_c > 1) != (first->hero_c > 1)) return false;
+        cap = std::min<int64_t>(cap, std::max(1, W / ftb::conn_fanout(base[j])));
+        total += count[j];
+        ++jobs;
     }
-    // A render that is one streaming pass has no second wave beside it, so its buffer takes the
-    // room of both: with twice the paths in flight a frame has half as many launches that end
-    // on their slowest warps (glass, 2^27 photons, 2^22 against 2^23 paths: 220.8 / 214.1 ms).
-    // A pass keeps W / fanout paths in flight, so few photons of a large fan-out get more room.
-    const int64_t cap = s->eng->wave_cap, room = one_pass(s->eng->shape, base, count) ? 2 * cap : cap;
-    int32_t W = pick_wave(std::min(total, room) * fanout, (int32_t)room);
-    ftb_status st = ensure_waves(s, W, log, hero);   // may keep a larger buffer; waves use W slots
-    if (st == FTB_ERR_OOM && W > cap) st = ensure_waves(s, W = (int32_t)cap, log, hero);
-    if (st != FTB_OK) return st;
+    return jobs <= ftb::kWaveJobs && total <= cap;
+}
+
+// Launch the passes or waves of run_jobs, of at most W slots each, alternately on `buffers`
+// wave buffers and their streams.
+ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<ftb::DevJob>& base,
+                       const std::vector<int64_t>& count, const std::vector<uint64_t>& seed, ftb_photon_log* d_logs,
+                       int64_t log_base) {
     ftb::Frame f;
     f.stats = s->prof_mode == 2 ? s->stats : nullptr;
     f.status = s->eng->status;
-    cudaEvent_t ready = nullptr;
-    CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "event");
-    CK(cudaEventRecord(ready, user_stream), "event record");
-    for (auto st2 : s->eng->streams) CK(cudaStreamWaitEvent(st2, ready, 0), "stream wait");
     size_t j = 0;
     int64_t done_in_job = 0;
     int k = 0;
@@ -836,13 +832,13 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         }
         if (table.empty()) break;
         slots = (int32_t)std::min<int64_t>(slots, std::max<int64_t>(1, g));
-        if ((k & 1) && (st = ensure_second_wave(s, W)) != FTB_OK) return st;
-        ftb::Wave& w = s->eng->waves[k & 1];
-        cudaStream_t ws = s->eng->streams[k & 1];
+        const int b = k % buffers;
+        ftb::Wave& w = s->eng->waves[b];
+        cudaStream_t ws = s->eng->streams[b];
         w.logs = d_logs;
         w.log_base = log_base;
-        cudaError_t e = s->eng->stage[k & 1].push(table.data(), (int)table.size(), slots, w, ws, g,
-                                                  ftb::stream_half_cap(g, slots, max_bounce));
+        cudaError_t e = s->eng->stage[b].push(table.data(), (int)table.size(), slots, w, ws, g,
+                                              ftb::stream_half_cap(g, slots, max_bounce));
         if (e != cudaSuccess) return cuda_fail(e, "job table upload");
         ftb::WaveKind kind;
         kind.instances = inst;
@@ -853,7 +849,7 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.deep = deep;
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
-                               s->eng->graphs[k & 1]);
+                               s->eng->graphs[b]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
         ++k;
     }
@@ -891,12 +887,12 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
             if (done_in_job >= count[j]) { ++j; done_in_job = 0; }
         }
         if (table.empty()) break;
-        if ((k & 1) && (st = ensure_second_wave(s, W)) != FTB_OK) return st;
-        ftb::Wave& w = s->eng->waves[k & 1];
-        cudaStream_t ws = s->eng->streams[k & 1];
+        const int b = k % buffers;
+        ftb::Wave& w = s->eng->waves[b];
+        cudaStream_t ws = s->eng->streams[b];
         w.logs = d_logs;
         w.log_base = log_base;
-        cudaError_t e = s->eng->stage[k & 1].push(table.data(), (int)table.size(), slots, w, ws);
+        cudaError_t e = s->eng->stage[b].push(table.data(), (int)table.size(), slots, w, ws);
         if (e != cudaSuccess) return cuda_fail(e, "job table upload");
         ftb::WaveKind kind;
         kind.instances = inst;
@@ -907,16 +903,59 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
         kind.deep = deep;
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
-                             s->eng->graphs[k & 1]);
+                             s->eng->graphs[b]);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
         ++k;
     }
-    for (auto st2 : s->eng->streams) {
-        CK(cudaEventRecord(ready, st2), "event record");
-        CK(cudaStreamWaitEvent(user_stream, ready, 0), "stream wait");
-    }
-    cudaEventDestroy(ready);
     return FTB_OK;
+}
+
+// Pack jobs' photon ranges into waves of at most W slots and kWaveJobs segments, launch
+// them alternately on the scene's two streams (handing off from and back to `user_stream`).
+// `base[j]` is job j's DevJob template; each segment gets its photon0 / slot range.  All device
+// memory is made before the first launch, and a call that fails returns with nothing in flight.
+ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const std::vector<int64_t>& count,
+                    const std::vector<uint64_t>& seed, bool log, ftb_photon_log* d_logs, int64_t log_base,
+                    cudaStream_t user_stream) {
+    int64_t total = 0;
+    int32_t hero = 1, fanout = 1;
+    for (size_t i = 0; i < count.size(); ++i) {
+        total += count[i];
+        hero = std::max(hero, base[i].hero_c);
+        fanout = std::max(fanout, ftb::conn_fanout(base[i]));
+    }
+    // A render that is one streaming pass has no second wave beside it, so its buffer takes the
+    // room of both: with twice the paths in flight a frame has half as many launches that end
+    // on their slowest warps (glass, 2^27 photons, 2^22 against 2^23 paths: 220.8 / 214.1 ms).
+    // A pass keeps W / fanout paths in flight, so few photons of a large fan-out get more room.
+    const bool pass = one_pass(s->eng->shape, base, count);
+    const int64_t cap = s->eng->wave_cap, room = pass ? 2 * cap : cap;
+    int32_t W = pick_wave(std::min(total, room) * fanout, (int32_t)room);
+    ftb_status st = ensure_waves(s, W, log, hero);   // may keep a larger buffer; waves use W slots
+    if (st == FTB_ERR_OOM && W > cap) st = ensure_waves(s, W = (int32_t)cap, log, hero);
+    if (st != FTB_OK) return st;
+    // Where the second buffer does not fit, the first one takes every pass, one after another.
+    int buffers = pass || (!s->eng->shape.regenerate && one_wave(W, base, count)) ? 1 : 2;
+    if (buffers == 2 && (st = ensure_second_wave(s, W)) != FTB_OK) {
+        if (st != FTB_ERR_OOM) return st;
+        buffers = 1;
+        st = FTB_OK;
+    }
+    cudaEvent_t ready = nullptr;
+    CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "event");
+    cudaError_t e = cudaEventRecord(ready, user_stream);
+    for (auto es : s->eng->streams) if (e == cudaSuccess) e = cudaStreamWaitEvent(es, ready, 0);
+    if (e == cudaSuccess) st = launch_jobs(s, W, buffers, base, count, seed, d_logs, log_base);
+    for (auto es : s->eng->streams) {
+        if (e == cudaSuccess) e = cudaEventRecord(ready, es);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(user_stream, ready, 0);
+    }
+    // The caller may give its film back at once when the call has failed: wait for what was
+    // launched before the failure.
+    if (st != FTB_OK || e != cudaSuccess)
+        for (auto es : s->eng->streams) cudaStreamSynchronize(es);
+    cudaEventDestroy(ready);
+    return st != FTB_OK || e == cudaSuccess ? st : cuda_fail(e, "stream order");
 }
 
 // Trace n photons from seed_base into d_film / tally, on the scene's streams.

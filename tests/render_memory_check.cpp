@@ -202,11 +202,58 @@ void error_left_behind() {
             check(fake::last == cudaSuccess, "a CUDA error is left on the thread", where);
         }
 }
+
+// Memory limits from nothing to plenty under renders of one and of several passes or waves:
+// the render is whole, or it fails with nothing in flight.
+void second_buffer() {
+    for (int regenerate : {1, 0})
+        for (int graphs : {1, 0})
+            for (const std::vector<int>& heroes : {std::vector<int>{1, 1}, std::vector<int>{1, 4, 1}}) {
+                int whole = 0, refused = 0;
+                const size_t step = ftb::wave_bytes(kSlots, false, 4) / 3;
+                for (size_t limit = 0; limit <= 12 * step; limit += step) {
+                    fake::reset();
+                    Host h(regenerate, graphs);
+                    fake::limit = fake::live + 4096 + limit;
+                    const cudaStream_t user = (cudaStream_t)(uintptr_t)77777;
+                    const ftb_status st = h.batch(heroes, 3 * kSlots, user);
+                    const std::string where = "regenerate " + std::to_string(regenerate) + " graphs " +
+                                              std::to_string(graphs) + " jobs " + std::to_string(heroes.size()) +
+                                              " limit " + std::to_string(limit);
+                    check(fake::overlaps == 0, "a buffer is used by two launches at once", where);
+                    check(fake::in_flight(user) == 0, "launches are in flight beside the caller's stream", where);
+                    if (st == FTB_OK) {
+                        ++whole;
+                        check(photons_launched(0) == (int64_t)heroes.size() * 3 * kSlots, "photons are missing", where);
+                    } else {
+                        ++refused;
+                        check(st == FTB_ERR_OOM, "another error than out of memory", where);
+                        check(fake::launches.empty(), "launches before the render was refused", where);
+                    }
+                }
+                check(whole > 0 && refused > 0, "limits that do not bite", std::to_string(whole));
+            }
+    // a launch that fails after others: nothing stays in flight, and the event is given back
+    for (int regenerate : {1, 0}) {
+        fake::reset();
+        Host h(regenerate, 1);
+        const cudaStream_t user = (cudaStream_t)(uintptr_t)77777;
+        check(h.batch({1, 4, 1}, 3 * kSlots, user) == FTB_OK, "render", "warm");
+        fake::reset();
+        const int events = fake::events;
+        fake::launch_fails_at = 2;
+        check(h.batch({1, 4, 1}, 3 * kSlots, user) == FTB_ERR_CUDA, "no error", "failing launch");
+        for (int k = 0; k < (int)fake::launches.size(); ++k)
+            check(fake::done.count(k) == 1, "a launch is in flight after the error", "failing launch");
+        check(fake::events == events, "an event is lost", "failing launch");
+    }
+}
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "error_left_behind") error_left_behind();
+    else if (what == "second_buffer") second_buffer();
     else return 2;
     std::printf("%s: %s\n", what.c_str(), failures ? "wrong" : "ok");
     return failures ? 1 : 0;

@@ -30,3 +30,7 @@ def check(tmp_path_factory):
 
 def test_no_error_is_left_on_the_thread(check):
     check("error_left_behind")
+
+
+def test_nothing_is_in_flight_after_a_failed_render(check):
+    check("second_buffer")
