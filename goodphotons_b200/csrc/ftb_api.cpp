@@ -281,14 +281,19 @@ struct ftb_blas {
 namespace {
 // The wave buffers, streams and scratch every render on one device uses.  Shared by all
 // scenes of the device (a scene, its clones, the scenes of a batch), so their number does
-// not multiply the ~300 B per wave slot; renders on a device serialize on `mu`.
+// not multiply the ~640 B per wave slot (ftb::wave_bytes); renders on a device serialize on
+// `mu`.
 struct Engine {
     int device = 0;
     std::mutex mu;
     cudaStream_t streams[2] = {nullptr, nullptr};
-    ftb::Wave waves[2]{};
+    // One allocation in two forms: whole, for a render of one pass or wave, or as two halves,
+    // on a stream each, for one of several -- a device never holds more than the two buffers
+    // of the footprint.  Launches in one form come after those of the other.
+    void* block = nullptr;
+    ftb::Wave whole{}, half[2]{};
+    int32_t buffers_used = 0;         // the form of the last render: 1 whole, 2 halves
     JobStage stage[2];
-    int32_t wave_W = 0;
     bool wave_log = false;
     int64_t* film = nullptr;          // film of the host-film entry points
     size_t film_words = 0;
@@ -296,7 +301,7 @@ struct Engine {
     int32_t* status = nullptr;
     unsigned long long* batch_tally = nullptr;   // 8 words per job of the last batch
     size_t batch_cap = 0;
-    ftb::WaveGraphs* graphs[2] = {nullptr, nullptr};
+    ftb::WaveGraphs* graphs[3] = {nullptr, nullptr, nullptr};   // of the whole and of each half
     ftb::LaunchShape shape;                      // grid and graph choice (autotuned)
     int32_t wave_cap = 1 << 22;                  // largest wave (autotuned)
     ~Engine() {
@@ -304,7 +309,7 @@ struct Engine {
         cudaGetDevice(&cur);
         cudaSetDevice(device);
         for (auto g : graphs) ftb::wave_graphs_destroy(g);
-        for (auto& w : waves) ftb::wave_free(w);
+        if (block) cudaFree(block);
         for (auto s : streams) if (s) cudaStreamDestroy(s);
         if (film) cudaFree(film);
         if (tally) cudaFree(tally);
@@ -667,38 +672,42 @@ DevCam dev_cam(const ftb_camera* c) {
     return d;
 }
 
-// The first wave buffer, of at least W paths.  The second is made before the first launch of a
-// render that has a second wave or pass to put in it (ensure_second_wave).
-ftb_status ensure_waves(ftb_scene* s, int32_t W, bool log, int32_t hero = 1) {
+// Wave buffers of at least W paths: one, or two beside each other.  A larger block that is
+// there already is kept, and its room where it has to be made anew (for logs, or for bundles of
+// more wavelengths), unless only the room asked for fits.
+ftb_status ensure_waves(ftb_scene* s, int32_t W, int buffers, bool log, int32_t hero) {
     Engine& e = *s->eng;
-    if (e.wave_W >= W && e.wave_log == log && e.waves[0].block && e.waves[0].hero >= hero) return FTB_OK;
-    hero = std::max(hero, e.waves[0].block ? e.waves[0].hero : 1);   // keep the bundle room
-    if (e.wave_log == log) W = std::max(W, e.wave_W);
-    for (auto& w : e.waves) ftb::wave_free(w);
+    if (e.block && e.wave_log == log && e.whole.hero >= hero && W <= (buffers == 2 ? e.half[0].W : e.whole.W))
+        return FTB_OK;
+    for (auto& st : e.streams)
+        if (!st) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream create");
+    for (auto& sg : e.stage) CK(sg.init(), "job staging");
+    const int32_t kept_W = e.block && e.wave_log == log ? e.whole.W : 0, kept_hero = e.block ? e.whole.hero : 1;
+    if (e.block) cudaFree(e.block);
+    e.block = nullptr;
+    e.whole = e.half[0] = e.half[1] = ftb::Wave{};
     for (auto& g : e.graphs) {   // captured graphs hold the old buffers' addresses
         ftb::wave_graphs_destroy(g);
         g = ftb::wave_graphs_create();
     }
-    e.wave_W = 0;
-    cudaError_t err = ftb::wave_alloc(e.waves[0], W, log, hero);
-    if (err != cudaSuccess) return cuda_fail(err, "wave allocation");
-    for (auto& st : e.streams)
-        if (!st) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream create");
-    CK(e.stage[0].init(), "job staging");
-    e.wave_W = W;
+    const int32_t least = buffers * W;
+    int32_t room = std::max(least, kept_W), bundle = std::max(hero, kept_hero);
+    auto bytes = [&] {
+        return std::max(ftb::wave_bytes(room, log, bundle), 2 * ftb::wave_bytes(std::max(1, room / 2), log, bundle));
+    };
+    cudaError_t err = cudaMalloc(&e.block, bytes());
+    if (err == cudaErrorMemoryAllocation && (room > least || bundle > hero)) {
+        cudaGetLastError();
+        room = least;
+        bundle = hero;
+        err = cudaMalloc(&e.block, bytes());
+    }
+    if (err != cudaSuccess) { e.block = nullptr; return cuda_fail(err, "wave allocation"); }
+    const int32_t half = std::max(1, room / 2);
+    ftb::wave_carve(e.whole, e.block, room, log, bundle);
+    for (int b = 0; b < 2; ++b)
+        ftb::wave_carve(e.half[b], (char*)e.block + b * ftb::wave_bytes(half, log, bundle), half, log, bundle);
     e.wave_log = log;
-    return FTB_OK;
-}
-ftb_status ensure_second_wave(ftb_scene* s, int32_t W) {
-    Engine& e = *s->eng;
-    ftb::Wave& w = e.waves[1];
-    if (w.block && w.W >= W && w.hero >= e.waves[0].hero) return FTB_OK;
-    ftb::wave_free(w);
-    ftb::wave_graphs_destroy(e.graphs[1]);
-    e.graphs[1] = ftb::wave_graphs_create();
-    cudaError_t err = ftb::wave_alloc(w, W, e.wave_log, e.waves[0].hero);
-    if (err != cudaSuccess) return cuda_fail(err, "wave allocation");
-    CK(e.stage[1].init(), "job staging");
     return FTB_OK;
 }
 
@@ -781,8 +790,8 @@ bool one_wave(int32_t W, const std::vector<ftb::DevJob>& base, const std::vector
     return jobs <= ftb::kWaveJobs && total <= cap;
 }
 
-// Launch the passes or waves of run_jobs, of at most W slots each, alternately on `buffers`
-// wave buffers and their streams.
+// Launch the passes or waves of run_jobs, of at most W slots each, on the whole buffer or
+// alternately on its two halves and their streams.
 ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<ftb::DevJob>& base,
                        const std::vector<int64_t>& count, const std::vector<uint64_t>& seed, ftb_photon_log* d_logs,
                        int64_t log_base) {
@@ -833,7 +842,8 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         if (table.empty()) break;
         slots = (int32_t)std::min<int64_t>(slots, std::max<int64_t>(1, g));
         const int b = k % buffers;
-        ftb::Wave& w = s->eng->waves[b];
+        ftb::Wave& w = buffers == 2 ? s->eng->half[b] : s->eng->whole;
+        ftb::WaveGraphs* graphs = s->eng->graphs[buffers == 2 ? 1 + b : 0];
         cudaStream_t ws = s->eng->streams[b];
         w.logs = d_logs;
         w.log_base = log_base;
@@ -849,7 +859,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.deep = deep;
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
-                               s->eng->graphs[b]);
+                               graphs);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
         ++k;
     }
@@ -888,7 +898,8 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         }
         if (table.empty()) break;
         const int b = k % buffers;
-        ftb::Wave& w = s->eng->waves[b];
+        ftb::Wave& w = buffers == 2 ? s->eng->half[b] : s->eng->whole;
+        ftb::WaveGraphs* graphs = s->eng->graphs[buffers == 2 ? 1 + b : 0];
         cudaStream_t ws = s->eng->streams[b];
         w.logs = d_logs;
         w.log_base = log_base;
@@ -903,7 +914,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.deep = deep;
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
-                             s->eng->graphs[b]);
+                             graphs);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
         ++k;
     }
@@ -931,20 +942,23 @@ ftb_status run_jobs(ftb_scene* s, const std::vector<ftb::DevJob>& base, const st
     const bool pass = one_pass(s->eng->shape, base, count);
     const int64_t cap = s->eng->wave_cap, room = pass ? 2 * cap : cap;
     int32_t W = pick_wave(std::min(total, room) * fanout, (int32_t)room);
-    ftb_status st = ensure_waves(s, W, log, hero);   // may keep a larger buffer; waves use W slots
-    if (st == FTB_ERR_OOM && W > cap) st = ensure_waves(s, W = (int32_t)cap, log, hero);
-    if (st != FTB_OK) return st;
-    // Where the second buffer does not fit, the first one takes every pass, one after another.
+    // Where two buffers do not fit, one takes every pass, one after another; where a buffer of
+    // the room of both does not, one of the tuning's slots does.
     int buffers = pass || (!s->eng->shape.regenerate && one_wave(W, base, count)) ? 1 : 2;
-    if (buffers == 2 && (st = ensure_second_wave(s, W)) != FTB_OK) {
-        if (st != FTB_ERR_OOM) return st;
-        buffers = 1;
-        st = FTB_OK;
-    }
+    ftb_status st = ensure_waves(s, W, buffers, log, hero);   // may keep larger buffers; waves use W slots
+    if (st == FTB_ERR_OOM && buffers == 2) st = ensure_waves(s, W, buffers = 1, log, hero);
+    if (st == FTB_ERR_OOM && W > cap) st = ensure_waves(s, W = (int32_t)cap, buffers, log, hero);
+    if (st != FTB_OK) return st;
     cudaEvent_t ready = nullptr;
     CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "event");
     cudaError_t e = cudaEventRecord(ready, user_stream);
     for (auto es : s->eng->streams) if (e == cudaSuccess) e = cudaStreamWaitEvent(es, ready, 0);
+    if (s->eng->buffers_used != buffers)   // the forms share their memory, on other streams
+        for (int b = 0; b < 2; ++b) {
+            if (e == cudaSuccess) e = cudaEventRecord(ready, s->eng->streams[b]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(s->eng->streams[1 - b], ready, 0);
+        }
+    s->eng->buffers_used = buffers;
     if (e == cudaSuccess) st = launch_jobs(s, W, buffers, base, count, seed, d_logs, log_base);
     for (auto es : s->eng->streams) {
         if (e == cudaSuccess) e = cudaEventRecord(ready, es);

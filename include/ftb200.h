@@ -257,7 +257,9 @@ typedef struct ftb_footprint {
     uint64_t scene_bytes;     /* BVH + primitive records + tables */
     uint64_t film_bytes;      /* per camera film */
     uint64_t wave_bytes;      /* path state, queues and connection records of the device's
-                                 two wave buffers at its current tuning (wave_slots) */
+                                 two wave buffers at its current tuning (wave_slots), all
+                                 that its renders hold at once: ~640 B per slot and buffer,
+                                 ~80 C more once bundles of C wavelengths were rendered */
     uint64_t total_bytes;
 } ftb_footprint;
 
@@ -456,15 +458,16 @@ ftb_status ftb_scene_set_profiling(ftb_scene* scene, int32_t mode);
 ftb_status ftb_scene_profile(ftb_scene* scene, ftb_kernel_profile* out, int32_t reset);
 
 /* ---- launch tuning (no counterpart in the reference) ---------------------------------
- * How a device's renders are launched: photon slots per wave (path state is ~400 B per
- * slot, two waves in flight), blocks per SM of the queue-driven kernels, whether each
+ * How a device's renders are launched: photon slots per wave (~640 B per slot,
+ * two waves in flight), blocks per SM of the queue-driven kernels, whether each
  * wave's bounce loop (about 5 launches per bounce) is replayed from a captured CUDA graph,
  * and whether closest-hit rays are always ordered before traversal.
  * Renders on the device use the setting current when they start; results do not depend on
  * it (photons are keyed by index, films are fixed point). */
 typedef struct ftb_tuning {
     int32_t wave_slots;   /* paths in flight per wave buffer, 1 .. 2^24; a render that is one
-                             streaming pass takes the room of both buffers as one */
+                             streaming pass takes the room of both buffers as one, and one
+                             buffer serves where the device has no room for two */
     int32_t grid_mult;    /* 1 .. 64 */
     int32_t use_graphs;   /* 0 / 1 */
     int32_t sort_rays;    /* reorder closest-hit rays by origin and direction before traversal:

@@ -64,7 +64,11 @@ void reset() {
 
 extern "C" {
 cudaError_t cudaMalloc(void** p, size_t n) { return fake::take(p, n); }
-cudaError_t cudaFree(void* p) { fake::give(p); return cudaSuccess; }
+cudaError_t cudaFree(void* p) {   // waits for the device
+    for (int k = 0; k < (int)fake::launches.size(); ++k) fake::done.insert(k);
+    fake::give(p);
+    return cudaSuccess;
+}
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return fake::take(p, n); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { fake::give(p); return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::calloc(1, n); return cudaSuccess; }
@@ -248,12 +252,38 @@ void second_buffer() {
         check(fake::events == events, "an event is lost", "failing launch");
     }
 }
+
+// Renders of one and of several passes in turn, from streams that do not wait for one another:
+// the device's buffers stay within the footprint the library states, and no launch uses a
+// buffer that another may still be using.
+void stated_memory() {
+    for (int regenerate : {1, 0})
+        for (bool several_first : {true, false}) {
+            fake::reset();
+            Host h(regenerate, 1);
+            const std::vector<int> one{1, 1}, several(300, 1);
+            ftb_footprint fp;
+            check(ftb_scene_footprint(h.s, 4, 4, &fp) == FTB_OK, "footprint", "");
+            const size_t before = fake::live, small = 300 * 64 + 4096;   // tallies, status
+            for (int k = 0; k < 4; ++k) {
+                const bool sev = (k & 1) == (several_first ? 0 : 1);
+                const std::string where = "regenerate " + std::to_string(regenerate) + " render " + std::to_string(k);
+                const size_t from = fake::launches.size();
+                const ftb_status st = h.batch(sev ? several : one, sev ? 100 : 3 * kSlots, (cudaStream_t)(uintptr_t)(90000 + k));
+                check(st == FTB_OK, ftb_last_error(), where);
+                check(!sev || fake::launches.size() - from > 1, "one pass only", where);
+                check(fake::live - before <= fp.wave_bytes + small, "more than the stated buffers", where);
+                check(fake::overlaps == 0, "a buffer is used by two launches at once", where);
+            }
+        }
+}
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "error_left_behind") error_left_behind();
     else if (what == "second_buffer") second_buffer();
+    else if (what == "stated_memory") stated_memory();
     else return 2;
     std::printf("%s: %s\n", what.c_str(), failures ? "wrong" : "ok");
     return failures ? 1 : 0;

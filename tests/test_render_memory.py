@@ -34,3 +34,7 @@ def test_no_error_is_left_on_the_thread(check):
 
 def test_nothing_is_in_flight_after_a_failed_render(check):
     check("second_buffer")
+
+
+def test_buffers_stay_within_the_stated_footprint(check):
+    check("stated_memory")
