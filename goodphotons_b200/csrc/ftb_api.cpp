@@ -324,13 +324,13 @@ std::weak_ptr<Engine> g_engines[256];
 ftb_tuning g_tuning[256];          // per device; a new engine starts from it
 bool g_tuning_set[256] = {};
 
-ftb_tuning default_tuning() { return ftb_tuning{1 << 22, 16, 1, 0, 1}; }
+ftb_tuning default_tuning() { return ftb_tuning{1 << 22, 16, 1, ftb::kSortLarge, 1}; }
 
 void apply_tuning(Engine& e, const ftb_tuning& t) {
     e.wave_cap = t.wave_slots;
     e.shape.grid_mult = t.grid_mult;
     e.shape.graph = t.use_graphs != 0;
-    e.shape.sort_rays = t.sort_rays != 0;
+    e.shape.sort_rays = ftb::sort_setting(t.sort_rays);
     e.shape.regenerate = t.regenerate != 0;
 }
 
@@ -856,7 +856,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
-        kind.deep = deep;
+        kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep);
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                graphs);
@@ -911,7 +911,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
-        kind.deep = deep;
+        kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep);
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                              graphs);
@@ -1957,6 +1957,7 @@ ftb_status ftb_autotune(ftb_scene* s, const ftb_camera* cam, int64_t n, int32_t 
         const int waves[] = {1 << 20, 1 << 21, 1 << 22, 1 << 23, 1 << 24};
         for (int pass = 0; pass < 5 && st == FTB_OK; ++pass) {
             std::vector<ftb_tuning> cand;
+            if (pass == 4) best_ms = 1e300;   // the default, by scene, is the same launches as one of the two
             if (pass == 0) for (int u = 0; u < 2; ++u) { ftb_tuning t = best; t.regenerate = u; cand.push_back(t); }
             if (pass == 1) for (int g : grids) { ftb_tuning t = best; t.grid_mult = g; cand.push_back(t); }
             if (pass == 2) for (int w : waves) { ftb_tuning t = best; t.wave_slots = w; cand.push_back(t); }

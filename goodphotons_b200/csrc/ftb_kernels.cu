@@ -3020,7 +3020,6 @@ struct Issue {
     const WaveKind& kind;
     const Frame& f;
     int grid;
-    bool sorted;
     cudaStream_t st;
     LaunchSink* sink;
     int32_t sms;
@@ -3076,7 +3075,7 @@ struct Issue {
         else if (kind.mirrors) trav<LaunchShadowMirror>(w, (const DevJob*)w.jobs, f);
         else {
             const int32_t* order = nullptr;
-            if (kind.deep) {
+            if (kind.order.connections) {
                 // 4-byte positions in an array of 8-byte values that only bundles and mirror
                 // connections use
                 int32_t* o = reinterpret_cast<int32_t*>(w.slam);
@@ -3113,7 +3112,7 @@ struct Issue {
     void extend(const PathState& in, int32_t* c) {
         mark(K_EXTEND, false);
         const int32_t* order = nullptr;
-        if (sorted) {
+        if (kind.order.rays) {
             k_sort_queue<<<sort_grid(w.W, kRayChunk, 4), kRayThreads, 0, st>>>(w, w.jobs, in, c, w.perm);
             order = w.perm;
         }
@@ -3257,7 +3256,6 @@ struct WaveGraphs {
     struct Entry {
         int32_t max_bounce, grid;   // max_bounce -1: a streaming pass, -2: one of few photons, -3: a wave of few
         WaveKind kind;
-        bool sorted;
         int32_t* status;
         cudaGraphExec_t exec;
     };
@@ -3266,9 +3264,9 @@ struct WaveGraphs {
     ~WaveGraphs() {
         for (auto& e : entries) cudaGraphExecDestroy(e.exec);
     }
-    cudaGraphExec_t find(int32_t max_bounce, int32_t grid, const WaveKind& kind, bool sorted, int32_t* status) const {
+    cudaGraphExec_t find(int32_t max_bounce, int32_t grid, const WaveKind& kind, int32_t* status) const {
         for (auto& e : entries)
-            if (e.max_bounce == max_bounce && e.grid == grid && e.kind == kind && e.sorted == sorted && e.status == status)
+            if (e.max_bounce == max_bounce && e.grid == grid && e.kind == kind && e.status == status)
                 return e.exec;
         return nullptr;
     }
@@ -3294,27 +3292,26 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
                         bool whole_paths) {
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;   // the buffer carries no bundles
     const int grid = launch_grid(w, sms, shape);
-    const bool sorted = shape.sort_rays || kind.deep;
     // A graph bakes the kernel arguments: the wave's buffers and status word are fixed for the
     // life of its cache, but a log buffer changes per call, so logging waves launch directly.
     if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
-        Issue I{w, kind, f, grid, sorted, st, sink, sms};
+        Issue I{w, kind, f, grid, st, sink, sms};
         if (whole_paths) issue_wave_paths(I);
         else issue_wave(I, max_bounce);
         return cudaGetLastError();
     }
     if (whole_paths) max_bounce = -3;
-    if (cudaGraphExec_t ex = graphs->find(max_bounce, grid, kind, sorted, f.status))
+    if (cudaGraphExec_t ex = graphs->find(max_bounce, grid, kind, f.status))
         return cudaGraphLaunch(ex, st);
     cudaGraph_t g = nullptr;
     cudaError_t err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (err != cudaSuccess) return err;
-    Issue I{w, kind, f, grid, sorted, st, nullptr, sms};
+    Issue I{w, kind, f, grid, st, nullptr, sms};
     if (whole_paths) issue_wave_paths(I);
     else issue_wave(I, max_bounce);
     err = cudaStreamEndCapture(st, &g);
     if (err != cudaSuccess) return err;
-    WaveGraphs::Entry e{max_bounce, grid, kind, sorted, f.status, nullptr};
+    WaveGraphs::Entry e{max_bounce, grid, kind, f.status, nullptr};
     err = cudaGraphInstantiate(&e.exec, g, 0);
     cudaGraphDestroy(g);
     if (err != cudaSuccess) return err;
@@ -3326,12 +3323,11 @@ cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKin
                           const LaunchShape& shape, cudaStream_t st, LaunchSink* sink, WaveGraphs* graphs) {
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;
     const int grid = launch_grid(w, sms, shape);
-    const bool sorted = shape.sort_rays || kind.deep;
     const bool few = !f.stats && photons <= std::min(slots, trace_limit(sms));
     if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
         // host-driven: the graph's loop body (two half-iterations) at a time, the progress
         // word read after each, so the launches are the ones a graph replay makes
-        Issue I{w, kind, f, grid, sorted, st, sink, sms};
+        Issue I{w, kind, f, grid, st, sink, sms};
         if (few) {
             stream_paths(I);
             return cudaGetLastError();
@@ -3352,12 +3348,12 @@ cudaError_t launch_stream(Wave& w, int64_t photons, int32_t slots, const WaveKin
         }
     }
     const int32_t key = few ? -2 : -1;
-    if (cudaGraphExec_t ex = graphs->find(key, grid, kind, sorted, f.status)) return cudaGraphLaunch(ex, st);
+    if (cudaGraphExec_t ex = graphs->find(key, grid, kind, f.status)) return cudaGraphLaunch(ex, st);
     // prologue, then a conditional while node whose body is two half-iterations (the queues
     // swap roles between them; the last advance of the body sets the loop condition), then the
     // paths still queued and the connections
-    Issue I{w, kind, f, grid, sorted, st, nullptr, sms};
-    WaveGraphs::Entry entry{key, grid, kind, sorted, f.status, nullptr};
+    Issue I{w, kind, f, grid, st, nullptr, sms};
+    WaveGraphs::Entry entry{key, grid, kind, f.status, nullptr};
     cudaGraph_t g = nullptr;
     cudaError_t err = graphs->side.init();
     if (err != cudaSuccess) return err;

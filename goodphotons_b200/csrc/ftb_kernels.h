@@ -169,12 +169,12 @@ struct LaunchSink {
 };
 
 // Launch shape chosen by the autotuner: blocks per SM of the queue-driven kernels, whether a
-// wave is replayed from a captured CUDA graph, and whether closest-hit rays are always
-// reordered by origin and direction.
+// wave is replayed from a captured CUDA graph, and whether rays are ordered before traversal.
+enum SortRays { kSortNever = 0, kSortAlways = 1, kSortLarge = 2 };   // ftb_tuning.sort_rays
 struct LaunchShape {
     int32_t grid_mult = 16;
     bool graph = true;
-    bool sort_rays = false;   // order closest-hit rays in every scene (large ones always do)
+    int32_t sort_rays = kSortLarge;   // closest-hit rays: in no scene, in every one, where it pays
     bool regenerate = true;   // streaming passes: freed slots are refilled with new photons
 };
 
@@ -184,6 +184,12 @@ struct WaveGraphs;
 WaveGraphs* wave_graphs_create();
 void wave_graphs_destroy(WaveGraphs* g);
 
+// Whether a launch's closest-hit rays are ordered (by origin and direction) and its
+// connections (by image tile) before they are traversed.
+struct RayOrder {
+    bool rays = false, connections = false;
+};
+
 // Which kernel variants a wave needs, from the jobs of its table.
 struct WaveKind {
     bool instances = false;   // some scene has instance records (two-level traversal)
@@ -191,11 +197,12 @@ struct WaveKind {
     bool media = false;       // some scene has participating media
     bool shapes = false;      // some scene has spheres or curves (not only triangles)
     bool mirrors = false;     // some scene has planar mirrors (mirror connections queued)
-    bool deep = false;        // some scene's hierarchy is large (scene_is_deep)
+    RayOrder order;           // which rays are ordered before traversal (ray_order)
     int32_t multi = 0;        // table_class() of the table's jobs (it must be exactly that)
     bool operator==(const WaveKind& o) const {
         return instances == o.instances && bundles == o.bundles && media == o.media && shapes == o.shapes &&
-               mirrors == o.mirrors && deep == o.deep && multi == o.multi;
+               mirrors == o.mirrors && order.rays == o.order.rays && order.connections == o.order.connections &&
+               multi == o.multi;
     }
 };
 // Tables by size: 0 one job, 1 at most kSmallTable, 2 more.  The tally kernels hold a row per
@@ -207,14 +214,23 @@ inline int32_t table_class(size_t jobs) { return jobs <= 1 ? 0 : (jobs <= (size_
 // W / fanout so that the shadow queue (kShadowPerSlot records per slot) cannot overflow.
 inline int conn_fanout(const DevJob& J) { return (J.n_views > 1 ? J.n_views : 1) * (1 + J.sc.n_planes); }
 // Whether ordering a scene's closest-hit rays (by origin and direction) and its connections
-// (by image tile) before traversal pays for itself; launches do it then, whatever the tuning
-// says: the hierarchy has to be large enough that rays near each other share nodes that others
-// do not.  Whole frames with / without the order of the rays, by direction alone (B200): glass
+// (by image tile) before traversal pays for itself: the hierarchy has to be large enough that
+// rays near each other share nodes that others do not.  Whole frames with / without the order of the rays, by direction alone (B200): glass
 // of 327,680 triangles (37 k nodes) 220.8 / 225.4 ms, fog + 250 k strands 113.2 / 116.1, glass
 // of 81,920 triangles (9 k nodes) 25.8 / 25.8, showroom (2 k nodes) 27.75 / 27.75, Cornell (9
 // nodes) 11.9 / 11.4.
 constexpr int32_t kSortNodes = 8192;
 inline bool scene_is_deep(const DevScene& sc) { return sc.max_nodes >= kSortNodes; }
+inline int32_t sort_setting(int32_t sort_rays) {   // of ftb_tuning.sort_rays
+    return sort_rays == kSortLarge ? kSortLarge : (sort_rays ? kSortAlways : kSortNever);
+}
+// The order of a launch; deep: some scene of its jobs is large.
+inline RayOrder ray_order(int32_t setting, bool deep) {
+    RayOrder o;
+    o.rays = setting == kSortAlways || (setting == kSortLarge && deep);
+    o.connections = setting != kSortNever && deep;
+    return o;
+}
 // Whether a scene's world records include spheres or curves.
 inline bool scene_has_shapes(const DevScene& sc) { return (int64_t)sc.n_recs > sc.n_tris + sc.n_inst; }
 

@@ -276,7 +276,7 @@ void start_job_locked(ftb_server* s, Job* j) {
 // to the jobs with the least work left.  cap = the pass's photon budget (4 W in a
 // streaming pass, W in a wave).  One entry per job (mu held).
 int64_t build_table_locked(ftb_server* s, std::vector<ftb::DevJob>& table, std::vector<Job*>& members,
-                           int32_t& max_bounce, ftb::WaveKind& kind, int& fanout) {
+                           int32_t& max_bounce, ftb::WaveKind& kind, int& fanout, bool& deep) {
     std::vector<Job*> c;
     for (Job* j : s->active)
         if (j->next < j->req.n_photons) c.push_back(j);
@@ -308,6 +308,7 @@ int64_t build_table_locked(ftb_server* s, std::vector<ftb::DevJob>& table, std::
     int64_t photons = 0;
     max_bounce = 0;
     fanout = 1;
+    deep = false;
     kind = ftb::WaveKind{};
     for (size_t i = 0; i < c.size(); ++i) {
         if (give[i] <= 0) continue;
@@ -337,7 +338,7 @@ int64_t build_table_locked(ftb_server* s, std::vector<ftb::DevJob>& table, std::
         kind.media |= J.sc.n_med > 0;
         kind.shapes |= ftb::scene_has_shapes(J.sc);
         kind.mirrors |= J.sc.n_planes > 0;
-        kind.deep |= ftb::scene_is_deep(J.sc);
+        deep |= ftb::scene_is_deep(J.sc);
         fanout = std::max(fanout, ftb::conn_fanout(J));
     }
     return photons;
@@ -377,11 +378,12 @@ void scheduler(ftb_server* s) {
         int64_t photons = 0;
         int32_t mb = 0;
         int fanout = 1;
+        bool deep = false;
         ftb::WaveKind kind;
         {
             std::unique_lock<std::mutex> lk(s->mu);
             admit_locked(s);
-            photons = build_table_locked(s, table, members, mb, kind, fanout);
+            photons = build_table_locked(s, table, members, mb, kind, fanout, deep);
             if (photons == 0) {
                 bool busy = s->ws[0].busy || s->ws[1].busy;
                 if (!busy) {
@@ -405,6 +407,7 @@ void scheduler(ftb_server* s) {
         const bool stream = s->shape.regenerate;
         // the pass's connection fan-out (planar mirrors) bounds its paths in flight
         const int32_t slots = (int32_t)std::min<int64_t>(photons, std::max(1, s->W / fanout));
+        kind.order = ftb::ray_order(s->shape.sort_rays, deep);
         int32_t* par = reinterpret_cast<int32_t*>(w.table + ftb::kWaveJobs);
         par[0] = (int32_t)table.size();
         par[1] = slots;
@@ -529,7 +532,7 @@ ftb_status ftb_server_create(const ftb_server_config* cfg, ftb_server** out) {
             if (!cfg->wave_slots) s->W = t.wave_slots;
             s->shape.grid_mult = t.grid_mult;
             s->shape.graph = t.use_graphs != 0;
-            s->shape.sort_rays = t.sort_rays != 0;
+            s->shape.sort_rays = ftb::sort_setting(t.sort_rays);
             s->shape.regenerate = t.regenerate != 0;
         }
     }

@@ -161,7 +161,7 @@ class _Lib:
                    regenerate=None):
         t = self.get_tuning(device)
         if sort_rays is not None:
-            t.sort_rays = int(bool(sort_rays))
+            t.sort_rays = 2 if sort_rays == 2 else int(bool(sort_rays))
         if regenerate is not None:
             t.regenerate = int(bool(regenerate))
         if wave_slots is not None:

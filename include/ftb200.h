@@ -461,7 +461,7 @@ ftb_status ftb_scene_profile(ftb_scene* scene, ftb_kernel_profile* out, int32_t 
  * How a device's renders are launched: photon slots per wave (~640 B per slot,
  * two waves in flight), blocks per SM of the queue-driven kernels, whether each
  * wave's bounce loop (about 5 launches per bounce) is replayed from a captured CUDA graph,
- * and whether closest-hit rays are always ordered before traversal.
+ * and whether rays are ordered before traversal.
  * Renders on the device use the setting current when they start; results do not depend on
  * it (photons are keyed by index, films are fixed point). */
 typedef struct ftb_tuning {
@@ -470,8 +470,10 @@ typedef struct ftb_tuning {
                              buffer serves where the device has no room for two */
     int32_t grid_mult;    /* 1 .. 64 */
     int32_t use_graphs;   /* 0 / 1 */
-    int32_t sort_rays;    /* reorder closest-hit rays by origin and direction before traversal:
-                             1 always, 0 where the scene is large enough to gain */
+    int32_t sort_rays;    /* order closest-hit rays by origin and direction, and connections by
+                             image tile, before traversal: 0 never, 2 (the default) where the
+                             scene is large enough to gain, 1 the rays of every scene and the
+                             connections of large ones */
     int32_t regenerate;   /* 0 / 1: streaming passes -- a slot freed by a finished path is
                              refilled with the next photon at once, so the device stays full
                              until the last photons (1), or waves traced to their last bounce

@@ -1,4 +1,4 @@
-// Device memory and stream order of the render entry points (ftb_api.cpp) against a CUDA
+// Device memory, stream order and ray order of the render entry points (ftb_api.cpp) on a CUDA
 // runtime made of host memory (test infrastructure, built and run by
 // tests/test_render_memory.py).  cudaMalloc fails past a limit, launches of the wave buffers
 // are recorded instead of run, and the runtime knows which launches each stream, event and
@@ -14,7 +14,7 @@
 
 // ---- the runtime ------------------------------------------------------------------------
 namespace fake {
-struct Launch { const char *lo, *hi; int64_t photons; };
+struct Launch { const char *lo, *hi; int64_t photons; ftb::RayOrder order; };
 std::vector<Launch> launches;
 std::map<cudaStream_t, std::set<int>> after;         // launches a stream's next work runs after
 std::map<cudaEvent_t, std::set<int>> recorded;
@@ -41,9 +41,9 @@ void give(void* p) {
     std::free(p);
 }
 void sync(cudaStream_t s) { done.insert(after[s].begin(), after[s].end()); }
-cudaError_t launch(const ftb::Wave& w, int64_t photons, cudaStream_t st) {
+cudaError_t launch(const ftb::Wave& w, int64_t photons, const ftb::WaveKind& kind, cudaStream_t st) {
     if ((int)launches.size() == launch_fails_at) return err(cudaErrorLaunchFailure);
-    const Launch l{(const char*)w.block, (const char*)w.block + w.bytes, photons};
+    const Launch l{(const char*)w.block, (const char*)w.block + w.bytes, photons, kind.order};
     for (int k = 0; k < (int)launches.size(); ++k)
         if (launches[k].lo < l.hi && l.lo < launches[k].hi && !done.count(k) && !after[st].count(k)) ++overlaps;
     after[st].insert((int)launches.size());
@@ -137,14 +137,14 @@ WaveGraphs* wave_graphs_create() { return new WaveGraphs(); }
 void wave_graphs_destroy(WaveGraphs* g) { delete g; }
 int32_t trace_limit(int32_t) { return 75776; }
 // as the real ones: launches without a graph end in a look at the thread's last error
-cudaError_t launch_stream(Wave& w, int64_t photons, int32_t, const WaveKind&, const Frame&, int32_t,
+cudaError_t launch_stream(Wave& w, int64_t photons, int32_t, const WaveKind& kind, const Frame&, int32_t,
                           const LaunchShape& shape, cudaStream_t st, LaunchSink*, WaveGraphs*) {
-    cudaError_t e = fake::launch(w, photons, st);
+    cudaError_t e = fake::launch(w, photons, kind, st);
     return e != cudaSuccess || shape.graph ? e : cudaGetLastError();
 }
-cudaError_t launch_wave(Wave& w, int32_t, const WaveKind&, const Frame&, int32_t, const LaunchShape& shape,
+cudaError_t launch_wave(Wave& w, int32_t, const WaveKind& kind, const Frame&, int32_t, const LaunchShape& shape,
                         cudaStream_t st, LaunchSink*, WaveGraphs*, bool) {
-    cudaError_t e = fake::launch(w, w.params[1], st);
+    cudaError_t e = fake::launch(w, w.params[1], kind, st);
     return e != cudaSuccess || shape.graph ? e : cudaGetLastError();
 }
 bool build_wide_lbvh_device(const std::vector<Box>&, int, int, WideBvh&, std::string& err) {
@@ -165,9 +165,9 @@ struct Host {   // a scene without geometry: nothing is launched for real
     ftb_scene* s = new ftb_scene();
     ftb_camera cam{};
     std::vector<int64_t> film = std::vector<int64_t>(4 * 4 * 4);
-    Host(int regenerate, int graphs) {
+    Host(int regenerate, int graphs, int32_t slots = kSlots, int sort_rays = 2) {
         ftb_tuning t{};
-        t.wave_slots = kSlots; t.grid_mult = 16; t.use_graphs = graphs; t.regenerate = regenerate;
+        t.wave_slots = slots; t.sort_rays = sort_rays; t.grid_mult = 16; t.use_graphs = graphs; t.regenerate = regenerate;
         ftb_set_tuning(0, &t);
         s->eng = engine_for(0);
         s->tables = std::make_shared<DevBlock>();
@@ -277,6 +277,27 @@ void stated_memory() {
             }
         }
 }
+
+// Rays are ordered where the tuning says so: never, always, or where the scene is large.
+void ray_order() {
+    struct Row { int nodes; bool shapes; int32_t slots; bool rays, connections; };   // for sort_rays 2
+    const Row rows[] = {{100000, false, 1 << 22, true, true}, {100, false, 1 << 22, false, false}};
+    for (int regenerate : {1, 0})
+        for (const Row& r : rows)
+            for (int sort_rays : {0, 1, 2}) {
+                fake::reset();
+                Host h(regenerate, 1, 1 << 22, sort_rays);
+                h.s->dev.max_nodes = r.nodes;
+                h.s->dev.n_recs = r.shapes;
+                const std::string where = "sort_rays " + std::to_string(sort_rays) + " nodes " + std::to_string(r.nodes) +
+                                          " paths " + std::to_string(r.slots) + (r.shapes ? " shapes" : "");
+                check(h.batch({1}, r.slots, nullptr) == FTB_OK && fake::launches.size() == 1, ftb_last_error(), where);
+                const ftb::RayOrder o = fake::launches.empty() ? ftb::RayOrder{} : fake::launches[0].order;
+                check(o.rays == (sort_rays == 2 ? r.rays : sort_rays == 1), "closest-hit rays", where);
+                check(o.connections == (sort_rays == 2 ? r.connections : sort_rays == 1 && r.nodes > 10000),
+                      "connections", where);
+            }
+}
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -284,6 +305,7 @@ int main(int argc, char** argv) {
     if (what == "error_left_behind") error_left_behind();
     else if (what == "second_buffer") second_buffer();
     else if (what == "stated_memory") stated_memory();
+    else if (what == "ray_order") ray_order();
     else return 2;
     std::printf("%s: %s\n", what.c_str(), failures ? "wrong" : "ok");
     return failures ? 1 : 0;

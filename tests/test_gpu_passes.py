@@ -58,7 +58,7 @@ def test_passes_equal_whole_paths(gpu, tuning, slots, heroes):
 
 
 @pytest.mark.parametrize("name,build", [
-    ("glass", lambda L: scenes.make_glass(L, freq=90)),                # ~18 k nodes: rays ordered by direction
+    ("glass", lambda L: scenes.make_glass(L, freq=90)),                # ~18 k nodes
     ("fog_strands", lambda L: scenes.make_fog_strands(L, n_strands=40_000)),
     ("instanced", lambda L: scenes.make_glass_instanced(L, level=6)),   # the large hierarchy is the BLAS's
 ])
@@ -68,7 +68,7 @@ def test_ordered_queues_of_large_scenes(gpu, tuning, name, build):
     cam = scenes.default_camera(gpu, 40)
     n, mb = 150_000, 12
     ref, fx = _solo(gpu, torch, sc, cam, n, 5, mb, 1)
-    for kw in (dict(wave_slots=30_000), dict(wave_slots=30_000, regenerate=0)):
+    for kw in (dict(wave_slots=30_000, sort_rays=1), dict(wave_slots=30_000, sort_rays=1, regenerate=0)):
         tuning(**kw)
         film = torch.zeros((40, 40, 4), dtype=torch.int64, device="cuda:0")
         _, en = sc.render_device(cam, n, film.data_ptr(), seed_base=5, max_bounce=mb, frac_bits=24,
@@ -91,7 +91,7 @@ def test_ordered_queues_of_mixed_scenes(gpu, tuning, n_jobs):
         films.append(film)
         jobs.append(dict(scene=scs[k % 3], cam=cam, d_film=film.data_ptr(), n=120_000 // n_jobs + k,
                          seed_base=10_000 * k, max_bounce=6 + k % 5, frac_bits=24))
-    tuning(wave_slots=20_000)
+    tuning(wave_slots=20_000, sort_rays=1)
     _, ens = gpu.render_batch(jobs, stream=torch.cuda.current_stream().cuda_stream)
     tuning(wave_slots=1 << 22)
     for job, film, en in zip(jobs, films, ens):

@@ -1,4 +1,5 @@
-"""Renders that run out of device memory, or whose launches fail: compiles and runs
+"""The host side of renders -- device memory that runs out, launches that fail, the order of rays
+that a tuning asks for: compiles and runs
 tests/render_memory_check.cpp, in which goodphotons_b200/csrc/ftb_api.cpp runs on a CUDA
 runtime made of host memory."""
 import os
@@ -38,3 +39,7 @@ def test_nothing_is_in_flight_after_a_failed_render(check):
 
 def test_buffers_stay_within_the_stated_footprint(check):
     check("stated_memory")
+
+
+def test_rays_are_ordered_as_the_tuning_says(check):
+    check("ray_order")
