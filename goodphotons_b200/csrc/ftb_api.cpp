@@ -856,7 +856,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
-        kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep);
+        kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep, shapes, slots);
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                graphs);
@@ -911,7 +911,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.media = media;
         kind.shapes = shapes;
         kind.mirrors = mirrors;
-        kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep);
+        kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep, shapes, slots);
         kind.multi = ftb::table_class(table.size());
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                              graphs);

@@ -1774,11 +1774,14 @@ __global__ void __launch_bounds__(kRayThreads) k_sort_queue(Wave w, const DevJob
 }
 
 // Traversal order of the queued connections: all of a view's rays end at its eye, so those of
-// one tile of the image (a 16 x 16 grid in Morton order) cross the same nodes.  In large scenes
-// only, as for the closest-hit rays.  Whole frames (B200): fog + strands 110.7 -> 103.7 ms
-// (the connections alone 29.1 -> 24.0), glass 205.6 -> 202.7, animation batch 68.5 -> 66.1,
-// served jobs 83.0 -> 79.1; Cornell, where it does not run, would take 0.4 ms more.  Pieces of
-// 4096 gain 1 ms more on the strands and lose 1.2 on glass.
+// one tile of the image (a 16 x 16 grid in Morton order) cross the same nodes.  Where it runs:
+// ray_order.  Whole frames (B200), beside ordered closest-hit rays: fog + strands 107.4 ->
+// 100.2 ms, glass 200.8 -> 197.8, animation batch 65.8 -> 64.3, served jobs 79.7 -> 75.9;
+// Cornell, where it does not run, would take 0.4 ms more.  The launches themselves, order
+// included and nothing beside them: strands 14 % shorter, triangles 3 to 7 % longer with one
+// view and 5 to 9 % with four, whose rays end at four eyes and share tiles; with the
+// closest-hit launch beside them their frames are shorter all the same.  Pieces of 4096 gain
+// 1 ms more on the strands and lose 1.2 on glass.
 constexpr int kConnChunk = 1024, kConnThreads = 128, kConnKeys = 256;
 __global__ void __launch_bounds__(kConnThreads) k_sort_connections(Wave w, const DevJob* __restrict__ jobs,
                                                                    int32_t* order) {

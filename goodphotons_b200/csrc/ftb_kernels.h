@@ -213,22 +213,44 @@ inline int32_t table_class(size_t jobs) { return jobs <= 1 ? 0 : (jobs <= (size_
 // planar mirror, for each of the job's views.  A wave or pass keeps its slots at most
 // W / fanout so that the shadow queue (kShadowPerSlot records per slot) cannot overflow.
 inline int conn_fanout(const DevJob& J) { return (J.n_views > 1 ? J.n_views : 1) * (1 + J.sc.n_planes); }
-// Whether ordering a scene's closest-hit rays (by origin and direction) and its connections
-// (by image tile) before traversal pays for itself: the hierarchy has to be large enough that
-// rays near each other share nodes that others do not.  Whole frames with / without the order of the rays, by direction alone (B200): glass
-// of 327,680 triangles (37 k nodes) 220.8 / 225.4 ms, fog + 250 k strands 113.2 / 116.1, glass
-// of 81,920 triangles (9 k nodes) 25.8 / 25.8, showroom (2 k nodes) 27.75 / 27.75, Cornell (9
-// nodes) 11.9 / 11.4.
+// The rule of the order.  It pays where the hierarchy is large enough that rays near each
+// other share nodes that others do not, and where a queue is long enough that the order's
+// launch, some 10 us whatever the length, is small beside its traversal: the paths in flight
+// are the queue's length while photons are left.  Whole renders without / with one order, ms
+// (B200; frames of 512^2, as many paths in flight as photons):
+//   closest-hit rays                      connections
+//   glass, 82 k triangles (9 k nodes)     the same
+//     2^20  3.36 / 3.49                     2^19  2.43 / 2.46
+//     2^21  4.95 / 5.04                     2^20  3.36 / 3.37
+//     2^22  7.93 / 7.93                     2^21  4.95 / 4.92
+//     2^23  13.79 / 13.64                   2^22  7.93 / 7.88
+//   glass, 328 k triangles (37 k nodes)   the same
+//     2^21  5.62 / 5.73                     2^19  2.79 / 2.80
+//     2^22  8.86 / 8.88                     2^20  3.84 / 3.83
+//     2^23  15.36 / 15.15                   2^22  8.86 / 8.75
+//   fog + 60 k strands                    the same
+//     2^18  2.95 / 3.00                     2^19  4.07 / 4.12
+//     2^19  4.07 / 4.03                     2^20  6.01 / 5.94
+//     2^22  16.74 / 15.99                   2^22  16.74 / 16.11
+// A frame of 2^27 photons through the larger glass, 2^23 in flight: neither 211.3, rays 200.8,
+// connections 209.9, both 197.8; fog + 250 k strands, 2^25 photons: 113.8, 107.4, 107.2, 100.2.
+// Four views of the smaller glass (2^21 in flight): 21.6, rays 22.0, connections 21.5.  By
+// nodes: Cornell (9) 11.4 without the order of the rays, 11.9 with it (by direction alone),
+// showroom (2 k) equal, glass of 20 k triangles 24.0 / 23.4 with 2^23 in flight.
 constexpr int32_t kSortNodes = 8192;
+constexpr int64_t kSortRaysTriangles = (int64_t)1 << 22, kSortRaysShapes = (int64_t)1 << 19;
+constexpr int64_t kSortConnections = (int64_t)1 << 20;
 inline bool scene_is_deep(const DevScene& sc) { return sc.max_nodes >= kSortNodes; }
 inline int32_t sort_setting(int32_t sort_rays) {   // of ftb_tuning.sort_rays
     return sort_rays == kSortLarge ? kSortLarge : (sort_rays ? kSortAlways : kSortNever);
 }
-// The order of a launch; deep: some scene of its jobs is large.
-inline RayOrder ray_order(int32_t setting, bool deep) {
+// The order of a launch with at most `paths` paths in flight; deep: some scene of its jobs is
+// large; shapes: some scene has spheres or curves.
+inline RayOrder ray_order(int32_t setting, bool deep, bool shapes, int64_t paths) {
     RayOrder o;
-    o.rays = setting == kSortAlways || (setting == kSortLarge && deep);
-    o.connections = setting != kSortNever && deep;
+    if (setting == kSortNever) return o;
+    o.rays = setting == kSortAlways || (deep && paths >= (shapes ? kSortRaysShapes : kSortRaysTriangles));
+    o.connections = deep && (setting == kSortAlways || paths >= kSortConnections);
     return o;
 }
 // Whether a scene's world records include spheres or curves.

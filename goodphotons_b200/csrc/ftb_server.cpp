@@ -407,7 +407,7 @@ void scheduler(ftb_server* s) {
         const bool stream = s->shape.regenerate;
         // the pass's connection fan-out (planar mirrors) bounds its paths in flight
         const int32_t slots = (int32_t)std::min<int64_t>(photons, std::max(1, s->W / fanout));
-        kind.order = ftb::ray_order(s->shape.sort_rays, deep);
+        kind.order = ftb::ray_order(s->shape.sort_rays, deep, kind.shapes, slots);
         int32_t* par = reinterpret_cast<int32_t*>(w.table + ftb::kWaveJobs);
         par[0] = (int32_t)table.size();
         par[1] = slots;

@@ -472,8 +472,8 @@ typedef struct ftb_tuning {
     int32_t use_graphs;   /* 0 / 1 */
     int32_t sort_rays;    /* order closest-hit rays by origin and direction, and connections by
                              image tile, before traversal: 0 never, 2 (the default) where the
-                             scene is large enough to gain, 1 the rays of every scene and the
-                             connections of large ones */
+                             scene and the paths in flight are enough to gain, 1 the rays of
+                             every scene and the connections of large ones */
     int32_t regenerate;   /* 0 / 1: streaming passes -- a slot freed by a finished path is
                              refilled with the next photon at once, so the device stays full
                              until the last photons (1), or waves traced to their last bounce

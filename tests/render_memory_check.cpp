@@ -278,10 +278,16 @@ void stated_memory() {
         }
 }
 
-// Rays are ordered where the tuning says so: never, always, or where the scene is large.
+// Rays are ordered where the tuning says so: never, always, or where the scene is large and the
+// paths in flight are many.
 void ray_order() {
     struct Row { int nodes; bool shapes; int32_t slots; bool rays, connections; };   // for sort_rays 2
-    const Row rows[] = {{100000, false, 1 << 22, true, true}, {100, false, 1 << 22, false, false}};
+    const Row rows[] = {
+        {100000, false, 1 << 19, false, false}, {100000, false, 1 << 20, false, true},
+        {100000, false, 1 << 21, false, true},  {100000, false, 1 << 22, true, true},
+        {100000, true, 1 << 18, false, false},  {100000, true, 1 << 19, true, false},
+        {100000, true, 1 << 20, true, true},    {100, false, 1 << 22, false, false},
+        {100, true, 1 << 22, false, false}};
     for (int regenerate : {1, 0})
         for (const Row& r : rows)
             for (int sort_rays : {0, 1, 2}) {
