@@ -63,7 +63,7 @@ def test_films_equal_around_the_limit(gpu, tuning, name):
     sc.close()
 
 
-def _bright_room(L, hero):
+def _bright_room(L):
     """Nearly every vertex connects and few paths die: translucent walls of albedo ~1."""
     sb = scenes.SceneBuilder()
     wall = sb.material(abi.MAT_DIFFUSE_TRANSMIT, reflect=sb.const(0.9), transmit=sb.const(0.099))
@@ -72,19 +72,49 @@ def _bright_room(L, hero):
     return sb.build(L)
 
 
+def _mirror_room(L):
+    """A white room open to the camera whose back wall is a mirror: a vertex connects to the eye
+    and, through the mirror, a second time."""
+    sb = scenes.SceneBuilder()
+    white = sb.diffuse(sb.const(0.99))
+    sb.quad((0, 0, 0), (0, 0, 2), (2, 0, 0), white)
+    sb.quad((0, 2, 0), (2, 0, 0), (0, 0, 2), white)
+    sb.quad((0, 0, 0), (0, 2, 0), (0, 0, 2), white)
+    sb.quad((2, 0, 0), (0, 0, 2), (0, 2, 0), white)
+    sb.quad((0, 0, 0), (2, 0, 0), (0, 2, 0), sb.material(abi.MAT_MIRROR, reflect=sb.const(0.95)))
+    sb.area_light((0.75, 1.9, 0.75), (0.5, 0, 0), (0, 0, 0.5), (0, -1, 0), sb.blackbody(6500.0))
+    return sb.build(L)
+
+
+def _connections(sc, cam, n, mb, hero, film, stream):
+    """Connections n photons make (the occlusion rays and mirror records of a counting render)."""
+    sc.set_profiling(2)
+    sc.profile(True)
+    _device(sc, cam, n, 3, mb, hero, film, stream)
+    made = sc.profile(True).counters[3]
+    sc.set_profiling(0)
+    return made
+
+
 @pytest.mark.parametrize("hero", [1, 4])
-def test_connections_beyond_the_queue(gpu, tuning, hero):
+@pytest.mark.parametrize("room,planes", [(_bright_room, 0), (_mirror_room, 1)])
+def test_connections_beyond_the_queue(gpu, tuning, room, planes, hero):
     torch = pytest.importorskip("torch")
-    sc = lib.Scene(_bright_room(gpu, hero), 0, gpu)
+    sc = lib.Scene(room(gpu), 0, gpu)
     cam = scenes.default_camera(gpu, 40)
-    n, mb = 20_000, 24
+    n, mb = 16_000, 24
     stream = torch.cuda.current_stream().cuda_stream
     films, tallies = [], []
     for regenerate in (1, 0):
         tuning(regenerate=regenerate)
+        # a log makes the wave buffer anew, so the next render's has room for its n photons only:
+        # a slot per photon and fan-out, three connection records per slot
+        sc.trace_log(cam, 1)
         film = torch.zeros((40, 40, 4), dtype=torch.int64, device="cuda:0")
         tallies.append(_device(sc, cam, n, 3, mb, hero, film, stream))
         films.append(film.cpu().numpy())
+    made = _connections(sc, cam, n, mb, hero, film, stream)
+    assert made > 1.25 * 3 * n * (1 + planes)   # a quarter of the queue and more found it full
     if hero == 1:
         film = torch.zeros((40, 40, 4), dtype=torch.int64, device="cuda:0")
         p, info, en = abi.RenderParams(n, 3, mb, 24, 1, 0), abi.FilmInfo(), abi.Energy()
@@ -92,8 +122,9 @@ def test_connections_beyond_the_queue(gpu, tuning, hero):
                                                    C.byref(info), C.byref(en), C.c_void_p(stream)))
         films.append(film.cpu().numpy())
         tallies.append(np.array(list(en.fx), dtype=np.int64))
+        assert made > 1.25 * 3 * abi.NOALLOC_MAX_PHOTONS   # and the fixed one of this entry point
     sc.close()
-    assert films[1][..., 3].sum() > n   # (a path makes ~20 connections, most of them occluded)
+    assert films[1][..., 3].sum() > n   # (in the closed room most connections are occluded)
     for f, t in zip(films[1:], tallies[1:]):
         np.testing.assert_array_equal(films[0], f)
         np.testing.assert_array_equal(tallies[0], t)
