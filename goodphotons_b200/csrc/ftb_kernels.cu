@@ -508,10 +508,10 @@ __device__ void hit_attributes(const double* __restrict__ tri_n, const RayCtx& R
 // box grown by 2^-18 x the scene's largest coordinate M (the builders check each against the
 // exact box), and a plane x is entered at t = fma(x, ix, cx) with ix = 1/d and cx = -o*ix
 // rounded to float.  The rounding of o, of cx and of the fma move t by at most ~2^-23 M |ix|
-// (far inside the box growth, 2^-18 M |ix|); the rounding of d (2^-24), of 1/d (the
-// approximate reciprocal, 1 ulp: 2^-23) and of the fma's result (2^-24) scale t by at most
-// ~(1 +- 2^-22) on either side of the interval, inside its widening by 2^-20 (T_WIDE).  So no
-// ray culls a child whose primitives the exact fp64 test would hit.
+// (far inside the box growth, 2^-18 M |ix|); the rounding of d, of 1/d and of the fma's result
+// (2^-24 each) scale t by less than 1 +- 2^-22 on either side of the interval, inside its
+// widening by 1.25 x 2^-20 (T_WIDE).  So no ray culls a child whose primitives the exact fp64
+// test would hit.
 struct RayF {
     float ix, iy, iz;
     float cx, cy, cz;       // -o * ix per axis
@@ -520,11 +520,6 @@ struct RayF {
 // Rows of planes in a node: lo x, y, z at 32, 64, 96 and hi x, y, z at 128, 160, 192, so an
 // axis' near and far offsets add up to kRowSum + 64 * axis.
 constexpr uint32_t kRowLo = 32, kRowSide = 96, kRowSum = 2 * kRowLo + kRowSide;
-__device__ __forceinline__ float rcp_approx(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ RayF make_rayf(D3 o, D3 d) {
     RayF r;
     float dx = (float)d.x, dy = (float)d.y, dz = (float)d.z;
@@ -533,7 +528,9 @@ __device__ __forceinline__ RayF make_rayf(D3 o, D3 d) {
     dx = fabsf(dx) > 1e-20f ? dx : copysignf(1e-20f, dx);
     dy = fabsf(dy) > 1e-20f ? dy : copysignf(1e-20f, dy);
     dz = fabsf(dz) > 1e-20f ? dz : copysignf(1e-20f, dz);
-    r.ix = rcp_approx(dx); r.iy = rcp_approx(dy); r.iz = rcp_approx(dz);
+    // correctly rounded; the approximate reciprocal would save 0.2 % of the walk (glass 111.1
+    // against 110.8 ms of closest hits a frame)
+    r.ix = __frcp_rn(dx); r.iy = __frcp_rn(dy); r.iz = __frcp_rn(dz);
     r.cx = -(float)o.x * r.ix; r.cy = -(float)o.y * r.iy; r.cz = -(float)o.z * r.iz;
     r.nx = kRowLo + (dx < 0.0f ? kRowSide : 0u);   // near is the hi side where d is negative
     r.ny = kRowLo + 32 + (dy < 0.0f ? kRowSide : 0u);
