@@ -111,3 +111,28 @@ def test_noalloc_hero_request_in_media_traces_one_wavelength(gpu):
         assert list(ea.fx) == list(eb.fx)
     finally:
         sc.close()
+
+
+def test_noalloc_calls_of_several_scene_kinds_leave_memory_unchanged(gpu):
+    """The first call of a kind of scene loads its kernels and may make the driver set more local
+    memory aside; after one call of each kind, calls in any order leave the device's free memory
+    unchanged."""
+    torch = pytest.importorskip("torch")
+    L = gpu
+    kinds = [mk for mk, _ in SCENES.values()] + [cases.make_mirrors]
+    scs = [lib.Scene(mk(L), 0, L) for mk in kinds]
+    cam = scenes.default_camera(L, RES)
+    film = torch.zeros((RES, RES, 4), dtype=torch.int64, device="cuda:0")
+    stream = torch.cuda.current_stream()
+    try:
+        for sc in scs:
+            _noalloc(L, sc, cam, film, 8000, 1, 16, stream=stream.cuda_stream)
+        torch.cuda.synchronize()
+        free = _free_bytes(L)
+        for sc in scs[::-1] + scs:
+            _noalloc(L, sc, cam, film, 8000, 1, 16, stream=stream.cuda_stream)
+            torch.cuda.synchronize()
+            assert _free_bytes(L) == free
+    finally:
+        for sc in scs:
+            sc.close()
