@@ -857,7 +857,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.shapes = shapes;
         kind.mirrors = mirrors;
         kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep, shapes, slots);
-        kind.multi = ftb::table_class(table.size());
+        kind.rows = ftb::table_rows(table.size());
         e = ftb::launch_stream(w, g, slots, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                                graphs);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
@@ -912,7 +912,7 @@ ftb_status launch_jobs(ftb_scene* s, int32_t W, int buffers, const std::vector<f
         kind.shapes = shapes;
         kind.mirrors = mirrors;
         kind.order = ftb::ray_order(s->eng->shape.sort_rays, deep, shapes, slots);
-        kind.multi = ftb::table_class(table.size());
+        kind.rows = ftb::table_rows(table.size());
         e = ftb::launch_wave(w, max_bounce, kind, f, s->sms, s->eng->shape, ws, s->prof_mode ? s->prof : nullptr,
                              graphs);
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");

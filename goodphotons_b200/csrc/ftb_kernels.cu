@@ -1347,10 +1347,10 @@ enum { T_EMIT = 0, T_ABS = 1, T_SENSOR = 2, T_ESC = 3, T_RES = 4 };
 // books changes -- often, in a streaming pass, where the paths of neighbouring jobs share
 // the queues -- and the block adds the table's nonzero entries to the jobs' tallies once
 // at the end, so the global atomics per launch do not grow with the job changes.  The table
-// is dynamic shared memory, as large as the launch's table class: eight blocks' full tables
-// take 82 KB of the SM's storage from the L1 that holds these kernels' spills (shading of a
-// frame of one job with the table / without it, B200: Cornell 4.67 / 4.34 ms, glass 54.7 /
-// 52.4, Cornell bundles 1.92 / 1.82; eight jobs, full / small table: 19.7 / 18.9).
+// is dynamic shared memory of table_rows() rows: eight blocks' full tables take 82 KB of the
+// SM's storage from the L1 that holds these kernels' spills (shading of a frame of one job with
+// the full table / without one, B200: Cornell 4.67 / 4.34 ms, glass 54.7 / 52.4, Cornell
+// bundles 1.92 / 1.82).
 constexpr size_t kTallyRow = sizeof(unsigned long long) * 5;
 struct TallyAcc {
     int job;
@@ -3030,7 +3030,7 @@ struct Issue {
         return std::max(1, std::min(sms * per_sm, (entries + chunk - 1) / chunk));
     }
     size_t tally() const {   // dynamic shared memory of the tally kernels
-        return kTallyRow * (kind.multi == 0 ? 0 : (kind.multi == 1 ? kSmallTable : kWaveJobs));
+        return kTallyRow * (size_t)kind.rows;
     }
     int32_t tail() const { return f.stats ? 0 : trace_limit(sms); }
 

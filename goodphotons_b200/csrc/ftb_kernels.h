@@ -198,17 +198,22 @@ struct WaveKind {
     bool shapes = false;      // some scene has spheres or curves (not only triangles)
     bool mirrors = false;     // some scene has planar mirrors (mirror connections queued)
     RayOrder order;           // which rays are ordered before traversal (ray_order)
-    int32_t multi = 0;        // table_class() of the table's jobs (it must be exactly that)
+    int32_t rows = 0;         // table_rows() of the table's jobs (it must be exactly that)
     bool operator==(const WaveKind& o) const {
         return instances == o.instances && bundles == o.bundles && media == o.media && shapes == o.shapes &&
                mirrors == o.mirrors && order.rays == o.order.rays && order.connections == o.order.connections &&
-               multi == o.multi;
+               rows == o.rows;
     }
 };
-// Tables by size: 0 one job, 1 at most kSmallTable, 2 more.  The tally kernels hold a row per
-// job in shared memory, and what they hold is taken from L1.
-constexpr int32_t kSmallTable = 32;
-inline int32_t table_class(size_t jobs) { return jobs <= 1 ? 0 : (jobs <= (size_t)kSmallTable ? 1 : 2); }
+// Rows of the tally table that the kernels hold in shared memory, one per job; none for one job.
+// What they take is lost to L1, in the steps in which an SM sets shared memory aside: with 1 KB
+// that each of its 8 blocks takes anyway, 64 rows of 40 B need 28 KB and so the same 32 KB as 32
+// rows, 128 rows the step of 64 KB and 256 rows that of 100 KB.  Shading of a batch of 2^24
+// photons through glass (B200): 8 jobs 9.48 ms with 32 or 64 rows, 9.68 with 128, 9.89 with
+// 256; 40 jobs 9.69 with 64, 10.12 with 256; 100 jobs 10.01 with 128, 10.24 with 256.
+inline int32_t table_rows(size_t jobs) {
+    return jobs <= 1 ? 0 : (jobs <= 64 ? 64 : (jobs <= 128 ? 128 : kWaveJobs));
+}
 // Connection records one path vertex of job J can queue: a camera connection and one per
 // planar mirror, for each of the job's views.  A wave or pass keeps its slots at most
 // W / fanout so that the shadow queue (kShadowPerSlot records per slot) cannot overflow.

@@ -400,7 +400,7 @@ void scheduler(ftb_server* s) {
         }
         retire(s, b);   // the buffer's previous wave
         WaveSlot& w = s->ws[b];
-        kind.multi = ftb::table_class(table.size());
+        kind.rows = ftb::table_rows(table.size());
         std::memcpy(w.table, table.data(), sizeof(ftb::DevJob) * table.size());
         // streaming pass: {ranges, paths in flight, photons (int64), half-iteration cap (int64)};
         // wave: {jobs, slots}

@@ -78,7 +78,7 @@ def test_ordered_queues_of_large_scenes(gpu, tuning, name, build):
     sc.close()
 
 
-@pytest.mark.parametrize("n_jobs", [3, 40])   # job tables of up to 32 rows, and of more
+@pytest.mark.parametrize("n_jobs", [3, 40, 64, 65, 128, 129])   # tally tables of 64, 128 and 256 rows
 def test_ordered_queues_of_mixed_scenes(gpu, tuning, n_jobs):
     """Each path is put on the grid of its own job's scene, and tallied to its own job."""
     torch = pytest.importorskip("torch")
