@@ -595,8 +595,6 @@ double box_maxabs(const ftb::Box& b, double m) {
     return m;
 }
 
-// Bake one BLAS on `device` (current): triangle boxes, wide BVH with a margin from the
-// local coordinate magnitude, records in leaf order (prim = the triangle's BLAS index).
 // Record rows (PrimRec): a triangle's vertices by axis, or up to three values per row; the
 // tail (prim, info) goes to the end of every row.
 void rec_triangle(PrimRec& R, const double* v) {
@@ -608,6 +606,8 @@ void rec_tail(PrimRec& R, int32_t prim, int32_t info) {
     for (auto& row : R.row) std::memcpy(&row[3], &tail, sizeof tail);
 }
 
+// Bake one BLAS on `device` (current): triangle boxes, wide BVH with a margin from the
+// local coordinate magnitude, records in leaf order (prim = the triangle's BLAS index).
 ftb_status bake_blas(const ftb_blas_desc& d, int device, ftb::BuildMethod method, std::shared_ptr<BlasDev>& out) {
     auto b = std::make_shared<BlasDev>();
     b->mem.device = device;

@@ -3025,13 +3025,13 @@ struct Issue {
     int32_t sms;
     static constexpr int T = 128;
 
-    // paths left to the whole-path kernels, which have no counting variant
     int sort_grid(int entries, int chunk, int per_sm) const {
         return std::max(1, std::min(sms * per_sm, (entries + chunk - 1) / chunk));
     }
     size_t tally() const {   // dynamic shared memory of the tally kernels
         return kTallyRow * (size_t)kind.rows;
     }
+    // paths left to the whole-path kernels, which have no counting variant
     int32_t tail() const { return f.stats ? 0 : trace_limit(sms); }
 
     void mark(int k, bool end) { if (sink) sink->mark(k, end, st); }
@@ -3254,7 +3254,7 @@ void stream_paths(Issue& I) {
 
 struct WaveGraphs {
     struct Entry {
-        int32_t max_bounce, grid;   // max_bounce -1: a streaming pass, -2: one of few photons, -3: a wave of few
+        int32_t max_bounce, grid;   // max_bounce -1: a streaming pass, -2: one of few photons
         WaveKind kind;
         int32_t* status;
         cudaGraphExec_t exec;
@@ -3293,22 +3293,21 @@ cudaError_t launch_wave(Wave& w, int32_t max_bounce, const WaveKind& kind, const
     if (kind.bundles && w.hero < 2) return cudaErrorInvalidValue;   // the buffer carries no bundles
     const int grid = launch_grid(w, sms, shape);
     // A graph bakes the kernel arguments: the wave's buffers and status word are fixed for the
-    // life of its cache, but a log buffer changes per call, so logging waves launch directly.
-    if (!(shape.graph && graphs) || sink || f.stats || w.logs) {
+    // life of its cache, but a log buffer changes per call, so logging waves launch directly, and
+    // so do whole paths (few launches, for a caller without a cache).
+    if (!(shape.graph && graphs) || sink || f.stats || w.logs || whole_paths) {
         Issue I{w, kind, f, grid, st, sink, sms};
         if (whole_paths) issue_wave_paths(I);
         else issue_wave(I, max_bounce);
         return cudaGetLastError();
     }
-    if (whole_paths) max_bounce = -3;
     if (cudaGraphExec_t ex = graphs->find(max_bounce, grid, kind, f.status))
         return cudaGraphLaunch(ex, st);
     cudaGraph_t g = nullptr;
     cudaError_t err = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (err != cudaSuccess) return err;
     Issue I{w, kind, f, grid, st, nullptr, sms};
-    if (whole_paths) issue_wave_paths(I);
-    else issue_wave(I, max_bounce);
+    issue_wave(I, max_bounce);
     err = cudaStreamEndCapture(st, &g);
     if (err != cudaSuccess) return err;
     WaveGraphs::Entry e{max_bounce, grid, kind, f.status, nullptr};

@@ -47,11 +47,11 @@ static_assert(sizeof(WNode) == 80, "WNode must be 80 bytes");
 // per axis and side, so a ray takes its near and far planes by its direction's signs with
 // no per-child select.  Every row of eight planes, and the header, is one 32-byte sector:
 // a node visit is six 32-byte loads and one of 16 (a node is 224 B, so rows stay aligned).
-// meta byte: 0 = empty; count<<5 | offset for a leaf (count 1..4, offset from prim_base);
-// 7<<5 | offset for an inner child (offset from child_base).  code byte, the same child as
-// the traversal adds it to a base: 0..127 an inner child's offset; 128 | offset<<2 |
-// (count - 1) a leaf's.  An empty child has lo = +inf and hi = -inf on every axis, which
-// every ray's slab test misses.
+// meta byte (what the builders' checks read): 0 = empty; count<<5 | offset for a leaf (count
+// 1..4, offset from prim_base); 7<<5 | offset for an inner child (offset from child_base).
+// code byte, the same child as the traversal adds it to a base: 0..127 an inner child's offset;
+// 128 | offset<<2 | (count - 1) a leaf's.  An empty child has lo = +inf and hi = -inf on every
+// axis, which every ray's slab test misses.
 struct alignas(32) FNode {
     uint32_t child_base;
     uint32_t prim_base;

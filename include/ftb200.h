@@ -449,9 +449,13 @@ ftb_status ftb_render_forward_noalloc(ftb_scene* scene, const ftb_camera* cam,
  * mode 0: off.  mode 1: every kernel launch of this scene's renders is bracketed by CUDA
  * events on its own stream; ftb_scene_profile sums the durations per kernel.  mode 2:
  * additionally run the counting variants of the traversal kernels, which tally rays, BVH
- * node visits and primitive-record tests (slower: never time a mode-2 render). */
+ * node visits and primitive-record tests (slower: never time a mode-2 render); it
+ * traces every path bounce by bounce, so that each ray is counted. */
 typedef struct ftb_kernel_profile {
-    double ms[4];          /* summed launch durations: emit, extend, shade, shadow */
+    double ms[4];          /* summed launch durations: emit, extend, shade, shadow; the order of
+                              rays with the traversal it serves, and launches that trace paths
+                              to their ends (passes of few photons, the tail of others),
+                              shading included, with extend */
     int64_t launches[4];
     uint64_t counters[8];  /* mode 2: closest-hit rays, their node visits, their record
                               tests; any-hit rays, node visits, record tests; the record
