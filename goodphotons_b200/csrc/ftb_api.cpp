@@ -1957,12 +1957,15 @@ ftb_status ftb_autotune(ftb_scene* s, const ftb_camera* cam, int64_t n, int32_t 
         const int waves[] = {1 << 20, 1 << 21, 1 << 22, 1 << 23, 1 << 24};
         for (int pass = 0; pass < 5 && st == FTB_OK; ++pass) {
             std::vector<ftb_tuning> cand;
-            if (pass == 4) best_ms = 1e300;   // the default, by scene, is the same launches as one of the two
+            // a large scene's choice is the rule or nothing, so that small scenes on the device keep
+            // theirs; a small scene's, whose rule is nothing, every scene's rays or nothing
+            const int order = ftb::scene_is_deep(s->dev) ? ftb::kSortLarge : ftb::kSortAlways;
+            if (pass == 4) best_ms = 1e300;   // the default is the same launches as one of the two
             if (pass == 0) for (int u = 0; u < 2; ++u) { ftb_tuning t = best; t.regenerate = u; cand.push_back(t); }
             if (pass == 1) for (int g : grids) { ftb_tuning t = best; t.grid_mult = g; cand.push_back(t); }
             if (pass == 2) for (int w : waves) { ftb_tuning t = best; t.wave_slots = w; cand.push_back(t); }
             if (pass == 3) for (int u = 0; u < 2; ++u) { ftb_tuning t = best; t.use_graphs = u; cand.push_back(t); }
-            if (pass == 4) for (int u = 0; u < 2; ++u) { ftb_tuning t = best; t.sort_rays = u; cand.push_back(t); }
+            if (pass == 4) for (int u : {(int)ftb::kSortNever, order}) { ftb_tuning t = best; t.sort_rays = u; cand.push_back(t); }
             for (const ftb_tuning& t : cand) {
                 double ms = 0;
                 st = trial(t, ms);

@@ -492,8 +492,9 @@ typedef struct ftb_tuning {
 ftb_status ftb_get_tuning(int32_t device, ftb_tuning* out);
 ftb_status ftb_set_tuning(int32_t device, const ftb_tuning* t);
 /* Autotuner: render n_photons of `scene` through `cam` (into a scratch film) under
- * candidate tunings -- grid sizes, wave sizes, graphs on and off, one knob at a time from the
- * current setting -- timing each with CUDA events after a warm-up, then keep the fastest
+ * candidate tunings -- grid sizes, wave sizes, graphs on and off, rays ordered or not (a large
+ * scene chooses between sort_rays 2 and 0, a small one between 1 and 0), one knob at a time from
+ * the current setting -- timing each with CUDA events after a warm-up, then keep the fastest
  * for the scene's device and return it.  n_photons of at least a few waves (>= 2^23) gives
  * stable timings. */
 ftb_status ftb_autotune(ftb_scene* scene, const ftb_camera* cam, int64_t n_photons, int32_t max_bounce,

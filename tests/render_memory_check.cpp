@@ -23,6 +23,7 @@ std::map<void*, size_t> blocks;
 size_t live = 0, peak = 0, limit = SIZE_MAX;
 int events = 0, overlaps = 0, launch_fails_at = -1;
 uintptr_t handles = 0;
+bool order_pays = true;
 cudaError_t last = cudaSuccess;
 
 cudaError_t err(cudaError_t e) { if (e != cudaSuccess) last = e; return e; }
@@ -108,7 +109,11 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
     fake::done.insert(fake::recorded[e].begin(), fake::recorded[e].end());
     return cudaSuccess;
 }
-cudaError_t cudaEventElapsedTime(float* t, cudaEvent_t, cudaEvent_t) { *t = 1.0f; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* t, cudaEvent_t, cudaEvent_t) {   // ordered rays take half the time, or twice
+    const bool ordered = !fake::launches.empty() && fake::launches.back().order.rays;
+    *t = ordered == fake::order_pays ? 1.0f : 2.0f;
+    return cudaSuccess;
+}
 }
 
 namespace ftb {
@@ -303,6 +308,18 @@ void ray_order() {
                 check(o.connections == (sort_rays == 2 ? r.connections : sort_rays == 1 && r.nodes > 10000),
                       "connections", where);
             }
+    // the autotuner's choice: by its times, and in a large scene one that leaves small scenes alone
+    for (int nodes : {100000, 100})
+        for (bool pays : {true, false}) {
+            fake::reset();
+            fake::order_pays = pays;
+            Host h(1, 1, 1 << 22);
+            h.s->dev.max_nodes = nodes;
+            ftb_tuning t{};
+            check(ftb_autotune(h.s, &h.cam, 1 << 22, 4, &t) == FTB_OK, ftb_last_error(), "autotune");
+            check(t.sort_rays == (pays ? (nodes > 10000 ? 2 : 1) : 0), "sort_rays",
+                  "autotune nodes " + std::to_string(nodes) + (pays ? " pays" : "") + " " + std::to_string(t.sort_rays));
+        }
 }
 }  // namespace
 
