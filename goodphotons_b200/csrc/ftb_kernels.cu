@@ -520,6 +520,17 @@ struct RayF {
 // Rows of planes in a node: lo x, y, z at 32, 64, 96 and hi x, y, z at 128, 160, 192, so an
 // axis' near and far offsets add up to kRowSum + 64 * axis.
 constexpr uint32_t kRowLo = 32, kRowSide = 96, kRowSum = 2 * kRowLo + kRowSide;
+// 1 / x of a normal x with a normal 1 / x: the approximate reciprocal (1 ulp) and one step of
+// Newton's iteration for the root of 1 / r - x.  Compared on a B200 with the correctly rounded
+// reciprocal over every mantissa at the exponents -66 .. 3: equal in all of them (the
+// approximation alone in 87 %).  The rounded reciprocal itself branches for subnormals, which
+// a ray's direction (make_rayf) never is: renders bound by one path's latency take 1.5 % longer
+// with it (preview of 2^16 photons 0.257 against 0.254 ms), small ones with planar mirrors 4 %.
+__device__ __forceinline__ float reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return __fmaf_rn(r, __fmaf_rn(-x, r, 1.0f), r);
+}
 __device__ __forceinline__ RayF make_rayf(D3 o, D3 d) {
     RayF r;
     float dx = (float)d.x, dy = (float)d.y, dz = (float)d.z;
@@ -528,9 +539,7 @@ __device__ __forceinline__ RayF make_rayf(D3 o, D3 d) {
     dx = fabsf(dx) > 1e-20f ? dx : copysignf(1e-20f, dx);
     dy = fabsf(dy) > 1e-20f ? dy : copysignf(1e-20f, dy);
     dz = fabsf(dz) > 1e-20f ? dz : copysignf(1e-20f, dz);
-    // correctly rounded; the approximate reciprocal would save 0.2 % of the walk (glass 111.1
-    // against 110.8 ms of closest hits a frame)
-    r.ix = __frcp_rn(dx); r.iy = __frcp_rn(dy); r.iz = __frcp_rn(dz);
+    r.ix = reciprocal(dx); r.iy = reciprocal(dy); r.iz = reciprocal(dz);
     r.cx = -(float)o.x * r.ix; r.cy = -(float)o.y * r.iy; r.cz = -(float)o.z * r.iz;
     r.nx = kRowLo + (dx < 0.0f ? kRowSide : 0u);   // near is the hi side where d is negative
     r.ny = kRowLo + 32 + (dy < 0.0f ? kRowSide : 0u);
