@@ -45,8 +45,9 @@ WORKLOADS = {
 METRIC = "photon paths/s on 1 B200"
 NODE_BYTES = 80     # a node in its compressed form (WNode, 8-bit child planes): the algorithmic
                     # unit, although the device reads the 208-byte widened form (FNode)
-NODE_READ_BYTES = 208   # FNode, the node as the kernels read it (the secondary figure)
-REC_BYTES = 80      # PrimRec
+NODE_READ_BYTES = 208   # of an FNode (224 B) as a visit reads it (the secondary figure)
+REC_BYTES = 80      # a record's nine doubles, index and material / type: the algorithmic unit
+REC_READ_BYTES = 96     # PrimRec, a record as the kernels read it
 RAY_IO_BYTES = 64   # extend: queue index 4 + ray 48 read, hit t 8 + record 4 written
 SHADOW_IO_BYTES = 140   # shadow: record read (origin 24, direction 24, max 8, XYZ 24, pixel, job,
                         # view 12) + 4 film words of 8 B updated (read + write)
@@ -810,7 +811,7 @@ def main():
     t = time.perf_counter()
     if args.tuning:   # a fixed setting instead (reproducible launch sequences for profiling)
         v = [int(x) for x in args.tuning.split(",")]
-        v += [0, 1][len(v) - 3:]
+        v += [2, 1][len(v) - 3:]
         tuning = L.set_tuning(local, wave_slots=v[0], grid_mult=v[1], use_graphs=v[2], sort_rays=v[3],
                               regenerate=v[4])
     else:
@@ -869,12 +870,14 @@ def main():
         ki, kname = 3, "k_shadow (any-hit traversal of the camera connections + splat)"
         srays_c = max(1, cp.counters[3])
         unit_bytes = (cp.counters[4] * NODE_BYTES + cp.counters[5] * REC_BYTES) / srays_c + SHADOW_IO_BYTES
-        read_bytes = unit_bytes + cp.counters[4] * (NODE_READ_BYTES - NODE_BYTES) / srays_c
+        read_bytes = unit_bytes + (cp.counters[4] * (NODE_READ_BYTES - NODE_BYTES)
+                                   + cp.counters[5] * (REC_READ_BYTES - REC_BYTES)) / srays_c
         units_timed = cp.counters[3] / n_count * n * args.steps
     else:
         ki, kname = 1, "k_extend (closest-hit traversal)"
         unit_bytes = bytes_per_ray
-        read_bytes = unit_bytes + nodes_c * (NODE_READ_BYTES - NODE_BYTES) / max(1, rays_c)
+        read_bytes = unit_bytes + (nodes_c * (NODE_READ_BYTES - NODE_BYTES)
+                                   + recs_c * (REC_READ_BYTES - REC_BYTES)) / max(1, rays_c)
         units_timed = rays_per_photon * n * args.steps   # of the profiled steps
         traffic_ray = ncu_traffic_per_ray(args.workload)
     launches_k = max(1, prof.launches[ki])
@@ -897,9 +900,9 @@ def main():
                     "achieved": round(achieved * read_bytes / unit_bytes, 1),
                     "frac": round(achieved * read_bytes / unit_bytes / peak, 4),
                     "note": f"the same launches with each node visit counted at the {NODE_READ_BYTES} B "
-                            "the kernel reads (nodes as laid out on the device); a wider layout raises "
-                            "this figure without moving more useful data, so `frac` above is the one "
-                            "to compare across layouts"},
+                            f"and each record test at the {REC_READ_BYTES} B the kernel reads; a wider "
+                            "layout raises this figure without moving more useful data, so `frac` above "
+                            "is the one to compare across layouts"},
         "node_visits_per_ray": round(nodes_c / max(1, rays_c), 3),
         "record_tests_per_ray": round(recs_c / max(1, rays_c), 3),
         "closest_hit_rays_per_photon": round(rays_per_photon, 4),
@@ -911,12 +914,13 @@ def main():
     }
     # kernels the profiled steps launched: the four traced kernels (counted by the profiler),
     # plus, in streaming passes, the progress kernel after every half-iteration (one per
-    # closest-hit launch) and a pass's set-up and first progress launch, and the queue sort
+    # shading launch) and a pass's set-up and first progress launch, and the order of the
+    # closest-hit rays where every scene has it (large scenes' orders by rule are not counted)
     gpu_launches = int(sum(prof.launches))
     if tuning.regenerate:
-        gpu_launches += int(prof.launches[1]) + 2 * args.steps
-    if tuning.sort_rays:
-        gpu_launches += int(prof.launches[1])
+        gpu_launches += int(prof.launches[2]) + 2 * args.steps
+    if tuning.sort_rays == 1:
+        gpu_launches += int(prof.launches[2])
 
     # the same frame on the GPU-built BVH (device LBVH: faster bake, looser tree)
     fa, fb = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
